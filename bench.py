@@ -189,12 +189,13 @@ def build_slabs(opr, N, args):
     opr.slab_scaling(args.slab_scaling)
     built = opr.build_slabs(slab_bytes=int(args.slab_mb * (1 << 20)), max_bytes=int(0.8 * free))
     dt = time.perf_counter() - t0
+    nbytes = free - torch.cuda.mem_get_info()[0]
     if not built:
         return {"built": False}
     passes, wc, entries = opr.slabs_info
     scaled = opr.slab_scaling()
     return {"built": True, "passes": passes, "columns_per_slab": wc, "entries": entries,
-            "bytes": entries * 4 + passes * N + passes * ((N + 31) // 32) * 4 + (17 * N if scaled else 0),
+            "bytes": nbytes,
             "build_s": dt, "scaled": scaled}
 
 
@@ -695,8 +696,7 @@ def run_gpu(args, wl):
                        "slab_table": dict(slab_info or {"built": False},
                                           used={"mixed": opr.slab_use("mixed") if slab_info and slab_info.get("built") else 0,
                                                 "fp64": opr.slab_use("fp64") if slab_info and slab_info.get("built") else 0},
-                                          use_codes="0 none, 1 slab product, 2 with cache hints, 3 eight entries "
-                                                    "per step, 4 both, 5 two lanes per row, 6 four lanes per row"),
+                                          use_codes="0 none, 1 to 6 slab product"),
                        "setup_s": t_space, "search_directory": dir_stats, "parent_map": map_info},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic, "peak_source": peak_src,
@@ -1016,8 +1016,7 @@ def main():
     ap.add_argument("--batch-launch", type=int, default=7, choices=[0, 1, 2, 3, 5, 6, 7],
                     help="batched workload with --tiling: the batch launch mode (edgpu_batch_set_launch)")
     ap.add_argument("--slab-mode", type=int, default=1, choices=[1, 2, 3, 4, 5, 6],
-                    help="with --tiling: the slab product's variant (1 plain, 2 cache hints, 3 eight entries "
-                         "per step, 4 both, 5 two lanes per row, 6 four lanes per row)")
+                    help="with --tiling: use the slab product (any value)")
     ap.add_argument("--slab-scaling", type=int, default=0, choices=[0, 1, 2],
                     help="slab table layout (edgpu_op_slab_scaling): 0 scaled on sectors of 2^22 rows or more "
                          "where that saves passes or the coefficients are complex, 1 never, 2 always")

@@ -207,9 +207,13 @@ struct edgpu_op_s {
     // column-slab table (optional, edgpu_op_build_slabs; mixed-precision products, hxslab.cu)
     struct Slab {
         unsigned* tab = nullptr;            // entries, pass after pass
-        unsigned char* counts = nullptr;    // [n_pass][dim] entries of each row in each pass
-        unsigned* off = nullptr;            // [n_pass][tiles] tile offsets relative to the pass
+        unsigned* mask = nullptr;           // the steps' row masks, pass after pass (null: padded)
+        int padded = 0;                     // every step has 32 entries
+        int tile_steps = 0;                 // mean steps of a tile in a pass
+        unsigned* off = nullptr;            // [n_pass][tiles + 1] first entries relative to the pass
+        unsigned* moff = nullptr;           // [n_pass][tiles + 1] first steps relative to the pass
         std::vector<long long> base;        // [n_pass + 1] first entry of each pass
+        std::vector<long long> mbase;       // [n_pass + 1] first step of each pass
         int n_pass = 0, colbits = 0, n_ids = 0, den = 1, nd = 1;
         long long wc = 0;                   // columns per slab
         int64_t n = 0;                      // entries
@@ -266,8 +270,9 @@ struct edgpu_op_s {
     void free_slabs() {
         drop_host_graphs();
         if (slab.tab) cudaFree(slab.tab);
-        if (slab.counts) cudaFree(slab.counts);
+        if (slab.mask) cudaFree(slab.mask);
         if (slab.off) cudaFree(slab.off);
+        if (slab.moff) cudaFree(slab.moff);
         if (slab.cls) cudaFree(slab.cls);
         slab.lut.release();
         slab.lut64.release();
@@ -1145,12 +1150,14 @@ void launch_slab_passes(edgpu_op_s* op, int prec, const Blob& B, const void* x, 
     r.y_c128 = y_c128;
     r.acc_c128 = acc_c128;
     r.accumulate = y_c128 ? 0 : accumulate;
-    r.hints = op->slab_hint[prec];
+    r.padded = S.padded;
+    r.tile_steps = S.tile_steps;
     const long long n_tiles = r.n_tiles;
     auto set_pass = [&](int q) {
-        r.cnt = S.counts + (size_t)q * r.n_rows;
-        r.off = S.off + (size_t)q * n_tiles;
+        r.off = S.off + (size_t)q * (n_tiles + 1);
+        r.moff = S.moff + (size_t)q * (n_tiles + 1);
         r.tab = S.tab + S.base[q];
+        r.mask = S.padded ? nullptr : S.mask + S.mbase[q];
         r.xs = (const char*)x + (size_t)q * S.wc * esz;
         r.first = q == 0;
         r.last = q == S.n_pass - 1;
@@ -2340,7 +2347,7 @@ int edgpu_op_build_slabs(edgpu_op oh, int64_t slab_bytes, int64_t max_bytes, int
         if (f != bc.flip[k] || f != bcu.flip[k]) return EDGPU_OK;
         n_pairs += f != 0;
     }
-    // a row's targets in one slab are counted in a byte: at most 255 pairs
+    // at most 255 pairs (steps of a tile in one pass)
     if (n_pairs > 255) return EDGPU_OK;
     auto& S = op->slab;
     const int n_slots = ncls * nb * 4;
@@ -2395,8 +2402,12 @@ int edgpu_op_build_slabs(edgpu_op oh, int64_t slab_bytes, int64_t max_bytes, int
         op->free_slabs();
         return EDGPU_OK;
     }
+    // a padding entry's id beside the others', where the columns of a slab leave room for it
     int idbits = 1;
-    while (((long long)1 << idbits) < n_ids) ++idbits;
+    while (((long long)1 << idbits) < n_ids + 1) ++idbits;
+    const bool pad_id = wc <= (long long)1 << (32 - idbits);
+    if (!pad_id)
+        for (idbits = 1; ((long long)1 << idbits) < n_ids;) ++idbits;
     const int colbits = 32 - idbits;
     const long long n_tiles = (sp.dim + 31) / 32;
     if (n_pass > 64) {
@@ -2420,50 +2431,84 @@ int edgpu_op_build_slabs(edgpu_op oh, int64_t slab_bytes, int64_t max_bytes, int
     sb.colbits = colbits;
     sb.n_slots = n_slots;
     sb.scaled = scaled ? 1 : 0;
-    sb.o_ctr = (int)align16(B.smem_bond);
-    // counts and tile offsets; a scaled table's orbit-size bytes and scaled-x buffer (complex128)
-    const size_t meta = (size_t)n_pass * sp.dim + (size_t)n_pass * n_tiles * 4 + (scaled ? (size_t)sp.dim * 17 : 0);
+    sb.cap = n_pass == 1 ? (n_pairs + 3) & ~3 : 256;   // a tile has at most n_pairs <= 255 steps in a pass
+    sb.o_scratch = (int)align16(B.smem_bond);
+    // tile offsets; a scaled table's orbit-size bytes and scaled-x buffer (complex128)
+    const size_t n_off = (size_t)n_pass * (n_tiles + 1);
+    const size_t meta = n_off * 8 + (scaled ? (size_t)sp.dim * 17 : 0);
     if ((double)meta > (double)max_bytes) {
         op->free_slabs();
         return EDGPU_OK;
     }
-    DevBuf<unsigned> tile_sum;
+    DevBuf<unsigned> tile_sum, tile_steps;
     DevBuf<unsigned short> d_amp;
     DevBuf<long long> d_base;
     try {
-        EDGPU_CUDA(cudaMalloc(&S.counts, std::max<size_t>((size_t)n_pass * sp.dim, 16)));
-        EDGPU_CUDA(cudaMalloc(&S.off, std::max<size_t>((size_t)n_pass * n_tiles * 4, 16)));
+        EDGPU_CUDA(cudaMalloc(&S.off, n_off * 4));
+        EDGPU_CUDA(cudaMalloc(&S.moff, n_off * 4));
         tile_sum.ensure((size_t)n_pass * n_tiles);
+        tile_steps.ensure((size_t)n_pass * n_tiles);
         if (scaled) {
             EDGPU_CUDA(cudaMalloc(&S.cls, (size_t)sp.dim));
             S.xsc.ensure(2 * (size_t)sp.dim);
         }
         sb.cls = S.cls;
-        sb.counts = S.counts;
         sb.tile_sum = tile_sum.p;
-        hx_slab_build(sp.w32, prec, 1, p, sb, (size_t)sb.o_ctr + (size_t)n_pass * HX_THREADS, st);
-        std::vector<unsigned long long> totals;
+        sb.tile_steps = tile_steps.p;
+        hx_slab_build(sp.w32, prec, 1, p, sb, st);
+        std::vector<unsigned long long> totals, steps;
         hx_slab_scan(tile_sum.p, S.off, n_pass, n_tiles, totals, st);
-        S.base.assign((size_t)n_pass + 1, 0);
+        hx_slab_scan(tile_steps.p, S.moff, n_pass, n_tiles, steps, st);
+        S.n = 0;
+        int64_t n_steps = 0;
         for (int q = 0; q < n_pass; ++q) {
-            require(totals[q] < ((unsigned long long)1 << 32), EDGPU_ERR_ARG, "slab pass with 2^32 entries or more");
-            S.base[q + 1] = S.base[q] + (long long)totals[q];
+            S.n += (int64_t)totals[q];
+            n_steps += (int64_t)steps[q];
+            require(totals[q] < ((unsigned long long)1 << 32) && steps[q] < ((unsigned long long)1 << 32),
+                    EDGPU_ERR_ARG, "slab pass with 2^32 entries or more");
         }
-        S.n = S.base[n_pass];
-        if ((double)meta + (double)S.n * 4.0 > (double)max_bytes) {
+        // padded or with masks
+        constexpr int PAD = 2 * 128;   // entries after a padded pass: the product reads two groups ahead
+        S.padded = pad_id && (double)n_steps * 32.0 <= SLAB_PAD_MOST * (double)S.n &&
+                   (double)meta + ((double)n_steps * 32.0 + (double)PAD * n_pass) * 4.0 <= (double)max_bytes;
+        S.tile_steps = (int)(n_steps / ((int64_t)n_pass * n_tiles));
+        S.base.assign((size_t)n_pass + 1, 0);
+        S.mbase.assign((size_t)n_pass + 1, 0);
+        for (int q = 0; q < n_pass; ++q) {
+            // (with masks one padding entry ends every pass)
+            S.base[q + 1] = S.base[q] + (S.padded ? (long long)steps[q] * 32 + PAD : ((long long)totals[q] + 4) / 4 * 4);
+            S.mbase[q + 1] = S.mbase[q] + (S.padded ? 0 : (long long)steps[q]);
+        }
+        const long long n_entries = S.base[n_pass], n_masks = S.mbase[n_pass];
+        if ((double)meta + ((double)n_entries + (double)n_masks) * 4.0 > (double)max_bytes) {
             op->free_slabs();
             return EDGPU_OK;
         }
-        EDGPU_CUDA(cudaMalloc(&S.tab, std::max<size_t>((size_t)S.n * 4, 16)));
+        EDGPU_CUDA(cudaMalloc(&S.tab, std::max<size_t>((size_t)n_entries * 4, 16)));
+        if (!S.padded) {
+            EDGPU_CUDA(cudaMalloc(&S.mask, std::max<size_t>((size_t)n_masks * 4, 16)));
+        }
+        for (int q = 0; q < n_pass; ++q) {   // after a pass: entries without effect on the slab's first column
+            const long long used = S.padded ? (long long)steps[q] * 32 : (long long)totals[q];
+            const std::vector<unsigned> fill((size_t)(S.base[q + 1] - S.base[q] - used),
+                                             S.padded ? (unsigned)n_ids << colbits : 0u);
+            EDGPU_CUDA(cudaMemcpy(S.tab + S.base[q] + used, fill.data(), fill.size() * 4, cudaMemcpyHostToDevice));
+        }
+        sb.padded = S.padded;
+        sb.n_ids = (int)n_ids;
         d_amp.ensure((size_t)n_slots);
-        d_base.ensure((size_t)n_pass);
+        d_base.ensure(2 * (size_t)n_pass);
         EDGPU_CUDA(cudaMemcpyAsync(d_amp.p, amp_id.data(), (size_t)n_slots * 2, cudaMemcpyHostToDevice, st));
         EDGPU_CUDA(cudaMemcpyAsync(d_base.p, S.base.data(), (size_t)n_pass * 8, cudaMemcpyHostToDevice, st));
+        EDGPU_CUDA(cudaMemcpyAsync(d_base.p + n_pass, S.mbase.data(), (size_t)n_pass * 8, cudaMemcpyHostToDevice, st));
         sb.off = S.off;
+        sb.moff = S.moff;
         sb.base = d_base.p;
+        sb.mbase = d_base.p + n_pass;
         sb.tab = S.tab;
+        sb.mask = S.mask;
         sb.amp_id = d_amp.p;
-        hx_slab_build(sp.w32, prec, 2, p, sb, (size_t)sb.o_ctr + (size_t)n_pass * HX_THREADS * 4, st);
+        hx_slab_build(sp.w32, prec, 2, p, sb, st);
         EDGPU_CUDA(cudaStreamSynchronize(st));
         S.n_pass = n_pass;
         S.wc = wc;
@@ -2622,7 +2667,7 @@ int edgpu_op_autotune(edgpu_op oh, int32_t precision, int32_t* rows_per_tile_out
     const bool mapped = op->space->d_map != nullptr;
     if (pair_ok) {
         if (op->slab.tab)
-            for (int hint : {0, 1, 2, 3, 4, 5}) cands.push_back({1, 4, 1, -1, 0, 0, 1, hint});
+            cands.push_back({1, 4, 1, -1, 0, 0, 1, 0});
         if (op->d_tab) {
             for (int nt : {8, 4, 2})
                 for (int pf : {0, 4, 64}) cands.push_back({1, nt, 1, -1, pf, 0});

@@ -343,31 +343,42 @@ void hx_adj_launch(bool w32, int prec, const HxParams& p, size_t smem, cudaStrea
 // ---- column-slab table of the pair-flip schedule (hxslab.cu) -------------------------------------
 // The target table's entries regrouped by column slab: slab q holds the columns [q wc, (q + 1) wc).
 // Pass q of the product gathers only from slab q (sized to stay in L2 while the pass runs) and adds
-// its share to y.  Per pass: a count byte per row, a 32-bit offset per warp tile of 32 rows
-// (relative to the pass's first entry), and the entries tile by tile, row by row, each row's
-// entries in the target table's order; an entry is (column - q wc) | id << colbits, where id
-// indexes the coefficient table: id = ((amplitude id x den + character index) x nd + orbit-size
-// index of the row) x nd + orbit-size index of the column.
+// its share to y.  Within a pass and a warp tile of 32 rows the entries lie in steps of at most one entry
+// per row: per tile as many as the row with the most entries, rounded up to a multiple of four.  An entry
+// is (column - q wc) | id << colbits.  Two forms: padded, 32 entries per step (a row without one has a
+// padding entry of id n_ids), four steps of a row side by side; or per step a 32-bit mask of the rows that
+// have an entry, and their entries in row order.  Per pass and tile a 32-bit offset of its first step and
+// (with masks) of its first entry, relative to the pass ([n_tiles + 1], the last one the total).
+// id indexes the coefficient table: id = ((amplitude id x den + character index) x nd +
+// orbit-size index of the row) x nd + orbit-size index of the column.
 struct SlabBuild {
     long long wc;                   // columns per slab
     int n_pass;
     long long n_tiles;
-    unsigned char* counts;          // [n_pass][n_rows] (written by the count pass)
-    unsigned* tile_sum;             // [n_pass][n_tiles] (written by the count pass)
-    const unsigned* off;            // [n_pass][n_tiles] tile offsets relative to the pass (fill pass)
+    unsigned* tile_sum;             // [n_pass][n_tiles] entries (written by the count pass)
+    unsigned* tile_steps;           // [n_pass][n_tiles] steps (written by the count pass)
+    const unsigned* off;            // [n_pass][n_tiles + 1] first entries relative to the pass (fill pass)
+    const unsigned* moff;           // [n_pass][n_tiles + 1] first steps relative to the pass (fill pass)
     const long long* base;          // [n_pass] first entry of each pass (fill pass)
+    const long long* mbase;         // [n_pass] first step of each pass (fill pass)
     unsigned* tab;                  // the entries (fill pass)
+    unsigned* mask;                 // the steps' row masks (fill pass)
     const unsigned short* amp_id;   // [n_slots] amplitude id of every pair-flip slot (fill pass)
     unsigned char* cls;             // [n_rows] every row's orbit-size index (count pass; null: not kept)
     int n_slots;
     int colbits;
     int scaled;                     // ids without the orbit-size indices (amplitude id x den + character)
-    int o_ctr;                      // shared-memory offset of the per-thread pass counters / cursors
+    int padded;                     // every step has 32 entries (no masks)
+    int n_ids;                      // coefficient ids (a padding entry has the id n_ids)
+    int cap;                        // steps a warp of the fill pass lays out at a time (>= the most of one tile)
+    int o_scratch;                  // shared-memory offset of the passes' scratch
 };
 struct SlabRun {
-    const unsigned char* cnt;       // this pass's count bytes [n_rows]
-    const unsigned* off;            // this pass's tile offsets [n_tiles]
+    const unsigned* off;            // this pass's first entries by tile [n_tiles + 1]
+    const unsigned* moff;           // this pass's first steps by tile [n_tiles + 1]
     const unsigned* tab;            // this pass's entries
+    const unsigned* mask;           // this pass's steps (null on a padded table)
+    int padded;
     const void* xs;                 // x from the slab's first column
     const void* x;                  // x (first pass: the diagonal's product)
     void* y;
@@ -378,9 +389,7 @@ struct SlabRun {
     unsigned colmask;
     int colbits, n_lut, lut_real;
     int first, last, accumulate, acc_c128;
-    int hints;                      // 0 to 3: one lane per row (bit 0: gathers cached in L2 only,
-                                    // streamed data evict-first; bit 1: eight entries per lane and step
-                                    // instead of four); 4, 5: two, four lanes per row
+    int tile_steps;                 // mean steps of a tile in a pass
     int lut_mode;                   // 0: one shared-memory copy of the coefficients; 1: a copy per
                                     // bank group (conflict-free lookups); 2: real, at most 4, in registers
     // scaled tables: xs and x hold sqrt(|O_c|) x_c; the last pass multiplies row r by 1/sqrt(|O_r|)
@@ -390,8 +399,14 @@ struct SlabRun {
     const void* scale;              // R[2 nd]: sqrt(|O|) by orbit-size index, then 1 / sqrt(|O|)
     int nd;
     long long tile0;                // the launch covers the tiles [tile0, tile0 + n_tiles)
+    int chunk;                      // consecutive tiles of a warp (set by hx_slab_launch)
     int blocks_per_sm;              // 0: as many as fit; > 0: at most that many; < 0: leave -blocks_per_sm free
 };
+// A table is padded (32 entries in every step, no masks) where that takes at most this many entries per
+// target: the padded product takes a third of the instructions per step (4x8: 1.72 against 2.16 ms, 6x5:
+// 0.68 against 0.75 ms), and one pass over a sector needs 1.1 to 1.4; at 18 passes of a few entries per
+// row it is above 2, which would double the memory of the largest tables.
+constexpr double SLAB_PAD_MOST = 1.5;
 // Coefficient tables of at most this many entries go to registers (real) or to one copy per shared-
 // memory bank group (SLAB_REP_BYTES in all, which keeps eight blocks of the slab kernel per SM).
 constexpr int SLAB_REG_LUT = 4;
@@ -404,11 +419,10 @@ void launch_slab_xscale(int prec, const void* x, const unsigned char* cls, const
 void launch_slab_xscale_c128_c64(const double* x, const unsigned char* cls, const float* scale, float* out,
                                  int64_t c0, int64_t c1, cudaStream_t st);
 // Count pass (1) or fill pass (2) of the slab table from the target table.  p: the table-flavour
-// pair-flip template (tab, tile_off set; lpr = 1); smem: its image plus s.o_ctr's counters.
-void hx_slab_build(bool w32, int prec, int pass, const HxParams& p, const SlabBuild& s, size_t smem,
-                   cudaStream_t st);
+// pair-flip template (tab, tile_off set; lpr = 1), whose image ends at s.o_scratch.
+void hx_slab_build(bool w32, int prec, int pass, const HxParams& p, const SlabBuild& s, cudaStream_t st);
 // Per pass: exclusive scan of the tile sums [n_pass][n_tiles] into 32-bit offsets relative to the
-// pass; totals[q] = entries of pass q (host, after a synchronisation).
+// pass [n_pass][n_tiles + 1]; totals[q] = sum of pass q (host, after a synchronisation).
 void hx_slab_scan(const unsigned* tile_sum, unsigned* off, int n_pass, long long n_tiles,
                   std::vector<unsigned long long>& totals, cudaStream_t st);
 // One pass of the slab product.

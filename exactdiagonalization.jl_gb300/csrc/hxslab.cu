@@ -10,49 +10,100 @@
 // The entries are those of the target table (itself the (row, target) form of the reference's
 // basis_mapping_index, symmetry_reduce_generic.jl:33-35), with the coefficient of each element
 // (amplitude x character x orbit-size ratio, reduced_operator_representation.jl:57-85) replaced by an
-// index into a small table of the distinct coefficients.  Within a pass every row adds its entries
-// in the target table's order and the passes are added in order, so results are reproducible run to
-// run; they differ from the one-pass product by the order of the additions.  A scaled table's index
-// leaves the orbit-size ratio sqrt(|O_c| / |O_r|) out: x is scaled by sqrt(|O_c|) before the passes
-// (k_slab_xscale) and each row's result by 1 / sqrt(|O_r|) in the last pass.
+// index into a small table of the distinct coefficients.  Within a pass and a warp tile of 32 rows they
+// are laid out in steps of at most one entry per row, so that the lanes of a warp read neighbouring
+// entries and, because the targets of one bond are kept together, gather from few lines of x
+// (hx_slab_fill_kernel).  Within a pass every row adds its entries in a fixed order and the passes are
+// added in order, so results are reproducible run to run; they differ from the one-pass product by the
+// order of the additions.  A scaled table's index leaves the orbit-size ratio sqrt(|O_c| / |O_r|) out: x
+// is scaled by sqrt(|O_c|) before the passes (k_slab_xscale) and each row's result by 1 / sqrt(|O_r|) in
+// the last pass.
+//
+// What bounds the product, and what the steps gave (complex64, H x in device time, before -> now;
+// before, every lane walked its own row's run of entries): triangular 6x5, 5.2 million rows, one pass,
+// 1167 -> 685 us; square 4x8, 18.8 million rows, two passes, 2960 -> 1750 us; square 6x6, 252 million
+// rows, 18 passes, 70.6 -> 63.9 ms; chain L = 24, 112,720 rows, 5.5 -> 5.1 us.  It was bound by the L1
+// data pipe (every entry load and every gather a line of its own); now a gather touches 0.2 (chains) to
+// 0.4 (tori) lines per entry, and the L1 tag lookups of those lines and the L2 requests behind them
+// share the limit.  In FP64 the FP64 pipe sets the pace, before and now (chain L = 28 107.6 -> 107.8 us,
+// 6x6 130 -> 131.5 ms): a double-precision FMA occupies it for 16 cycles of an SM per warp, so the mean
+// filling of the steps counts there.
 #include "hx_bond.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace edgpu {
 
 namespace {
 
-// Calls f(slot, c, sx, g) for every target of the row state b in the target table's order (class,
-// then start bit), reading the entries from position tpos on; slot = (class n + i) << 2 | v.
-template <typename W, int PREC, typename F>
-__device__ __forceinline__ void slab_walk(const HxParams& p, const BondTables<W, PREC>& bt,
-                                          const RowsSector<PREC>& sc, W b, long long tpos, F&& f) {
-    const int n = p.nbits;
-    const W full = (W)p.full;
-    for (int cls = 0; cls < p.bond_ncls; ++cls) {
-        W m = bond_class_mask<W, PREC>(b, bt, cls, n, full);
-        const bool cpar = (bt.ninfo[cls] >> 8) != 0;
-        while (m) {
-            const int i = lowest_bit<W>(m);
-            m &= m - 1;
-            const int ti = cls * n + i;
-            int v = (int)(b >> i) & 1;
-            if (cpar) v |= (__popcll((unsigned long long)(b & bt.flip[ti])) != 1) << 1;
+// Shared-memory scratch of the fill pass: words per warp, and the most bytes of a block.
+__host__ __device__ constexpr size_t slab_fill_words(int cap, int n_pass) { return (size_t)33 * cap + n_pass + 1; }
+constexpr size_t SLAB_FILL_SMEM = 200 * 1024;
+
+// Pass 1 counts every tile's entries and steps per slab: a step holds at most one entry of a row, so a
+// tile has as many steps as the row with the most entries (rounded up to a multiple of four).
+template <typename W, int PREC>
+__global__ void __launch_bounds__(HX_THREADS) hx_slab_count_kernel(const HxParams p, const SlabBuild s) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    {
+        const int4* src = (const int4*)p.blob;
+        int4* dst = (int4*)sm;
+        for (int i = threadIdx.x; i < p.blob_words16; i += blockDim.x) dst[i] = src[i];
+    }
+    __syncthreads();
+    const BondTables<W, PREC> bt(p, sm);
+    RowsSector<PREC> sc{};
+    sc.tab = p.tab;
+    sc.tile_off = p.tile_off;
+    sc.tab_wide = p.tab_wide;
+    sc.tab_cb = p.tab_cb;
+    const W* __restrict__ keys = (const W*)p.keys;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+    const W smask = (W)((((W)1) << p.sb) - 1);
+    const unsigned wc = (unsigned)s.wc;
+    unsigned char* ctr = sm + s.o_scratch;   // [n_pass][thread]
+    for (long long tile = (long long)blockIdx.x * wpb + warp; tile < s.n_tiles; tile += (long long)gridDim.x * wpb) {
+        const long long row = tile * 32 + lane;
+        const bool act = row < p.n_rows;
+        const W kr = act ? keys[row] : (W)0;
+        const int cnt = bond_row_count<W, PREC>(kr >> p.sb, bt, act ? p.bond_ncls : 0, p.nbits, (W)p.full);
+        int incl = cnt;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += u;
+        }
+        const long long tpos = p.tile_off[tile] + (incl - cnt);
+        if (s.cls && act) s.cls[row] = (unsigned char)(kr & smask);
+        for (int q = 0; q < s.n_pass; ++q) ctr[q * HX_THREADS + threadIdx.x] = 0;
+        for (int t = 0; t < cnt; ++t) {
             long long c;
             int sx, g;
-            table_entry<PREC>(sc, tpos, true, p.sb, c, sx, g);
-            ++tpos;
-            f((ti << 2) | v, c, sx, g);
+            table_entry<PREC>(sc, tpos + t, true, p.sb, c, sx, g);
+            if (c >= 0) ++ctr[((unsigned)c / wc) * HX_THREADS + threadIdx.x];
+        }
+        for (int q = 0; q < s.n_pass; ++q) {
+            const unsigned v = ctr[q * HX_THREADS + threadIdx.x];
+            const unsigned sum = __reduce_add_sync(0xffffffffu, v), most = __reduce_max_sync(0xffffffffu, v);
+            if (lane == 0) {
+                s.tile_sum[(size_t)q * s.n_tiles + tile] = sum;
+                s.tile_steps[(size_t)q * s.n_tiles + tile] = (most + 3u) & ~3u;
+            }
         }
     }
 }
 
-// Pass 1 counts every row's targets per slab (counts[q][row], tile sums); pass 2 writes every entry
-// at its place (a per-thread cursor per slab, started at the tile's offset plus the counts of the
-// tile's earlier rows).
-template <typename W, int PREC, int PASS>
-__global__ void __launch_bounds__(HX_THREADS) hx_slab_build_kernel(const HxParams p, const SlabBuild s) {
+// Pass 2 lays out every tile's steps and writes their row masks and entries.  The targets of one bond
+// pair, of the tile's rows that have one in the slab, are placed together: into the step where most of
+// these rows are still free, what is left of them into the next best, and so on (a row's entries fit,
+// whatever their order, because the tile has a step for each).  Neighbouring rows' targets by one bond
+// are often neighbours too (they are when the targets are representatives themselves), so a step's
+// gathers share lines of x; taking every row's next entry instead touches 1.3 to 1.5 times the lines.
+// One warp per tile; scratch: per warp s.cap steps of 32 entries, their masks and the slabs' first
+// steps; the slabs are taken in runs whose steps fit there.
+template <typename W, int PREC>
+__global__ void __launch_bounds__(HX_THREADS) hx_slab_fill_kernel(const HxParams p, const SlabBuild s) {
     extern __shared__ __align__(16) unsigned char sm[];
     {
         const int4* src = (const int4*)p.blob;
@@ -69,61 +120,121 @@ __global__ void __launch_bounds__(HX_THREADS) hx_slab_build_kernel(const HxParam
     const int* num = (const int*)(sm + p.o_num);
     const W* __restrict__ keys = (const W*)p.keys;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+    const unsigned below = (1u << lane) - 1u;
     const W smask = (W)((((W)1) << p.sb) - 1);
+    const W full = (W)p.full;
+    const int n = p.nbits;
     const unsigned wc = (unsigned)s.wc;
-    const int P = s.n_pass;
+    const size_t stride = (size_t)s.n_tiles + 1;   // of the tile offsets of one pass
+    unsigned* ent = (unsigned*)(sm + s.o_scratch) + (size_t)warp * slab_fill_words(s.cap, s.n_pass);
+    unsigned* occ = ent + 32 * s.cap;   // row masks of the steps
+    unsigned* first = occ + s.cap;      // [n_pass + 1] first step of each slab of the run
     for (long long tile = (long long)blockIdx.x * wpb + warp; tile < s.n_tiles; tile += (long long)gridDim.x * wpb) {
         const long long row = tile * 32 + lane;
         const bool act = row < p.n_rows;
         const W kr = act ? keys[row] : (W)0;
         const W b = kr >> p.sb;
         const int ri = (int)(kr & smask);
-        const int cnt = bond_row_count<W, PREC>(b, bt, act ? p.bond_ncls : 0, p.nbits, (W)p.full);
+        const int cnt = bond_row_count<W, PREC>(b, bt, act ? p.bond_ncls : 0, n, full);
         int incl = cnt;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const int u = __shfl_up_sync(0xffffffffu, incl, d);
             if (lane >= d) incl += u;
         }
-        const long long tpos = p.tile_off[tile] + (incl - cnt);
-        if constexpr (PASS == 1) {
-            if (s.cls && act) s.cls[row] = (unsigned char)ri;
-            unsigned char* ctr = sm + s.o_ctr;
-            for (int q = 0; q < P; ++q) ctr[q * HX_THREADS + threadIdx.x] = 0;
-            if (act)
-                slab_walk<W, PREC>(p, bt, sc, b, tpos, [&](int, long long c, int, int) {
-                    if (c >= 0) ++ctr[((unsigned)c / wc) * HX_THREADS + threadIdx.x];
-                });
-            for (int q = 0; q < P; ++q) {
-                const unsigned v = ctr[q * HX_THREADS + threadIdx.x];
-                if (act) s.counts[(size_t)q * p.n_rows + row] = (unsigned char)v;
-                unsigned t = v;
-#pragma unroll
-                for (int d = 16; d > 0; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
-                if (lane == 0) s.tile_sum[(size_t)q * s.n_tiles + tile] = t;
+        const long long tpos0 = p.tile_off[tile] + (incl - cnt);
+        for (int qa = 0; qa < s.n_pass;) {
+            // the run of slabs [qa, qb) whose steps fit in the scratch (a slab's always do)
+            int qb = qa;
+            unsigned used = 0;
+            __syncwarp();
+            for (; qb < s.n_pass; ++qb) {
+                const unsigned* mo = s.moff + qb * stride + tile;
+                const unsigned S = mo[1] - mo[0];
+                if (used + S > (unsigned)s.cap) break;
+                if (lane == 0) first[qb - qa] = used;
+                used += S;
             }
-        } else {
-            unsigned* cur = (unsigned*)(sm + s.o_ctr);
-            for (int q = 0; q < P; ++q) {
-                const unsigned v = act ? s.counts[(size_t)q * p.n_rows + row] : 0u;
-                unsigned inc = v;
-#pragma unroll
-                for (int d = 1; d < 32; d <<= 1) {
-                    const unsigned u = __shfl_up_sync(0xffffffffu, inc, d);
-                    if (lane >= d) inc += u;
+            if (lane == 0) first[qb - qa] = used;
+            for (unsigned j = lane; j < used; j += 32) occ[j] = 0u;
+            __syncwarp();
+            long long tpos = tpos0;
+            for (int cls = 0; cls < p.bond_ncls; ++cls) {
+                const W m = act ? bond_class_mask<W, PREC>(b, bt, cls, n, full) : (W)0;
+                const bool cpar = (bt.ninfo[cls] >> 8) != 0;
+                W u = warp_or<W>(m);
+                while (u) {
+                    const int i = lowest_bit<W>(u);
+                    u &= u - 1;
+                    const bool on = (m >> i) & 1;
+                    const int ti = cls * n + i;
+                    int v = (int)(b >> i) & 1;
+                    if (cpar) v |= (__popcll((unsigned long long)(b & bt.flip[ti])) != 1) << 1;
+                    long long c;
+                    int sx, g;
+                    table_entry<PREC>(sc, tpos, on, p.sb, c, sx, g);
+                    tpos += on ? 1 : 0;
+                    const bool has = on && c >= 0;
+                    const int q = has ? (int)((unsigned)c / wc) : -1;
+                    unsigned entry = 0;
+                    if (has) {
+                        const unsigned ph = p.want_arg ? (unsigned)num[g] : 0u;
+                        const unsigned ap = (unsigned)__ldg(s.amp_id + ((ti << 2) | v)) * (unsigned)p.den + ph;
+                        const unsigned id = s.scaled ? ap : (ap * (unsigned)p.nd + (unsigned)ri) * (unsigned)p.nd + (unsigned)sx;
+                        entry = ((unsigned)c - (unsigned)q * wc) | (id << s.colbits);
+                    }
+                    unsigned pending = __ballot_sync(0xffffffffu, q >= qa && q < qb);
+                    while (pending) {
+                        const int q0 = __shfl_sync(0xffffffffu, q, __ffs((int)pending) - 1);
+                        unsigned rest = __ballot_sync(0xffffffffu, q == q0);
+                        pending &= ~rest;
+                        const unsigned f0 = first[q0 - qa], S = first[q0 - qa + 1] - f0;
+                        while (rest) {
+                            // the step with the most of these rows free (the lowest of them)
+                            unsigned best = 0;
+                            for (unsigned k = lane; k < S; k += 32)
+                                best = max(best, ((unsigned)__popc(rest & ~occ[f0 + k]) << 16) | (0xffffu - k));
+                            best = __reduce_max_sync(0xffffffffu, best);
+                            const unsigned k = f0 + (0xffffu - (best & 0xffffu));
+                            const unsigned o = occ[k], got = rest & ~o;
+                            if ((got >> lane) & 1u) ent[k * 32 + lane] = entry;
+                            __syncwarp();
+                            if (lane == 0) occ[k] = o | got;
+                            __syncwarp();
+                            rest &= ~got;
+                        }
+                    }
                 }
-                cur[q * HX_THREADS + threadIdx.x] = s.off[(size_t)q * s.n_tiles + tile] + (inc - v);
             }
-            if (act)
-                slab_walk<W, PREC>(p, bt, sc, b, tpos, [&](int slot, long long c, int sx, int g) {
-                    if (c < 0) return;
-                    const unsigned q = (unsigned)c / wc;
-                    const unsigned rel = cur[q * HX_THREADS + threadIdx.x]++;
-                    const unsigned ph = p.want_arg ? (unsigned)num[g] : 0u;
-                    const unsigned ap = (unsigned)__ldg(s.amp_id + slot) * (unsigned)p.den + ph;
-                    const unsigned id = s.scaled ? ap : (ap * (unsigned)p.nd + (unsigned)ri) * (unsigned)p.nd + (unsigned)sx;
-                    s.tab[s.base[q] + rel] = ((unsigned)c - q * wc) | (id << s.colbits);
-                });
+            for (int q = qa; q < qb; ++q) {
+                const unsigned f0 = first[q - qa], S = first[q - qa + 1] - f0;
+                if (s.padded) {
+                    // 32 entries a step, four steps of a lane side by side; a row without one gets a padding
+                    // entry on the column of another row's in the step
+                    const unsigned pad = (unsigned)s.n_ids << s.colbits, colmask = (1u << s.colbits) - 1u;
+                    uint4* tab = (uint4*)(s.tab + s.base[q] + (size_t)s.moff[q * stride + tile] * 32) + lane;
+                    for (unsigned k = 0; k < S; k += 4, tab += 32) {
+                        unsigned v[4];
+                        for (int h = 0; h < 4; ++h) {
+                            const unsigned o = occ[f0 + k + h];
+                            const int src = o ? __ffs((int)o) - 1 : 0;
+                            v[h] = (o >> lane) & 1u ? ent[(f0 + k + h) * 32 + lane]
+                                                    : pad | (o ? ent[(f0 + k + h) * 32 + src] & colmask : 0u);
+                        }
+                        *tab = make_uint4(v[0], v[1], v[2], v[3]);
+                    }
+                    continue;
+                }
+                unsigned* tab = s.tab + s.base[q] + s.off[q * stride + tile];
+                unsigned* mask = s.mask + s.mbase[q] + s.moff[q * stride + tile];
+                for (unsigned k = lane; k < S; k += 32) mask[k] = occ[f0 + k];
+                for (unsigned k = 0; k < S; ++k) {
+                    const unsigned o = occ[f0 + k];
+                    if ((o >> lane) & 1u) tab[__popc(o & below)] = ent[(f0 + k) * 32 + lane];
+                    tab += __popc(o);
+                }
+            }
+            qa = qb;
         }
     }
 }
@@ -165,7 +276,7 @@ __global__ void k_slab_scan_out(const unsigned* ts, long long n_tiles, const uns
     __shared__ long long tmp[32];
     const int q = blockIdx.y;
     const unsigned* a = ts + (size_t)q * n_tiles;
-    unsigned* o = off + (size_t)q * n_tiles;
+    unsigned* o = off + (size_t)q * (n_tiles + 1);
     const long long beg = (long long)blockIdx.x * SLAB_CHUNK + (long long)threadIdx.x * 16;
     const long long end = min(n_tiles, beg + 16);
     long long s = 0;
@@ -175,6 +286,7 @@ __global__ void k_slab_scan_out(const unsigned* ts, long long n_tiles, const uns
         o[i] = (unsigned)ex;
         ex += a[i];
     }
+    if (beg < n_tiles && end == n_tiles) o[n_tiles] = (unsigned)ex;   // the pass's total
 }
 
 // acc += c x with explicit fused multiply-adds (the same roundings in every kernel of this file)
@@ -187,156 +299,241 @@ __device__ __forceinline__ V cfma_acc(V acc, V c, V x) {
     return acc;
 }
 
-// Loads and stores with or without cache hints (CH): the gathers of x cached in L2 only (they have
-// no reuse in L1), the streamed count bytes, offsets and y marked evict-first, so that the slab of x
-// keeps its place in L2.
-template <bool CH, typename T>
-__device__ __forceinline__ T ld_gather(const T* p) {
-    if constexpr (CH) return __ldcg(p);
-    else return *p;
-}
-template <bool CH, typename T>
+// The entries, masks and y are read (and written) once per pass: evict-first, so that the slab of x
+// keeps its place in L1 and L2 (18.8 million rows in two passes: 2.00 -> 1.72 ms).
+template <typename T>
 __device__ __forceinline__ T ld_stream(const T* p) {
-    if constexpr (CH) return __ldcs(p);
-    else return *p;
+    return __ldcs(p);
 }
-template <bool CH, typename T>
+template <typename T>
 __device__ __forceinline__ void st_stream(T* p, T v) {
-    if constexpr (CH) __stcs(p, v);
-    else *p = v;
+    __stcs(p, v);
 }
 
-// One pass of the product: a warp per tile of 32 rows with one lane per row (LPR = 1), or per part of
-// 32 / LPR rows of a tile with LPR lanes per row (lane sub of a row takes the row's entries sub,
-// sub + LPR, ...; the partial sums are added by a fixed butterfly).  A lane adds its entries of this
-// pass (NT per step, loads then gathers); the row's sum is then added to y (the first pass writes it,
-// the last adds the diagonal term too and may write complex128 to y_c128 instead).  LUTM: where the
-// coefficients are read (SlabRun::lut_mode).
-template <int PREC, bool REAL, int NT, bool CH, int LPR, int LUTM>
-__global__ void __launch_bounds__(HX_THREADS) hx_slab_kernel(const SlabRun r) {
+// The masks of the steps [k, k + 4) (k a multiple of four), 0 from k1 on.
+__device__ __forceinline__ void ld_masks(const unsigned* __restrict__ mask, unsigned k, unsigned k1, unsigned* m) {
+    const uint4 v = k < k1 ? ld_stream((const uint4*)(mask + k)) : make_uint4(0u, 0u, 0u, 0u);
+    m[0] = v.x;
+    m[1] = v.y;
+    m[2] = v.z;
+    m[3] = v.w;
+}
+
+// This lane's entries of four steps with the row masks m, the first of them at e0 (moved past them);
+// below: the bits of the lanes before this one.  A lane without an entry reads that of the next row
+// that has one (every pass ends with a padding entry).
+__device__ __forceinline__ void ld_entries(const unsigned* __restrict__ tab, const unsigned* m, unsigned below,
+                                           unsigned& e0, unsigned* e) {
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        e[h] = ld_stream(tab + (e0 + (unsigned)__popc(m[h] & below)));
+        e0 += (unsigned)__popc(m[h]);
+    }
+}
+
+// Adds a row's sum over this pass to y; some: the row has entries in the pass.  Passes add their sums in
+// order: the first writes y, the last adds the diagonal term diag x too (so that a pass needs only its
+// own slab of x, the last one all of it) and may write complex128 to y_c128 instead.
+template <int PREC>
+__device__ __forceinline__ void finish_row(const SlabRun& r, long long row, typename Cx<PREC>::V acc, bool some) {
     typedef typename Cx<PREC>::V V;
     typedef typename Cx<PREC>::R R;
-    typedef typename std::conditional<REAL, R, V>::type C;
-    constexpr int REPS = 128 / (int)sizeof(C);   // copies per coefficient: one per bank group
+    if (row >= r.n_rows) return;
+    V* y = (V*)r.y;
+    V t;
+    if (r.first) {
+        if (r.accumulate) {
+            V yo = ld_stream(y + row);
+            if (r.scaled) {
+                // y += H x on a scaled table: the old y_r enters the row's scaled sum as sqrt(|O_r|) y_r
+                const R sr = __ldg((const R*)r.scale + r.cls[row]);
+                yo.x *= sr;
+                yo.y *= sr;
+            }
+            t = cadd(yo, acc);
+        } else {
+            t = acc;
+        }
+    } else {
+        if (!some && !r.last) return;   // nothing to add to this row
+        t = cadd(ld_stream(y + row), acc);
+    }
+    if (r.last) {
+        t = cfma_acc(t, ld_stream((const V*)r.diag + row), ld_stream((const V*)r.x + row));
+        if (r.scaled) {
+            const R rs = __ldg((const R*)r.scale + r.nd + r.cls[row]);
+            t.x *= rs;
+            t.y *= rs;
+        }
+    }
+    if (r.last && r.y_c128 != nullptr) {
+        double2 o = make_double2((double)t.x, (double)t.y);
+        double2* yc = (double2*)r.y_c128;
+        if (r.acc_c128) {
+            const double2 old = yc[row];
+            o.x += old.x;
+            o.y += old.y;
+        }
+        yc[row] = o;
+    } else {
+        st_stream(y + row, t);
+    }
+}
+
+// The coefficient table of a launch: in registers (LUTM 2: real, at most 4), or in shared memory, a copy
+// per bank group (1) or one (0), with room for the id after the last (a padding entry's).
+template <int PREC, bool REAL, int LUTM>
+struct SlabLut {
+    typedef typename Cx<PREC>::V V;
+    typedef typename Cx<PREC>::R R;
+    typedef typename std::conditional<REAL, R, V>::type T;
+    static constexpr int REPS = LUTM == 1 ? 128 / (int)sizeof(T) : 1;   // copies per coefficient
+    R c0 = 0, c1 = 0, c2 = 0, c3 = 0;
+    const T* sm;
+    __device__ __forceinline__ SlabLut(const SlabRun& r, unsigned char* smem) : sm((const T*)smem) {
+        const T* src = (const T*)r.lut;
+        if constexpr (LUTM == 2) {
+            const R* lr0 = (const R*)r.lut;
+            c0 = __ldg(lr0);
+            c1 = __ldg(lr0 + min(1, r.n_lut - 1));
+            c2 = __ldg(lr0 + min(2, r.n_lut - 1));
+            c3 = __ldg(lr0 + min(3, r.n_lut - 1));
+        } else if constexpr (LUTM == 1) {
+            for (int i = threadIdx.x; i < r.n_lut * REPS; i += blockDim.x) ((T*)smem)[i] = src[i / REPS];
+            __syncthreads();
+            sm += threadIdx.x & (REPS - 1);
+        } else {
+            for (int i = threadIdx.x; i < r.n_lut; i += blockDim.x) ((T*)smem)[i] = src[i];
+            __syncthreads();
+        }
+    }
+    __device__ __forceinline__ T operator()(unsigned id) const {
+        if constexpr (LUTM == 2) return (id & 2u) ? ((id & 1u) ? c3 : c2) : ((id & 1u) ? c1 : c0);
+        else return sm[id * REPS];
+    }
+};
+
+// acc += c x when e < lim (predicated, without a branch)
+__device__ __forceinline__ void fma_if(float2& a, float c, float2 x, unsigned e, unsigned lim) {
+    asm("{.reg .pred p; setp.lt.u32 p, %5, %6; @p fma.rn.f32 %0, %2, %3, %0; @p fma.rn.f32 %1, %2, %4, %1;}"
+        : "+f"(a.x), "+f"(a.y) : "f"(c), "f"(x.x), "f"(x.y), "r"(e), "r"(lim));
+}
+__device__ __forceinline__ void fma_if(double2& a, double c, double2 x, unsigned e, unsigned lim) {
+    asm("{.reg .pred p; setp.lt.u32 p, %5, %6; @p fma.rn.f64 %0, %2, %3, %0; @p fma.rn.f64 %1, %2, %4, %1;}"
+        : "+d"(a.x), "+d"(a.y) : "d"(c), "d"(x.x), "d"(x.y), "r"(e), "r"(lim));
+}
+__device__ __forceinline__ void fma_if(float2& a, float2 c, float2 x, unsigned e, unsigned lim) {
+    fma_if(a, c.x, x, e, lim);
+    fma_if(a, c.y, make_float2(-x.y, x.x), e, lim);
+}
+__device__ __forceinline__ void fma_if(double2& a, double2 c, double2 x, unsigned e, unsigned lim) {
+    fma_if(a, c.x, x, e, lim);
+    fma_if(a, c.y, make_double2(-x.y, x.x), e, lim);
+}
+
+// One pass of the product through a padded table: one lane per row, one warp per tile of 32 rows and
+// r.chunk consecutive tiles, four steps at a time: a lane's four entries are one 16-byte load.  While a
+// group's gathers are under way, the entries of the group after the next are read, on through the
+// warp's tiles.  Mixed precision: four partial sums per row, by the entry's place in its group (a row
+// of 93 terms is half as far from its 64-bit sum as with one).  FP64: a step without entries (the last ones of a tile may be) is not added up, since
+// the FP64 pipe sets the pace (a warp's double-precision FMA takes 16 cycles of an SM).
+template <int PREC, bool REAL, int LUTM>
+__global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_pad_kernel(const SlabRun r) {
+    typedef typename Cx<PREC>::V V;
     extern __shared__ __align__(16) unsigned char sm[];
     pdl_launch_dependents();
-    const C* src = (const C*)r.lut;
-    R c0 = 0, c1 = 0, c2 = 0, c3 = 0;
-    if constexpr (LUTM == 2) {
-        const R* lr0 = (const R*)r.lut;
-        c0 = __ldg(lr0);
-        c1 = __ldg(lr0 + min(1, r.n_lut - 1));
-        c2 = __ldg(lr0 + min(2, r.n_lut - 1));
-        c3 = __ldg(lr0 + min(3, r.n_lut - 1));
-    } else if constexpr (LUTM == 1) {
-        for (int i = threadIdx.x; i < r.n_lut * REPS; i += blockDim.x) ((C*)sm)[i] = src[i / REPS];
-        __syncthreads();
-    } else {
-        for (int i = threadIdx.x; i < r.n_lut; i += blockDim.x) ((C*)sm)[i] = src[i];
-        __syncthreads();
-    }
+    const SlabLut<PREC, REAL, LUTM> lut(r, sm);
     pdl_wait();
-    const C* lut = (const C*)sm;
+    const V* __restrict__ xs = (const V*)r.xs;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+    const unsigned lim = (unsigned)r.n_lut << r.colbits;   // padding entries: from here on
+    // (rows are below 2^32, so tiles below 2^27)
+    const unsigned tile_end = (unsigned)(r.tile0 + r.n_tiles), hop = gridDim.x * wpb * r.chunk;
+    for (unsigned c0 = (unsigned)r.tile0 + (blockIdx.x * wpb + warp) * r.chunk; c0 < tile_end; c0 += hop) {
+        unsigned tile = c0;
+        const unsigned t1 = min(c0 + r.chunk, tile_end);
+        unsigned q = r.moff[tile] >> 2, qt = r.moff[tile + 1] >> 2;   // groups of four steps
+        const uint4* __restrict__ tp = (const uint4*)r.tab + ((size_t)q * 32 + lane);
+        uint4 e = ld_stream(tp), en = ld_stream(tp + 32);
+        auto add = [&](V& acc, unsigned g, const V& x, bool may_be_empty) {
+            if (PREC == 0 && may_be_empty && !__any_sync(0xffffffffu, g < lim)) return;
+            fma_if(acc, lut(g >> r.colbits), x, g, lim);
+        };
+        for (; tile < t1; ++tile) {
+            const unsigned qn = tile + 1 < t1 ? r.moff[tile + 2] >> 2 : qt;
+            V acc = czero<V>(), acc1 = acc, acc2 = acc, acc3 = acc;
+            for (; q < qt; ++q) {
+                const V x0 = xs[e.x & r.colmask], x1 = xs[e.y & r.colmask];
+                const V x2 = xs[e.z & r.colmask], x3 = xs[e.w & r.colmask];
+                tp += 32;
+                const uint4 e2 = ld_stream(tp + 32);
+                add(acc, e.x, x0, false);
+                add(PREC == 0 ? acc : acc1, e.y, x1, true);
+                add(PREC == 0 ? acc : acc2, e.z, x2, true);
+                add(PREC == 0 ? acc : acc3, e.w, x3, true);
+                e = en;
+                en = e2;
+            }
+            if (PREC == 1) acc = cadd(cadd(acc, acc1), cadd(acc2, acc3));
+            finish_row<PREC>(r, (long long)tile * 32 + lane, acc, true);
+            qt = qn;
+        }
+    }
+}
+
+// The same through a table with masks (large sectors in many passes, where padding would double the
+// table: on 6x6 it would take 54 ms instead of 64, and 164 GB instead of 80): a lane finds its entry of a
+// step by counting the rows before it, and the pipeline reads the next group's entries and the masks
+// after those.
+template <int PREC, bool REAL, int LUTM>
+__global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_kernel(const SlabRun r) {
+    typedef typename Cx<PREC>::V V;
+    extern __shared__ __align__(16) unsigned char sm[];
+    pdl_launch_dependents();
+    const SlabLut<PREC, REAL, LUTM> lut(r, sm);
+    pdl_wait();
     const V* __restrict__ xs = (const V*)r.xs;
     const unsigned* __restrict__ tab = r.tab;
-    V* y = (V*)r.y;
+    const unsigned* __restrict__ mask = r.mask;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    const int sub = lane & (LPR - 1);
-    const int rep = lane & (REPS - 1);
-    const bool to_c128 = r.last && r.y_c128 != nullptr;
-    const long long n_parts = r.n_tiles * LPR;
-    for (long long part = (long long)blockIdx.x * wpb + warp; part < n_parts; part += (long long)gridDim.x * wpb) {
-        const long long tile = r.tile0 + part / LPR;
-        // the counts of the tile's 32 rows and their exclusive prefix
-        const long long row32 = tile * 32 + lane;
-        const int c32 = row32 < r.n_rows ? (int)ld_stream<CH>(r.cnt + row32) : 0;
-        int incl = c32;
+    const unsigned bit = 1u << lane, below = bit - 1u;
+    // (rows are below 2^32, so tiles below 2^27)
+    const unsigned tile_end = (unsigned)(r.tile0 + r.n_tiles), hop = gridDim.x * wpb * r.chunk;
+    for (unsigned c0 = (unsigned)r.tile0 + (blockIdx.x * wpb + warp) * r.chunk; c0 < tile_end; c0 += hop) {
+        unsigned tile = c0;
+        const unsigned t1 = min(c0 + r.chunk, tile_end);
+        unsigned e0 = ld_stream(r.off + tile);
+        unsigned k = r.moff[tile], kt = r.moff[tile + 1];
+        const unsigned k1 = r.moff[t1];   // the tiles' steps (each tile has a multiple of four)
+        unsigned m[4], mn[4], e[4];
+        ld_masks(mask, k, k1, m);
+        ld_masks(mask, k + 4, k1, mn);
+        ld_entries(tab, m, below, e0, e);
+        for (; tile < t1; ++tile) {
+            const unsigned kn = tile + 1 < t1 ? r.moff[tile + 2] : kt;
+            V acc = czero<V>();
+            unsigned rows_on = 0;   // rows of the tile with entries in this pass
+            for (; k < kt; k += 4) {
+                V xv[4];
+                unsigned id[4], mc[4];
 #pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int u = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= d) incl += u;
-        }
-        // this lane's row in the tile
-        const int rl = LPR == 1 ? lane : (int)(part % LPR) * (32 / LPR) + lane / LPR;
-        const int cnt = LPR == 1 ? c32 : __shfl_sync(0xffffffffu, c32, rl);
-        const int excl = LPR == 1 ? incl - c32 : __shfl_sync(0xffffffffu, incl - c32, rl);
-        const long long row = tile * 32 + rl;
-        const bool act = row < r.n_rows;
-        const long long start = (long long)ld_stream<CH>(r.off + tile) + excl;
-        V acc = czero<V>();
-        for (int j = sub; __any_sync(0xffffffffu, j < cnt); j += NT * LPR) {
-            unsigned e[NT];
-#pragma unroll
-            for (int h = 0; h < NT; ++h) e[h] = (j + h * LPR < cnt) ? __ldg(tab + start + j + h * LPR) : 0u;
-            V xv[NT];
-#pragma unroll
-            for (int h = 0; h < NT; ++h)
-                xv[h] = (j + h * LPR < cnt) ? ld_gather<CH>(xs + (e[h] & r.colmask)) : czero<V>();
-#pragma unroll
-            for (int h = 0; h < NT; ++h) {
-                if (j + h * LPR >= cnt) continue;
-                const unsigned id = e[h] >> r.colbits;
-                C f;
-                if constexpr (LUTM == 2) {
-                    f = (id & 2u) ? ((id & 1u) ? c3 : c2) : ((id & 1u) ? c1 : c0);
-                } else if constexpr (LUTM == 1) {
-                    f = lut[id * REPS + rep];
-                } else {
-                    f = lut[id];
+                for (int h = 0; h < 4; ++h) {
+                    xv[h] = xs[e[h] & r.colmask];
+                    id[h] = e[h] >> r.colbits;
+                    mc[h] = m[h];
+                    rows_on |= m[h];
+                    m[h] = mn[h];
                 }
-                if constexpr (REAL) {
-                    acc.x = fma_r(f, xv[h].x, acc.x);
-                    acc.y = fma_r(f, xv[h].y, acc.y);
-                } else {
-                    acc = cfma_acc(acc, f, xv[h]);
+                ld_entries(tab, m, below, e0, e);
+                ld_masks(mask, k + 8, k1, mn);
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    if (PREC == 0 && h > 0 && mc[h] == 0u) continue;
+                    fma_if(acc, lut(id[h]), xv[h], ~mc[h] & bit, 1u);
                 }
             }
-        }
-#pragma unroll
-        for (int d = 1; d < LPR; d <<= 1) {
-            acc.x += __shfl_xor_sync(0xffffffffu, acc.x, d);
-            acc.y += __shfl_xor_sync(0xffffffffu, acc.y, d);
-        }
-        if (!act || sub != 0) continue;
-        // passes add their sums in order; the last adds the diagonal term diag x (so that a pass needs
-        // only its own slab of x, the last one all of it)
-        V t;
-        if (r.first) {
-            if (r.accumulate) {
-                V yo = ld_stream<CH>(y + row);
-                if (r.scaled) {
-                    // y += H x on a scaled table: the old y_r enters the row's scaled sum as sqrt(|O_r|) y_r
-                    const R sr = __ldg((const R*)r.scale + r.cls[row]);
-                    yo.x *= sr;
-                    yo.y *= sr;
-                }
-                t = cadd(yo, acc);
-            } else {
-                t = acc;
-            }
-        } else {
-            if (cnt == 0 && !r.last) continue;   // nothing to add to this row
-            t = cadd(ld_stream<CH>(y + row), acc);
-        }
-        if (r.last) {
-            t = cfma_acc(t, ld_stream<CH>((const V*)r.diag + row), ld_stream<CH>((const V*)r.x + row));
-            if (r.scaled) {
-                const R rs = __ldg((const R*)r.scale + r.nd + r.cls[row]);
-                t.x *= rs;
-                t.y *= rs;
-            }
-        }
-        if (to_c128) {
-            double2 o = make_double2((double)t.x, (double)t.y);
-            double2* yc = (double2*)r.y_c128;
-            if (r.acc_c128) {
-                const double2 old = yc[row];
-                o.x += old.x;
-                o.y += old.y;
-            }
-            yc[row] = o;
-        } else {
-            st_stream<CH>(y + row, t);
+            finish_row<PREC>(r, (long long)tile * 32 + lane, acc, (rows_on & bit) != 0u);
+            kt = kn;
         }
     }
 }
@@ -388,43 +585,43 @@ void slab_pdl_launch(K kern, const SlabRun& r, int blocks, size_t smem, cudaStre
     EDGPU_CUDA(cudaLaunchKernelEx(&cfg, kern, r));
 }
 
+// Blocks of a launch over n_warps warps of work.
 template <typename K>
-int slab_blocks(K kern, size_t smem, long long n_tiles, int per_sm = 0) {
+int slab_blocks(K kern, size_t smem, long long n_warps, int per_sm = 0) {
     raise_smem_limit((const void*)kern, smem);
     int n = 0;
     EDGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, HX_THREADS, smem));
     if (per_sm > 0) n = std::min(n, per_sm);
     else if (per_sm < 0) n = std::max(1, n + per_sm);
-    const long long need = (n_tiles + HX_THREADS / 32 - 1) / (HX_THREADS / 32);
+    const long long need = (n_warps + HX_THREADS / 32 - 1) / (HX_THREADS / 32);
     return (int)std::max<long long>(1, std::min<long long>(need, (long long)std::max(1, n) * sm_count()));
 }
 
 template <typename W, int PREC>
-void slab_build_t(int pass, const HxParams& p, const SlabBuild& s, size_t smem, cudaStream_t st) {
-    const int blocks = (int)std::max<long long>(
-        1, std::min<long long>((s.n_tiles + HX_THREADS / 32 - 1) / (HX_THREADS / 32), (long long)sm_count() * 8));
-    if (pass == 1) {
-        auto k = hx_slab_build_kernel<W, PREC, 1>;
-        raise_smem_limit((const void*)k, smem);
-        k<<<blocks, HX_THREADS, smem, st>>>(p, s);
-    } else {
-        auto k = hx_slab_build_kernel<W, PREC, 2>;
-        raise_smem_limit((const void*)k, smem);
-        k<<<blocks, HX_THREADS, smem, st>>>(p, s);
-    }
+void slab_build_t(int pass, const HxParams& p, const SlabBuild& s, cudaStream_t st) {
+    int threads = HX_THREADS;
+    if (pass == 2)   // as many warps as have room for their scratch (one always has)
+        while (threads > 32 && (size_t)s.o_scratch + threads / 32 * slab_fill_words(s.cap, s.n_pass) * 4 > SLAB_FILL_SMEM)
+            threads /= 2;
+    const size_t smem = (size_t)s.o_scratch + (pass == 1 ? (size_t)s.n_pass * HX_THREADS
+                                                         : threads / 32 * slab_fill_words(s.cap, s.n_pass) * 4);
+    auto k = pass == 1 ? hx_slab_count_kernel<W, PREC> : hx_slab_fill_kernel<W, PREC>;
+    raise_smem_limit((const void*)k, smem);
+    const long long warps = threads / 32;
+    const int blocks = (int)std::max<long long>(1, std::min<long long>((s.n_tiles + warps - 1) / warps, (long long)sm_count() * 16));
+    k<<<blocks, threads, smem, st>>>(p, s);
     EDGPU_CUDA(cudaGetLastError());
 }
 
 }  // namespace
 
-void hx_slab_build(bool w32, int prec, int pass, const HxParams& p, const SlabBuild& s, size_t smem,
-                   cudaStream_t st) {
+void hx_slab_build(bool w32, int prec, int pass, const HxParams& p, const SlabBuild& s, cudaStream_t st) {
     if (w32) {
-        if (prec == 0) slab_build_t<unsigned, 0>(pass, p, s, smem, st);
-        else slab_build_t<unsigned, 1>(pass, p, s, smem, st);
+        if (prec == 0) slab_build_t<unsigned, 0>(pass, p, s, st);
+        else slab_build_t<unsigned, 1>(pass, p, s, st);
     } else {
-        if (prec == 0) slab_build_t<unsigned long long, 0>(pass, p, s, smem, st);
-        else slab_build_t<unsigned long long, 1>(pass, p, s, smem, st);
+        if (prec == 0) slab_build_t<unsigned long long, 0>(pass, p, s, st);
+        else slab_build_t<unsigned long long, 1>(pass, p, s, st);
     }
 }
 
@@ -454,48 +651,38 @@ void hx_slab_scan(const unsigned* tile_sum, unsigned* off, int n_pass, long long
     if (e != cudaSuccess) throw Error(EDGPU_ERR_CUDA, std::string("slab scan: ") + cudaGetErrorString(e));
 }
 
-template <int PREC, bool REAL, bool CH, int NT, int LPR>
-void slab_launch_m(const SlabRun& r, size_t smem, cudaStream_t st) {
-    if constexpr (REAL) {
-        if (r.lut_mode == 2) {
-            auto k = hx_slab_kernel<PREC, true, NT, CH, LPR, 2>;
-            slab_pdl_launch(k, r, slab_blocks(k, 0, r.n_tiles * LPR, r.blocks_per_sm), 0, st);
-            return;
-        }
-    }
-    if (r.lut_mode == 1) {
-        auto k = hx_slab_kernel<PREC, REAL, NT, CH, LPR, 1>;
-        slab_pdl_launch(k, r, slab_blocks(k, smem, r.n_tiles * LPR, r.blocks_per_sm), smem, st);
+template <int PREC, bool REAL, int LUTM>
+void slab_launch_k(const SlabRun& r, size_t smem, cudaStream_t st) {
+    const long long warps = (r.n_tiles + r.chunk - 1) / r.chunk;
+    if (r.padded) {
+        auto k = hx_slab_pad_kernel<PREC, REAL, LUTM>;
+        slab_pdl_launch(k, r, slab_blocks(k, smem, warps, r.blocks_per_sm), smem, st);
     } else {
-        auto k = hx_slab_kernel<PREC, REAL, NT, CH, LPR, 0>;
-        slab_pdl_launch(k, r, slab_blocks(k, smem, r.n_tiles * LPR, r.blocks_per_sm), smem, st);
+        auto k = hx_slab_kernel<PREC, REAL, LUTM>;
+        slab_pdl_launch(k, r, slab_blocks(k, smem, warps, r.blocks_per_sm), smem, st);
     }
 }
 
-template <int PREC, bool CH, int NT, int LPR>
-void slab_launch_t(const SlabRun& r, size_t smem, cudaStream_t st) {
-    if (r.lut_real) slab_launch_m<PREC, true, CH, NT, LPR>(r, smem, st);
-    else slab_launch_m<PREC, false, CH, NT, LPR>(r, smem, st);
-}
-
-// hints: 0 to 3 one lane per row (bit 0 the cache hints, bit 1 eight entries per lane and step
-// instead of four); 4 and 5: two and four lanes per row, four entries per lane and step
 template <int PREC>
 void slab_launch_p(const SlabRun& r, size_t smem, cudaStream_t st) {
-    switch (r.hints) {
-        case 0: slab_launch_t<PREC, false, 4, 1>(r, smem, st); break;
-        case 1: slab_launch_t<PREC, true, 4, 1>(r, smem, st); break;
-        case 2: slab_launch_t<PREC, false, 8, 1>(r, smem, st); break;
-        case 3: slab_launch_t<PREC, true, 8, 1>(r, smem, st); break;
-        case 4: slab_launch_t<PREC, false, 4, 2>(r, smem, st); break;
-        default: slab_launch_t<PREC, false, 4, 4>(r, smem, st); break;
+    if (r.lut_real) {
+        if (r.lut_mode == 2) slab_launch_k<PREC, true, 2>(r, 0, st);
+        else slab_launch_k<PREC, true, 0>(r, smem, st);
+    } else {
+        if (r.lut_mode == 1) slab_launch_k<PREC, false, 1>(r, smem, st);
+        else slab_launch_k<PREC, false, 0>(r, smem, st);
     }
 }
 
-void hx_slab_launch(int prec, const SlabRun& r, cudaStream_t st) {
-    if (r.n_tiles == 0) return;
+void hx_slab_launch(int prec, const SlabRun& run, cudaStream_t st) {
+    if (run.n_tiles == 0) return;
+    SlabRun r = run;
+    // Consecutive tiles of a warp: about 128 steps together (the pipeline fills once for them), but at
+    // least four chunks for every warp that fits, so that none is left with the last long one.
+    r.chunk = (int)std::max<long long>(1, std::min<long long>({16, 128 / std::max(1, r.tile_steps),
+                                                              r.n_tiles / ((long long)sm_count() * 48 * 4)}));
     const size_t csize = (size_t)(r.lut_real ? 1 : 2) * (prec == 0 ? 8 : 4);
-    const size_t smem = (size_t)r.n_lut * (r.lut_mode == 1 ? 128 : csize);
+    const size_t smem = (size_t)(r.n_lut + 1) * (r.lut_mode == 1 ? 128 : csize);   // (and a padding entry's id)
     if (prec == 0) slab_launch_p<0>(r, smem, st);
     else slab_launch_p<1>(r, smem, st);
 }

@@ -246,14 +246,8 @@ int edgpu_op_build_slabs(edgpu_op op, int64_t slab_bytes, int64_t max_bytes, int
 int edgpu_op_free_slabs(edgpu_op op);
 /* Slabs (passes), columns per slab and entries of the slab table; zeros without one. */
 int edgpu_op_slabs_info(edgpu_op op, int32_t* passes, int64_t* columns_per_slab, int64_t* entries);
-/* Whether products of this precision read the slab table, and how: use = 0 (no), or 1 + v for the
- * variant v = 0 to 5 sets it (1 to 6 need the table: EDGPU_ERR_STATE otherwise), -1 only queries;
- * *current = the setting.  v = 0 to 3: one lane per row (bit 0: cache hints, the gathers of x cached
- * in L2 only and the streamed counts, offsets and y evict-first; bit 1: eight entries per lane and
- * step instead of four), all four bit-identical; v = 4 and 5: two and four lanes per row (for sectors
- * too small to fill the GPU), whose partial sums are added in another fixed order, so their results
- * differ from v = 0 to 3 by rounding (each is deterministic).  Building the table sets 1 for both
- * precisions; the autotuner times the variants against the one-pass schedules. */
+/* Whether products of this precision read the slab table: use = 0 (no), or 1 to 6 (yes; one kernel
+ * serves them all, the value is kept for callers that set one); -1 only queries.  *current: the setting. */
 int edgpu_op_slab_use(edgpu_op op, int32_t precision, int32_t use, int32_t* current);
 /* Layout of the next slab table: mode 0 (default) scaled on sectors of 2^22 representatives or more
  * where that saves passes or the coefficients are complex (and wherever the unscaled ids do not fit in
