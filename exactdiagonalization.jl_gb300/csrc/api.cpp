@@ -260,6 +260,21 @@ struct edgpu_op_s {
         }
     }
     int slab_hint[2] = {0, 0};        // [precision]: the slab product's cache hints (chosen by the autotuner)
+    // Lanczos: pinned host memory the steps write their alpha, beta and norm to (three doubles a step and
+    // three more), and the events after which those of the even and odd steps are there
+    double* lz_slots = nullptr;
+    int lz_cap = 0;
+    cudaEvent_t lz_ev[2] = {nullptr, nullptr};
+    void ensure_lanczos_slots(int m) {
+        for (auto& e : lz_ev)
+            if (!e) EDGPU_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        if (m <= lz_cap) return;
+        if (lz_slots) cudaFreeHost(lz_slots);
+        lz_slots = nullptr;
+        lz_cap = 0;
+        EDGPU_CUDA(cudaHostAlloc((void**)&lz_slots, 3 * ((size_t)m + 1) * sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable));
+        lz_cap = m;
+    }
     // the optional tables change: cached graphs (this handle's host-buffer graphs, and batches, which
     // compare gen) must not replay launches that read the old ones
     void drop_host_graphs() {
@@ -314,6 +329,9 @@ struct edgpu_op_s {
             cudaStreamDestroy(blk_st);
         }
         for (auto e : blk_ev) cudaEventDestroy(e);
+        for (auto e : lz_ev)
+            if (e) cudaEventDestroy(e);
+        if (lz_slots) cudaFreeHost(lz_slots);
     }
 };
 
@@ -3914,17 +3932,24 @@ int edgpu_lanczos(edgpu_op oh, int32_t precision, int32_t n_steps, int32_t reort
     auto fits64 = [&](int k) { return (double)(k + 1) * (double)N * 16.0 <= limit; };
     auto fits32 = [&](int k) { return (double)(k + 1) * (double)N * 8.0 <= limit; };
 
-    DevBuf<double> V64, w, scal, scratch, h, md, psi, vstart;
+    DevBuf<double> V64, ww, small, psi, vstart;
     DevBuf<float> V32, y32;
-    scal.ensure(8);
-    scratch.ensure(dot_scratch_doubles());
-    h.ensure(2 * (size_t)(m + 1));
-    md.ensure(2 * (size_t)(m + 1) * 64);
-    w.ensure(2 * N);
+    // one allocation for the small buffers, one for w and (with reorthogonalisation) w1
+    const size_t n_scratch = std::max(dot_scratch_doubles(), lanczos_scratch_doubles(m + 1));
+    const size_t n_h = 2 * (size_t)(m + 1), n_groups = (size_t)m / 16 + 2;
+    small.ensure(16 + n_scratch + n_h + 2 * n_groups);
+    struct { double* p; } scal{small.p}, scratch{scal.p + 16}, h{scratch.p + n_scratch};
+    double* d_hmax = h.p + n_h;
+    struct { unsigned* p; } tickets{(unsigned*)(d_hmax + n_groups)};
+    EDGPU_CUDA(cudaMemsetAsync(tickets.p, 0, n_groups * sizeof(unsigned), st));
+    ww.ensure((reorth ? 4 : 2) * (size_t)N);
+    struct { double* p; } w{ww.p}, w1{reorth ? ww.p + 2 * (size_t)N : nullptr};
     double* d_alpha = scal.p;      // [0]=re [1]=im of <v, w>
-    double* d_beta = scal.p + 2;   // current beta
-    double* d_bprev = scal.p + 3;  // previous beta
-    double* d_tmp = scal.p + 4;
+    double* d_beta[2] = {scal.p + 2, scal.p + 4};   // |w| and 1 / |w| of the even and odd steps
+    double* d_tmp = scal.p + 6;
+    double* d_nrm2 = scal.p + 8;   // |w|^2 before the projections are subtracted
+    op->ensure_lanczos_slots(m);
+    double* const slots = op->lz_slots;   // per step: alpha, beta, |w|^2 before the projections
 
     // per-run layout
     int cur_prec = precision, cur_store = ROLL, cur_cap = m;
@@ -3977,52 +4002,87 @@ int edgpu_lanczos(edgpu_op oh, int32_t precision, int32_t n_steps, int32_t reort
                    int patience = 1) {
         std::vector<double> hist;   // lowest Ritz value after every step (with conv_tol > 0)
         int settled_for = 0;
-        for (int j = 0; j < steps; ++j) {
+        const bool c64 = cur_store == F32;
+        const void* basis = c64 ? (const void*)V32.p : (const void*)V64.p;
+        auto normalized = [&](int j) {   // v_{j+1} = w / beta_j
+            launch_normalize(N, w.p, d_beta[j & 1], vec64(j + 1), cur_prec == EDGPU_MIXED ? vin32(j + 1) : nullptr, st);
+        };
+        auto issue = [&](int j) {
             double* vj = vec64(j);
-            if (acc) {
-                launch_axpy_real(N, (*acc)[j], vj, psi.p, st);
-                if (j + 1 >= (int)acc->size()) break;
-            }
-            if (cur_prec == EDGPU_FP64) {
-                launch_product(op, EDGPU_FP64, 0, 0, vj, w.p, 0, nullptr, nullptr, st);
-            } else {
-                launch_product(op, EDGPU_MIXED, 0, 0, vin32(j), y32.p, 0, nullptr, nullptr, st);
-                launch_c64_to_c128(N, y32.p, w.p, 0, st);
-            }
-            launch_dot_c128(N, vj, w.p, scratch.p, d_alpha, st);
-            launch_lanczos_update(N, w.p, vj, j > 0 ? vec64(j - 1) : nullptr, d_alpha, j > 0 ? d_bprev : nullptr, st);
+            if (acc) launch_axpy_real(N, (*acc)[j], vj, psi.p, st);
+            if (acc && j + 1 >= (int)acc->size()) return;
+            if (cur_prec == EDGPU_FP64) launch_product(op, EDGPU_FP64, 0, 0, vj, w.p, 0, nullptr, nullptr, st);
+            else launch_product(op, EDGPU_MIXED, 0, 0, vin32(j), y32.p, 0, nullptr, nullptr, st);
+            launch_lanczos_alpha(N, vj, w.p, cur_prec == EDGPU_MIXED ? y32.p : nullptr, scratch.p, tickets.p, d_alpha, st);
+            const double* u = j > 0 ? vec64(j - 1) : nullptr;
+            const double* bu = j > 0 ? d_beta[(j - 1) & 1] : nullptr;
             if (cur_reorth) {
-                for (int pass = 0; pass < 2; ++pass) {
-                    if (cur_store == F64) {
-                        launch_multi_dot(N, j + 1, V64.p, N, w.p, md.p, h.p, st);
-                        launch_multi_axpy(N, j + 1, V64.p, N, h.p, w.p, st);
-                    } else {
-                        launch_multi_dot_c64(N, j + 1, V32.p, N, w.p, md.p, h.p, st);
-                        launch_multi_axpy_c64(N, j + 1, V32.p, N, h.p, w.p, st);
-                    }
-                }
+                launch_lanczos_project(N, j + 1, basis, c64, N, w.p, vj, u, d_alpha, bu, w1.p, scratch.p, tickets.p,
+                                       h.p, d_hmax, d_nrm2, st);
+                launch_lanczos_correct(N, j + 1, basis, c64, N, h.p, d_hmax, w1.p, nullptr, nullptr, d_alpha, nullptr, w.p,
+                                       scratch.p, tickets.p, d_beta[j & 1], d_nrm2, slots + 3 * j, st);
+            } else {
+                launch_lanczos_correct(N, 0, basis, c64, N, nullptr, nullptr, w.p, vj, u, d_alpha, bu, w.p, scratch.p, tickets.p,
+                                       d_beta[j & 1], nullptr, slots + 3 * j, st);
             }
-            launch_norm2_c128(N, w.p, scratch.p, d_beta, st);
-            double hb[2];
-            EDGPU_CUDA(cudaMemcpyAsync(hb, d_alpha, sizeof(double), cudaMemcpyDeviceToHost, st));
-            EDGPU_CUDA(cudaMemcpyAsync(hb + 1, d_beta, sizeof(double), cudaMemcpyDeviceToHost, st));
-            EDGPU_CUDA(cudaStreamSynchronize(st));
-            A.push_back(hb[0]);
-            const double beta = hb[1];
-            if (j == steps - 1 || beta <= 1e-12 * std::max(1.0, std::fabs(hb[0]))) break;
-            if (conv_tol > 0.0 && !acc) {
+            EDGPU_CUDA(cudaEventRecord(op->lz_ev[j & 1], st));
+            if (j + 1 < steps) normalized(j);
+        };
+        // Takes in step j's alpha and beta; false: the run ends there.  again: the step after it has to be
+        // issued (again).
+        auto consume = [&](int j, bool& again) {
+            EDGPU_CUDA(cudaEventSynchronize(op->lz_ev[j & 1]));
+            const double* sl = slots + 3 * j;
+            const double alpha = sl[0];
+            double beta = sl[1];
+            const double tiny = 1e-12 * std::max(1.0, std::fabs(alpha));
+            if (cur_reorth && j + 1 < steps && beta > tiny && beta * beta < 0.25 * sl[2]) {
+                // the projections took most of w away, so rounding errors of their size are left in it: once
+                // more, on v_{j+1} (the criterion of Daniel, Gragg, Kaufman and Stewart)
+                double* vn = vec64(j + 1);
+                launch_lanczos_project(N, j + 1, basis, c64, N, vn, nullptr, nullptr, nullptr, nullptr, w1.p, scratch.p,
+                                       tickets.p, h.p, d_hmax, d_nrm2, st);
+                launch_lanczos_correct(N, j + 1, basis, c64, N, h.p, d_hmax, w1.p, nullptr, nullptr, nullptr, nullptr, w.p,
+                                       scratch.p, tickets.p, d_tmp, d_nrm2, slots + 3 * m, st);
+                launch_normalize(N, w.p, d_tmp, vn, cur_prec == EDGPU_MIXED ? vin32(j + 1) : nullptr, st);
+                EDGPU_CUDA(cudaStreamSynchronize(st));
+                beta *= slots[3 * m + 1];
+                const double both[2] = {beta, 1.0 / beta};
+                EDGPU_CUDA(cudaMemcpyAsync(d_beta[j & 1], both, sizeof(both), cudaMemcpyHostToDevice, st));
+                EDGPU_CUDA(cudaStreamSynchronize(st));
+                again = true;
+            }
+            A.push_back(alpha);
+            if (j == steps - 1 || beta <= tiny) return false;
+            if (conv_tol > 0.0) {
                 const double e = lowest_eigenvalue(A, B);
                 hist.push_back(e);
-                const size_t h = hist.size();
-                const bool settled = h > 5 && std::fabs(e - hist[h - 6]) < conv_tol * std::max(1.0, std::fabs(e));
+                const size_t nh = hist.size();
+                const bool settled = nh > 5 && std::fabs(e - hist[nh - 6]) < conv_tol * std::max(1.0, std::fabs(e));
                 settled_for = settled ? settled_for + 1 : 0;
-                if (kt > 0.0 && (int)A.size() >= kt_min && kt_ok(A, B, beta, e, kt_th2, kt)) break;
-                if (settled_for >= (kt > 0.0 ? patience : 1)) break;
+                if (kt > 0.0 && (int)A.size() >= kt_min && kt_ok(A, B, beta, e, kt_th2, kt)) return false;
+                if (settled_for >= (kt > 0.0 ? patience : 1)) return false;
             }
             B.push_back(beta);
-            launch_normalize(N, w.p, d_beta, vec64(j + 1), cur_prec == EDGPU_MIXED ? vin32(j + 1) : nullptr, st);
-            EDGPU_CUDA(cudaMemcpyAsync(d_bprev, d_beta, sizeof(double), cudaMemcpyDeviceToDevice, st));
+            return true;
+        };
+        if (acc) {
+            for (int j = 0; j < std::min(steps, (int)acc->size()); ++j) issue(j);
+            return;
         }
+        // Short steps: a step is issued before the one before it is taken in, so that the GPU does not
+        // wait for the host between them (the run then computes one step more than it uses); from 2^20
+        // rows on a step is far longer than the 10 to 20 us that hides.  (With a complex64 basis the step
+        // issued ahead overwrites the complex128 v_j that a second projection would need.)
+        const bool ahead = N < ((int64_t)1 << 20) && !(cur_reorth && cur_store != F64);
+        issue(0);
+        for (int j = 0;; ++j) {
+            if (ahead && j + 1 < steps) issue(j + 1);
+            bool again = !ahead;
+            if (!consume(j, again)) break;
+            if (again) issue(j + 1);
+        }
+        EDGPU_CUDA(cudaStreamSynchronize(st));   // (a step issued ahead writes its slot)
     };
     auto lowest = [&](const std::vector<double>& A, const std::vector<double>& B) {
         return lowest_eigenvalue(A, std::vector<double>(B.begin(), B.begin() + (A.size() - 1)));
@@ -4044,8 +4104,9 @@ int edgpu_lanczos(edgpu_op oh, int32_t precision, int32_t n_steps, int32_t reort
                 coef[2 * k + 1] = 0.0;
             }
             EDGPU_CUDA(cudaMemcpyAsync(h.p, coef.data(), coef.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-            if (cur_store == F64) launch_multi_axpy(N, (int)s.size(), V64.p, N, h.p, psi.p, st);
-            else launch_multi_axpy_c64(N, (int)s.size(), V32.p, N, h.p, psi.p, st);
+            launch_lanczos_correct(N, (int)s.size(), cur_store == F64 ? (const void*)V64.p : (const void*)V32.p,
+                                   cur_store != F64, N, h.p, nullptr, psi.p, nullptr, nullptr, nullptr, nullptr, psi.p, scratch.p,
+                                   tickets.p, d_tmp, nullptr, nullptr, st);
         }
         EDGPU_CUDA(cudaStreamSynchronize(st));
     };
@@ -4126,14 +4187,11 @@ int edgpu_lanczos(edgpu_op oh, int32_t precision, int32_t n_steps, int32_t reort
             launch_norm2_c128(N, psi.p, scratch.p, d_tmp, st);
             launch_normalize(N, psi.p, d_tmp, psi.p, nullptr, st);
             launch_product(op, EDGPU_FP64, 0, 0, psi.p, w.p, 0, nullptr, nullptr, st);
-            launch_dot_c128(N, psi.p, w.p, scratch.p, d_alpha, st);
-            launch_lanczos_update(N, w.p, psi.p, nullptr, d_alpha, nullptr, st);
-            launch_norm2_c128(N, w.p, scratch.p, d_beta, st);
-            double hb[2];
-            EDGPU_CUDA(cudaMemcpyAsync(hb, d_alpha, sizeof(double), cudaMemcpyDeviceToHost, st));
-            EDGPU_CUDA(cudaMemcpyAsync(hb + 1, d_beta, sizeof(double), cudaMemcpyDeviceToHost, st));
+            launch_lanczos_alpha(N, psi.p, w.p, nullptr, scratch.p, tickets.p, d_alpha, st);
+            launch_lanczos_correct(N, 0, nullptr, false, N, nullptr, nullptr, w.p, psi.p, nullptr, d_alpha, nullptr, w.p, scratch.p,
+                                   tickets.p, d_tmp, nullptr, slots, st);
             EDGPU_CUDA(cudaStreamSynchronize(st));
-            const double e_rq = hb[0], rn = hb[1];
+            const double e_rq = slots[0], rn = slots[1];
             const double theta2 = kth_eigenvalue(A, std::vector<double>(B.begin(), B.begin() + (A.size() - 1)), 2);
             theta2_mixed = theta2;
             ++done;
@@ -4195,7 +4253,7 @@ int edgpu_random_vector_device(int64_t n, uint64_t seed, int32_t precision, void
         target = tmp.p;
     }
     scratch.ensure(dot_scratch_doubles());
-    nrm.ensure(1);
+    nrm.ensure(2);
     launch_random_c128(n, seed, target, st);
     launch_norm2_c128(n, target, scratch.p, nrm.p, st);
     launch_normalize(n, target, nrm.p, target, precision == EDGPU_MIXED ? (float*)dst : nullptr, st);

@@ -451,22 +451,29 @@ void launch_conj_c128(int64_t n, double* v, cudaStream_t st);
 // Deterministic FP64 reductions through a per-call scratch buffer of at least dot_scratch_doubles().
 size_t dot_scratch_doubles();
 void launch_dot_c128(int64_t n, const double* a, const double* b, double* scratch, double* out_dev, cudaStream_t st);
+// (a norm: |a|, 1 / |a|)
 void launch_norm2_c128(int64_t n, const double* a, double* scratch, double* out_dev, cudaStream_t st);
 void launch_reduce_grad(int nblocks, int ncoupl, const double* partial, double* out_dev, cudaStream_t st);
-// Lanczos helpers: w = w - a*v - b*u (a, b device scalars, b may be null)
-void launch_lanczos_update(int64_t n, double* w, const double* v, const double* u, const double* alpha_dev,
-                           const double* beta_dev, cudaStream_t st);
-// w = w - V h (h: k complex device values), and h = V^H w
-void launch_multi_dot(int64_t n, int k, const double* V, int64_t ldv, const double* w, double* scratch,
-                      double* h_dev, cudaStream_t st);
-void launch_multi_axpy(int64_t n, int k, const double* V, int64_t ldv, const double* h_dev, double* w,
-                       cudaStream_t st);
-// the same with a complex64 basis V (FP64 accumulation)
-void launch_multi_dot_c64(int64_t n, int k, const float* V, int64_t ldv, const double* w, double* scratch,
-                          double* h_dev, cudaStream_t st);
-void launch_multi_axpy_c64(int64_t n, int k, const float* V, int64_t ldv, const double* h_dev, double* w,
-                           cudaStream_t st);
-// v_next = w / beta (beta device scalar); also writes a complex64 copy when v32 != null
+// One Lanczos step.  scratch: lanczos_scratch_doubles(largest k); tickets: one zeroed counter per 16 basis
+// vectors (each launch leaves them zero).  Every null vector or scalar drops its term.
+// alpha = <v, w> (re, im); with y32, w is first written as the widened complex64 vector y32.
+size_t lanczos_scratch_doubles(int kmax);
+void launch_lanczos_alpha(int64_t n, const double* v, double* w, const float* y32, double* scratch, unsigned* tickets,
+                          double* alpha_dev, cudaStream_t st);
+// w1 = w - alpha v - beta u, h = V^H w1 (k vectors, complex128 or complex64), hmax = largest |Re h|, |Im h| of
+// every group of vectors (room for one per 16 vectors), nrm2 = |w1|^2
+void launch_lanczos_project(int64_t n, int k, const void* V, bool c64, int64_t ldv, const double* w, const double* v,
+                            const double* u, const double* alpha_dev, const double* beta_dev, double* w1,
+                            double* scratch, unsigned* tickets, double* h_dev, double* hmax_dev, double* nrm2_dev,
+                            cudaStream_t st);
+// w = w1 - alpha v - beta u - V h, beta_out = |w|, 1 / |w| (hmax, nrm2: those of the projections of w1, null for other
+// coefficients h); slot (host memory the device can address): alpha, |w| and
+// nrm2 (without one: |w|^2)
+void launch_lanczos_correct(int64_t n, int k, const void* V, bool c64, int64_t ldv, const double* h_dev,
+                            const double* hmax_dev, const double* w1, const double* v, const double* u, const double* alpha_dev,
+                            const double* beta_dev, double* w, double* scratch, unsigned* tickets, double* beta_out,
+                            const double* nrm2_dev, double* slot, cudaStream_t st);
+// v_next = w / beta (beta_dev: beta, 1 / beta); also writes a complex64 copy when v32 != null
 void launch_normalize(int64_t n, const double* w, const double* beta_dev, double* v_next, float* v32,
                       cudaStream_t st);
 void launch_axpy_real(int64_t n, double a, const double* x, double* y, cudaStream_t st);
