@@ -60,6 +60,8 @@ struct Layout {
     int popcount = -1;               // >= 0: spin-1/2-like sector = all words of nbits with this popcount
 };
 
+struct VectorTables;
+
 struct Space {
     Layout lay;
     bool reduced = false;
@@ -90,6 +92,7 @@ struct Space {
     int rank_wide = 0;               // rank table entries are uint64 (else uint32)
     int rank_split = 0;              // > 0: split rank tables A (high bits) and B (rank_split low bits)
     uint64_t map_gen = 0;            // bumped whenever the map is built or freed
+    mutable VectorTables* vec = nullptr;   // tables of the vector maps to and from the parent (on first use)
     ~Space();
 };
 // Build (or free) the parent-state map of a reduced space; false when it does not apply or would
@@ -130,6 +133,30 @@ struct GroupBuffers {
     void upload(const Group& g, const Layout& lay);
     void release();
     ~GroupBuffers() { release(); }
+};
+
+// Device tables of a reduced space's vector maps (reduce_vector): amplitudes chi sqrt(|stab| / |G|) by
+// (orbit-size index, character numerator), phases by numerator, sqrt(|stab| / |G|) / |stab| by orbit-size
+// index, and the split colex rank tables of a popcount parent.
+struct VectorTables {
+    struct Dev {
+        const double2* ampl;
+        const double2* phase;
+        const double* inv_norm;
+        const void* rank;
+        long long rank_hi;             // entries of the high part's table
+        int rank_split, rank_wide;     // low bits (0: no tables), 64-bit entries
+        int by_rank;                   // a parent index is the state's colex rank
+        int elem_bits;                 // index bits beside a 32-bit ring state
+    };
+    GroupBuffers gb;
+    double2* d_ampl = nullptr;
+    double* d_inv = nullptr;
+    void* d_rank = nullptr;
+    Dev dev{};
+    VectorTables() = default;
+    VectorTables(const VectorTables&) = delete;
+    ~VectorTables();
 };
 
 // Host helpers used by several units.

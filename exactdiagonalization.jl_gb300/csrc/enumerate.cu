@@ -12,6 +12,7 @@
 //   LIST   a materialised parent basis
 #include <algorithm>
 #include <cmath>
+#include <memory>
 #include <mutex>
 
 #include "edgpu_internal.h"
@@ -725,6 +726,13 @@ Space::~Space() {
     if (d_dir) cudaFree(d_dir);
     if (d_map) cudaFree(d_map);
     if (d_rank) cudaFree(d_rank);
+    delete vec;
+}
+
+VectorTables::~VectorTables() {
+    if (d_ampl) cudaFree(d_ampl);
+    if (d_inv) cudaFree(d_inv);
+    if (d_rank) cudaFree(d_rank);
 }
 
 void enumerate_parent(Space& s, cudaStream_t st) {
@@ -1055,6 +1063,23 @@ int bitlen_u64(unsigned long long v) {
     return b;
 }
 
+// Split colex rank tables of the n-bit words of popcount k: A over the high n - n / 2 bits, then B over the
+// low n / 2 (see build_parent_map).
+constexpr int RANK_SPLIT_BITS = 44;
+std::vector<unsigned long long> split_rank_table(int n, int k) {
+    const int lb = n / 2, hb = n - lb;
+    std::vector<unsigned long long> T(((size_t)1 << hb) + ((size_t)1 << lb), 0ull);
+    unsigned long long acc = 0;
+    for (size_t h = 0; h < ((size_t)1 << hb); ++h) {
+        T[h] = acc;
+        const int need = k - __builtin_popcountll(h);
+        acc += (need >= 0 && need <= lb) ? host_binom(lb, need) : 0ull;
+    }
+    std::vector<unsigned long long> cnt(lb + 1, 0ull);
+    for (size_t l = 0; l < ((size_t)1 << lb); ++l) T[((size_t)1 << hb) + l] = cnt[__builtin_popcountll(l)]++;
+    return T;
+}
+
 template <typename W>
 void build_map_t(Space& red, cudaStream_t st) {
     const Layout& L = red.lay;
@@ -1108,19 +1133,10 @@ bool build_parent_map(Space& red, int64_t max_bytes, cudaStream_t st) {
     // Chunk form (larger n): T[(c * (k + 1) + j) * 64 + v] = sum over the set bits b of v, in ascending
     // order t = 0, 1, ..., of C(6c + b, j + t + 1).
     const int rank_wide = np > 0xffffffffull ? 1 : 0;
-    const int split = n <= 44 ? n / 2 : 0;
+    const int split = n <= RANK_SPLIT_BITS ? n / 2 : 0;
     std::vector<unsigned long long> T;
     if (split) {
-        const int lb = split, hb = n - split;
-        T.assign(((size_t)1 << hb) + ((size_t)1 << lb), 0ull);
-        unsigned long long acc = 0;
-        for (size_t h = 0; h < ((size_t)1 << hb); ++h) {
-            T[h] = acc;
-            const int need = k - __builtin_popcountll(h);
-            acc += (need >= 0 && need <= lb) ? host_binom(lb, need) : 0ull;
-        }
-        std::vector<unsigned long long> cnt(lb + 1, 0ull);
-        for (size_t l = 0; l < ((size_t)1 << lb); ++l) T[((size_t)1 << hb) + l] = cnt[__builtin_popcountll(l)]++;
+        T = split_rank_table(n, k);
     } else {
         const int nc = (n + RANK_CHUNK - 1) / RANK_CHUNK;
         T.assign((size_t)nc * (k + 1) * 64, 0ull);
@@ -1278,86 +1294,169 @@ __device__ __forceinline__ long long colex_rank(W q, const unsigned long long* C
     return r;
 }
 
+// Colex rank through the split tables (rank_tables) or bit by bit.
+template <typename W>
+__device__ __forceinline__ long long parent_rank(W q, const VectorTables::Dev& t, const unsigned long long* C) {
+    if (t.rank_split) {
+        const unsigned long long hi = (unsigned long long)(q >> t.rank_split);
+        const unsigned long long lo = (unsigned long long)q & ((1ull << t.rank_split) - 1ull);
+        if (t.rank_wide) {
+            const unsigned long long* A = (const unsigned long long*)t.rank;
+            return (long long)(__ldg(A + hi) + __ldg(A + t.rank_hi + lo));
+        }
+        const unsigned* A = (const unsigned*)t.rank;
+        return (long long)(__ldg(A + hi) + __ldg(A + t.rank_hi + lo));
+    }
+    return colex_rank<W>(q, C);
+}
+
+constexpr int UNRED_E = 16;   // consecutive parent states per thread and round
+
 // large[i] = ampl(p_i) small[c(p_i)] (0 where the orbit has no representative), the parent index i
-// running over [0, n_parent).
+// running over [0, n_parent).  The amplitude chi(g) sqrt(|stab| / |G|) comes from a table by the key's
+// orbit-size index and the character (the square root and division it replaces kept the FP64 pipe busy
+// for most of the kernel), rings are canonicalised by funnel shifts, the representative's row comes from
+// the search directory, and a thread unranks one state in sixteen (the others are the next words), handed
+// to the block through shared memory so that large is written in order.  10.4 million states of
+// chain L = 26 at k = 1, complex128, this kernel and k_reduce, calls included: 892 -> 272 us; what is left
+// here is the ring search and the FP64 pipe (four FMAs a state: 66 us).
 template <typename W, typename PW, typename V>
-__global__ void k_unreduce(const PW* parent, long long n_parent, int n, int k, const unsigned long long* C,
-                           const W* reps, long long n_reps, int sb, GroupDev g, const double2* phase, const V* small,
-                           V* large) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n_parent;
-         i += (long long)gridDim.x * blockDim.x) {
-        const W q = parent ? (W)parent[i] : unrank_combo<W>((unsigned long long)i, n, k, C);
-        W rep = q;
-        int gb = 0, stab = 1;
-        if (g.kind == GK_TORUS) {
-            W keep[64];
-            for (int a = 0; a < g.L1; ++a) keep[a] = (W)g.keep[a];
-            canon_torus<W>(q, g.L1, g.L2, g.w, g.rowbits, g.nbits, (W)g.full, keep, true, true, rep, gb, stab);
-        } else if (g.kind == GK_GENERIC) {
-            stab = 0;
-            for (int e = 0; e < g.G; ++e) {
-                const W t = group_elem_apply<W>(q, e, g);
-                if (t < rep) {
-                    rep = t;
-                    gb = e;
+__global__ void __launch_bounds__(256, 4) k_unreduce(const PW* parent, long long n_parent, int n, int k,
+                                                  const unsigned long long* C, const W* reps, DirSearch ds, GroupDev g,
+                                                  VectorTables::Dev t, const V* small, V* large) {
+    __shared__ W st[256 * UNRED_E + 256 * UNRED_E / 32];   // (one word in 33 spare: no bank conflicts)
+    __shared__ W keep[64];
+    if (threadIdx.x < 64) keep[threadIdx.x] = g.kind == GK_TORUS && threadIdx.x < g.L1 ? (W)g.keep[threadIdx.x] : (W)0;
+    __syncthreads();
+    const bool want_arg = g.den > 1;
+    const bool ring = sizeof(W) == 4 && g.kind == GK_TORUS && g.L2 == 1 && g.nbits <= 31;
+    const int pb = t.elem_bits;
+    for (long long base = (long long)blockIdx.x * (256 * UNRED_E); base < n_parent;
+         base += (long long)gridDim.x * (256 * UNRED_E)) {
+        if (!parent) {
+            const long long i0 = base + (long long)threadIdx.x * UNRED_E;
+            W q = i0 < n_parent ? unrank_combo<W>((unsigned long long)i0, n, k, C) : (W)0;
+#pragma unroll
+            for (int j = 0; j < UNRED_E; ++j) {
+                const int at = threadIdx.x * UNRED_E + j;
+                st[at + at / 32] = q;
+                if (i0 + j + 1 < n_parent) q = gosper_next<W>(q);
+            }
+            __syncthreads();
+        }
+#pragma unroll 1
+        for (int j = 0; j < UNRED_E; j += 2) {
+            W rep[2];
+            int gb[2] = {0, 0}, sx[2];
+            bool act[2];
+            long long c[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int at = (j + h) * 256 + threadIdx.x;
+                const long long i = base + at;
+                act[h] = i < n_parent;
+                W q = 0;
+                if (act[h]) q = parent ? (W)parent[i] : st[at + at / 32];
+                rep[h] = q;
+                if (g.kind == GK_TORUS) {
+                    if (ring) {
+                        unsigned m;
+                        canon_ring((unsigned)q, g.nbits, g.L1, g.w, pb, want_arg, m, gb[h]);
+                        rep[h] = (W)m;
+                    } else {
+                        int stab;
+                        canon_torus<W>(q, g.L1, g.L2, g.w, g.rowbits, g.nbits, (W)g.full, keep, want_arg, false, rep[h],
+                                       gb[h], stab);
+                    }
+                } else if (g.kind == GK_GENERIC) {
+                    for (int e = 0; e < g.G; ++e) {
+                        const W u = group_elem_apply<W>(q, e, g);
+                        if (u < rep[h]) {
+                            rep[h] = u;
+                            gb[h] = e;
+                        }
+                    }
                 }
-                stab += (t == q);
+            }
+            if (ds.dir) {
+                key_find_sum2<W>(reps, ds, rep, act, c, sx);
+            } else {
+                c[0] = c[1] = -1;
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const long long i = base + (j + h) * 256 + threadIdx.x;
+                if (!act[h]) continue;
+                V out;
+                out.x = 0;
+                out.y = 0;
+                if (c[h] >= 0) {
+                    const double2 a = __ldg(t.ampl + (size_t)sx[h] * g.den + (want_arg ? __ldg(g.num + gb[h]) : 0));
+                    const V v = small[c[h]];
+                    out.x = (decltype(out.x))(a.x * (double)v.x - a.y * (double)v.y);
+                    out.y = (decltype(out.y))(a.x * (double)v.y + a.y * (double)v.x);
+                }
+                large[i] = out;
             }
         }
-        const long long c = key_find<W>(reps, n_reps, rep, sb, nullptr);
-        V out;
-        out.x = 0;
-        out.y = 0;
-        if (c >= 0) {
-            const double s = sqrt((double)stab / (double)g.G);
-            const double2 ph = phase[g.num[gb]];
-            const V v = small[c];
-            const double ar = ph.x * s, ai = ph.y * s;
-            out.x = (decltype(out.x))(ar * (double)v.x - ai * (double)v.y);
-            out.y = (decltype(out.y))(ar * (double)v.y + ai * (double)v.x);
-        }
-        large[i] = out;
+        if (!parent) __syncthreads();
     }
 }
 
 // small[c] = sum over the orbit members p of rep_c of conj(ampl(p)) large[i(p)].  Every element e of
 // the group gives the member e.rep_c with ampl = conj(chi(e)) sqrt(|stab| / |G|); each distinct
 // member occurs |stab| times among the |G| elements, so the sum over all elements is divided by
-// |stab|.  One thread per representative, elements in a fixed order (reproducible, no atomics).
+// |stab|.  One thread per representative, elements in a fixed order (reproducible, no atomics); the
+// parent index of a member by the split rank tables instead of a sum over its bits.  Bound by the FP64 pipe (four FMAs
+// a member: 66 us of the above) and by random sectors of large.
 template <typename W, typename PW, typename V>
-__global__ void k_reduce(const PW* parent, long long n_parent, const unsigned long long* C, const W* reps,
-                         long long n_reps, int sb, GroupDev g, const double2* phase, const V* large, V* small) {
+__global__ void __launch_bounds__(256) k_reduce(const PW* parent, long long n_parent, const unsigned long long* C,
+                                                const W* reps, long long n_reps, int sb, GroupDev g,
+                                                VectorTables::Dev t, const V* large, V* small) {
+    const int L1 = g.kind == GK_TORUS ? g.L1 : 1, L2 = g.kind == GK_TORUS ? g.L2 : 1;
+    const int G = g.kind == GK_TORUS ? L1 * L2 : g.G;
+    const W full = (W)g.full;
     for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < n_reps;
          c += (long long)gridDim.x * blockDim.x) {
-        const W rep = reps[c] >> sb;
-        int stab = 0;
-        for (int e = 0; e < g.G; ++e) stab += (group_elem_apply<W>(rep, e, g) == rep);
-        const double s = sqrt((double)stab / (double)g.G) / (double)stab;
+        const W key = reps[c], rep = key >> sb;
+        const double s = __ldg(t.inv_norm + (int)(key & (W)((((W)1) << sb) - 1)));
         double ar = 0.0, ai = 0.0;
-        for (int e = 0; e < g.G; ++e) {
-            const W t = group_elem_apply<W>(rep, e, g);
+        int a = 0;
+        W row = rep;   // TORUS: the rows moved up by b
+#pragma unroll 4
+        for (int e = 0; e < G; ++e) {
+            W m;
+            if (g.kind == GK_TORUS) {
+                m = a ? torus_row_rotate<W>(row, a * g.w, (W)__ldg(g.keep + a), full, g.rowbits) : row;
+                if (++a == L1) {
+                    a = 0;
+                    if (L2 > 1) row = (W)(((row << g.rowbits) | (row >> (g.nbits - g.rowbits))) & full);
+                }
+            } else {
+                m = group_elem_apply<W>(rep, e, g);
+            }
             long long i;
-            if (parent) {
+            if (t.by_rank) {
+                i = parent_rank<W>(m, t, C);
+            } else {
                 long long lo = 0, len = n_parent;
                 while (len > 0) {   // searchsortedfirst over the parent basis
                     const long long half = len >> 1;
-                    if ((W)parent[lo + half] < t) {
+                    if ((W)parent[lo + half] < m) {
                         lo += half + 1;
                         len -= half + 1;
                     } else {
                         len = half;
                     }
                 }
-                i = (lo < n_parent && (W)parent[lo] == t) ? lo : -1;
-            } else {
-                i = colex_rank<W>(t, C);
+                i = (lo < n_parent && (W)parent[lo] == m) ? lo : -1;
             }
             if (i < 0) continue;
-            // conj(ampl(t)) = chi(e) sqrt(|stab| / |G|); chi(e) = phase[num[e]]
-            const double2 ph = phase[g.num[e]];
+            // conj(ampl) = chi(e) sqrt(|stab| / |G|); chi(e) = phase[num[e]]
+            const double2 ph = __ldg(t.phase + __ldg(g.num + e));
             const V v = large[i];
-            ar += ph.x * (double)v.x - ph.y * (double)v.y;
-            ai += ph.x * (double)v.y + ph.y * (double)v.x;
+            ar = fma(ph.x, (double)v.x, fma(-ph.y, (double)v.y, ar));
+            ai = fma(ph.x, (double)v.y, fma(ph.y, (double)v.x, ai));
         }
         V out;
         out.x = (decltype(out.x))(ar * s);
@@ -1366,35 +1465,79 @@ __global__ void k_reduce(const PW* parent, long long n_parent, const unsigned lo
     }
 }
 
+// The tables of a reduced space's vector maps: built on first use (the caller holds the space's lock) and
+// kept with the space.
+const VectorTables& vector_tables(const Space& red, const Space& parent) {
+    if (red.vec) return *red.vec;
+    std::unique_ptr<VectorTables> v(new VectorTables);
+    v->gb.upload(red.group, parent.lay);
+    const int den = red.group.den, G = red.group.G;
+    std::vector<int> divs;
+    for (int d = 1; d <= G; ++d)
+        if (G % d == 0) divs.push_back(d);
+    const size_t nd = divs.size();
+    std::vector<double2> h((size_t)den * (nd + 1));   // amplitudes by (orbit-size index, character), then phases
+    std::vector<double> inv(nd);
+    for (int j = 0; j < den; ++j) {
+        const double ang = 2.0 * M_PI * (double)j / (double)den;
+        h[nd * den + j] = make_double2(std::cos(ang), std::sin(ang));
+        for (size_t x = 0; x < nd; ++x) {
+            const double f = std::sqrt((double)divs[x] / (double)G);
+            h[x * den + j] = make_double2(h[nd * den + j].x * f, h[nd * den + j].y * f);
+        }
+    }
+    for (size_t x = 0; x < nd; ++x) inv[x] = std::sqrt((double)divs[x] / (double)G) / (double)divs[x];
+    EDGPU_CUDA(cudaMalloc(&v->d_ampl, h.size() * sizeof(double2)));
+    EDGPU_CUDA(cudaMemcpy(v->d_ampl, h.data(), h.size() * sizeof(double2), cudaMemcpyHostToDevice));
+    EDGPU_CUDA(cudaMalloc(&v->d_inv, inv.size() * sizeof(double)));
+    EDGPU_CUDA(cudaMemcpy(v->d_inv, inv.data(), inv.size() * sizeof(double), cudaMemcpyHostToDevice));
+    VectorTables::Dev& t = v->dev;
+    t.ampl = v->d_ampl;
+    t.phase = v->d_ampl + nd * den;
+    t.inv_norm = v->d_inv;
+    // the element index beside a 32-bit ring state (canon_ring)
+    int pb = 0;
+    while ((1 << pb) < red.group.L1) ++pb;
+    t.elem_bits = red.lay.nbits + pb <= 32 ? pb : 0;
+    // the parent index is the colex rank where the parent is all words of a popcount
+    t.by_rank = parent.lay.popcount >= 0 ? 1 : 0;
+    const int n = parent.lay.nbits;
+    if (t.by_rank && n >= 2 && n <= RANK_SPLIT_BITS) {
+        const std::vector<unsigned long long> T = split_rank_table(n, parent.lay.popcount);
+        t.rank_split = n / 2;
+        t.rank_hi = 1ll << (n - n / 2);
+        t.rank_wide = host_binom(n, parent.lay.popcount) > 0xffffffffull ? 1 : 0;
+        const std::vector<unsigned> T32(T.begin(), T.end());
+        const size_t bytes = T.size() * (t.rank_wide ? 8 : 4);
+        EDGPU_CUDA(cudaMalloc(&v->d_rank, bytes));
+        EDGPU_CUDA(cudaMemcpy(v->d_rank, t.rank_wide ? (const void*)T.data() : (const void*)T32.data(), bytes, cudaMemcpyHostToDevice));
+        t.rank = v->d_rank;
+    }
+    red.vec = v.release();
+    return *red.vec;
+}
+
 template <typename W, typename PW, typename V>
 void reduce_vector_t(const Space& red, const Space& parent, bool unreduce, const void* in, void* out,
                      cudaStream_t st) {
-    GroupBuffers gb;
-    gb.upload(red.group, parent.lay);
-    std::vector<double> ph(2 * (size_t)red.group.den);
-    for (int j = 0; j < red.group.den; ++j) {
-        const double ang = 2.0 * M_PI * (double)j / (double)red.group.den;
-        ph[2 * j] = std::cos(ang);
-        ph[2 * j + 1] = std::sin(ang);
-    }
-    double2* d_ph = nullptr;
-    EDGPU_CUDA(cudaMalloc(&d_ph, ph.size() * sizeof(double)));
-    cudaError_t e = cudaMemcpyAsync(d_ph, ph.data(), ph.size() * sizeof(double), cudaMemcpyHostToDevice, st);
+    const VectorTables& vt = vector_tables(red, parent);
     const PW* pk = parent.d_keys ? (const PW*)parent.d_keys : nullptr;
     const long long n_parent = parent.d_keys ? parent.dim : (long long)host_binom(parent.lay.nbits, parent.lay.popcount);
-    const int blocks = std::max(1, sm_count() * 16);
-    if (e == cudaSuccess) {
-        if (unreduce)
-            k_unreduce<W, PW, V><<<blocks, 256, 0, st>>>(pk, n_parent, parent.lay.nbits, parent.lay.popcount,
-                                                          binomial_table(), (const W*)red.d_keys, red.dim, red.sb, gb.dev,
-                                                          d_ph, (const V*)in, (V*)out);
-        else
-            k_reduce<W, PW, V><<<blocks, 256, 0, st>>>(pk, n_parent, binomial_table(), (const W*)red.d_keys, red.dim,
-                                                        red.sb, gb.dev, d_ph, (const V*)in, (V*)out);
-        e = cudaGetLastError();
+    if (unreduce) {
+        const long long need = (n_parent + 256 * UNRED_E - 1) / (256 * UNRED_E);
+        const int blocks = (int)std::max<long long>(1, std::min<long long>(need, (long long)sm_count() * 16));
+        DirSearch ds{};
+        if (red.dim > 0) ds = dir_search_of(red);
+        k_unreduce<W, PW, V><<<blocks, 256, 0, st>>>(pk, n_parent, parent.lay.nbits, parent.lay.popcount,
+                                                     binomial_table(), (const W*)red.d_keys, ds, vt.gb.dev, vt.dev,
+                                                     (const V*)in, (V*)out);
+    } else if (red.dim > 0) {
+        const int blocks = (int)std::max<long long>(1, std::min<long long>((red.dim + 255) / 256, (long long)sm_count() * 16));
+        k_reduce<W, PW, V><<<blocks, 256, 0, st>>>(pk, n_parent, binomial_table(), (const W*)red.d_keys, red.dim, red.sb,
+                                                   vt.gb.dev, vt.dev, (const V*)in, (V*)out);
     }
+    cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(d_ph);
     if (e != cudaSuccess) throw Error(EDGPU_ERR_CUDA, std::string("vector reduction: ") + cudaGetErrorString(e));
 }
 
