@@ -210,6 +210,7 @@ struct edgpu_op_s {
         unsigned* mask = nullptr;           // the steps' row masks, pass after pass (null: padded)
         int padded = 0;                     // every step has 32 entries
         int tile_steps = 0;                 // mean steps of a tile in a pass
+        int in_order = 0;                   // a row's entries in the target table's order
         unsigned* off = nullptr;            // [n_pass][tiles + 1] first entries relative to the pass
         unsigned* moff = nullptr;           // [n_pass][tiles + 1] first steps relative to the pass
         std::vector<long long> base;        // [n_pass + 1] first entry of each pass
@@ -1169,6 +1170,7 @@ void launch_slab_passes(edgpu_op_s* op, int prec, const Blob& B, const void* x, 
     r.acc_c128 = acc_c128;
     r.accumulate = y_c128 ? 0 : accumulate;
     r.padded = S.padded;
+    r.two_sums = S.in_order && r.n_rows >= SLAB_TWO_SUMS;
     r.tile_steps = S.tile_steps;
     const long long n_tiles = r.n_tiles;
     auto set_pass = [&](int q) {
@@ -2512,7 +2514,9 @@ int edgpu_op_build_slabs(edgpu_op oh, int64_t slab_bytes, int64_t max_bytes, int
                                              S.padded ? (unsigned)n_ids << colbits : 0u);
             EDGPU_CUDA(cudaMemcpy(S.tab + S.base[q] + used, fill.data(), fill.size() * 4, cudaMemcpyHostToDevice));
         }
+        S.in_order = n_pass == 1 && S.tile_steps <= SLAB_IN_ORDER;
         sb.padded = S.padded;
+        sb.in_order = S.in_order;
         sb.n_ids = (int)n_ids;
         d_amp.ensure((size_t)n_slots);
         d_base.ensure(2 * (size_t)n_pass);

@@ -396,6 +396,7 @@ struct SlabBuild {
     int colbits;
     int scaled;                     // ids without the orbit-size indices (amplitude id x den + character)
     int padded;                     // every step has 32 entries (no masks)
+    int in_order;                   // one slab: step k holds every row's k-th entry, in the target table's order
     int n_ids;                      // coefficient ids (a padding entry has the id n_ids)
     int cap;                        // steps a warp of the fill pass lays out at a time (>= the most of one tile)
     int o_scratch;                  // shared-memory offset of the passes' scratch
@@ -406,6 +407,7 @@ struct SlabRun {
     const unsigned* tab;            // this pass's entries
     const unsigned* mask;           // this pass's steps (null on a padded table)
     int padded;
+    int two_sums;                   // mixed precision, padded: two partial sums per row (else four)
     const void* xs;                 // x from the slab's first column
     const void* x;                  // x (first pass: the diagonal's product)
     void* y;
@@ -434,6 +436,13 @@ struct SlabRun {
 // 0.68 against 0.75 ms), and one pass over a sector needs 1.1 to 1.4; at 18 passes of a few entries per
 // row it is above 2, which would double the memory of the largest tables.
 constexpr double SLAB_PAD_MOST = 1.5;
+// One slab of short rows (at most this many steps per tile on average: chains): the rows' entries stay in
+// the target table's order, which fills the steps as well and costs little where few gathers per row wait
+// for each other anyway (chain L = 24, complex64: 4.9 us in order, 4.5 by bond; L = 28, complex128: 104 us
+// in order, 108 by bond).  In mixed precision such a row has four partial sums, two from SLAB_TWO_SUMS rows
+// on: the sums, bit for bit, that four and two lanes per row gave these sectors.
+constexpr int SLAB_IN_ORDER = 32;
+constexpr int64_t SLAB_TWO_SUMS = 1 << 16;
 // Coefficient tables of at most this many entries go to registers (real) or to one copy per shared-
 // memory bank group (SLAB_REP_BYTES in all, which keeps eight blocks of the slab kernel per SM).
 constexpr int SLAB_REG_LUT = 4;

@@ -99,7 +99,8 @@ __global__ void __launch_bounds__(HX_THREADS) hx_slab_count_kernel(const HxParam
 // these rows are still free, what is left of them into the next best, and so on (a row's entries fit,
 // whatever their order, because the tile has a step for each).  Neighbouring rows' targets by one bond
 // are often neighbours too (they are when the targets are representatives themselves), so a step's
-// gathers share lines of x; taking every row's next entry instead touches 1.3 to 1.5 times the lines.
+// gathers share lines of x; taking every row's next entry instead (in_order) touches 1.3 to 1.5 times the
+// lines.
 // One warp per tile; scratch: per warp s.cap steps of 32 entries, their masks and the slabs' first
 // steps; the slabs are taken in runs whose steps fit there.
 template <typename W, int PREC>
@@ -159,6 +160,7 @@ __global__ void __launch_bounds__(HX_THREADS) hx_slab_fill_kernel(const HxParams
             for (unsigned j = lane; j < used; j += 32) occ[j] = 0u;
             __syncwarp();
             long long tpos = tpos0;
+            unsigned mine = 0;   // in_order: this row's entries so far
             for (int cls = 0; cls < p.bond_ncls; ++cls) {
                 const W m = act ? bond_class_mask<W, PREC>(b, bt, cls, n, full) : (W)0;
                 const bool cpar = (bt.ninfo[cls] >> 8) != 0;
@@ -183,6 +185,10 @@ __global__ void __launch_bounds__(HX_THREADS) hx_slab_fill_kernel(const HxParams
                         const unsigned id = s.scaled ? ap : (ap * (unsigned)p.nd + (unsigned)ri) * (unsigned)p.nd + (unsigned)sx;
                         entry = ((unsigned)c - (unsigned)q * wc) | (id << s.colbits);
                     }
+                    if (s.in_order) {   // (one slab)
+                        if (has) ent[mine++ * 32 + lane] = entry;
+                        continue;
+                    }
                     unsigned pending = __ballot_sync(0xffffffffu, q >= qa && q < qb);
                     while (pending) {
                         const int q0 = __shfl_sync(0xffffffffu, q, __ffs((int)pending) - 1);
@@ -205,6 +211,13 @@ __global__ void __launch_bounds__(HX_THREADS) hx_slab_fill_kernel(const HxParams
                         }
                     }
                 }
+            }
+            if (s.in_order) {
+                for (unsigned k = 0; k < used; ++k) {
+                    const unsigned o = __ballot_sync(0xffffffffu, k < mine);
+                    if (lane == 0) occ[k] = o;
+                }
+                __syncwarp();
             }
             for (int q = qa; q < qb; ++q) {
                 const unsigned f0 = first[q - qa], S = first[q - qa + 1] - f0;
@@ -434,10 +447,11 @@ __device__ __forceinline__ void fma_if(double2& a, double2 c, double2 x, unsigne
 // One pass of the product through a padded table: one lane per row, one warp per tile of 32 rows and
 // r.chunk consecutive tiles, four steps at a time: a lane's four entries are one 16-byte load.  While a
 // group's gathers are under way, the entries of the group after the next are read, on through the
-// warp's tiles.  Mixed precision: four partial sums per row, by the entry's place in its group (a row
-// of 93 terms is half as far from its 64-bit sum as with one).  FP64: a step without entries (the last ones of a tile may be) is not added up, since
-// the FP64 pipe sets the pace (a warp's double-precision FMA takes 16 cycles of an SM).
-template <int PREC, bool REAL, int LUTM>
+// warp's tiles.  SUMS: partial sums per row, by the entry's place in its group; mixed precision takes
+// four (a row of 93 terms is half as far from its 64-bit sum as with one) or two (SlabRun::two_sums).
+// FP64: a step without entries (the last ones of a tile may be) is not added up, since the FP64 pipe sets
+// the pace (a warp's double-precision FMA takes 16 cycles of an SM).
+template <int PREC, bool REAL, int LUTM, int SUMS>
 __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_pad_kernel(const SlabRun r) {
     typedef typename Cx<PREC>::V V;
     extern __shared__ __align__(16) unsigned char sm[];
@@ -468,13 +482,14 @@ __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_pad_ker
                 tp += 32;
                 const uint4 e2 = ld_stream(tp + 32);
                 add(acc, e.x, x0, false);
-                add(PREC == 0 ? acc : acc1, e.y, x1, true);
-                add(PREC == 0 ? acc : acc2, e.z, x2, true);
-                add(PREC == 0 ? acc : acc3, e.w, x3, true);
+                add(SUMS == 1 ? acc : acc1, e.y, x1, true);
+                add(SUMS == 4 ? acc2 : acc, e.z, x2, true);
+                add(SUMS == 4 ? acc3 : SUMS == 2 ? acc1 : acc, e.w, x3, true);
                 e = en;
                 en = e2;
             }
-            if (PREC == 1) acc = cadd(cadd(acc, acc1), cadd(acc2, acc3));
+            if (SUMS == 4) acc = cadd(cadd(acc, acc1), cadd(acc2, acc3));
+            if (SUMS == 2) acc = cadd(acc, acc1);
             finish_row<PREC>(r, (long long)tile * 32 + lane, acc, true);
             qt = qn;
         }
@@ -655,8 +670,10 @@ template <int PREC, bool REAL, int LUTM>
 void slab_launch_k(const SlabRun& r, size_t smem, cudaStream_t st) {
     const long long warps = (r.n_tiles + r.chunk - 1) / r.chunk;
     if (r.padded) {
-        auto k = hx_slab_pad_kernel<PREC, REAL, LUTM>;
-        slab_pdl_launch(k, r, slab_blocks(k, smem, warps, r.blocks_per_sm), smem, st);
+        auto go = [&](auto k) { slab_pdl_launch(k, r, slab_blocks(k, smem, warps, r.blocks_per_sm), smem, st); };
+        if constexpr (PREC == 0) go(hx_slab_pad_kernel<PREC, REAL, LUTM, 1>);
+        else if (r.two_sums) go(hx_slab_pad_kernel<PREC, REAL, LUTM, 2>);
+        else go(hx_slab_pad_kernel<PREC, REAL, LUTM, 4>);
     } else {
         auto k = hx_slab_kernel<PREC, REAL, LUTM>;
         slab_pdl_launch(k, r, slab_blocks(k, smem, warps, r.blocks_per_sm), smem, st);
