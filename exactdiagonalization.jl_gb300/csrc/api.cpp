@@ -435,6 +435,23 @@ struct BondClasses {
     std::vector<int32_t> cid;         // [ncls][n][4] coupling id of each slot's terms (-1: no term)
     bool cid_ok = true;               // the terms of every slot share one coupling id
     bool real = true;
+
+    // Whether every slot that a row can match has the same real amplitude a0 (n bits).
+    bool common_amplitude(int n, double& a0) const {
+        bool any = false;
+        a0 = 0.0;
+        for (int c = 0; c < ncls; ++c)
+            for (int k = 0; k < BOND_MAXC; ++k)
+                for (int i = 0; i < n; ++i)
+                    for (int v = 0; v < 4; ++v) {
+                        if (!((comp[((size_t)c * BOND_MAXC + k) * 4 + 1 + (v >> 1)] >> i) & 1ull)) continue;
+                        const double* a = &amp[(((size_t)c * n + i) * 4 + v) * 2];
+                        if (a[1] != 0.0 || (any && a[0] != a0)) return false;
+                        a0 = a[0];
+                        any = true;
+                    }
+        return any;
+    }
 };
 
 bool build_bond_classes(const Layout& lay, const std::vector<uint64_t>& masks, const std::vector<uint64_t>& rows,
@@ -726,6 +743,7 @@ void build_blob(edgpu_op_s* op, int prec, int dir, int mode) {
     const int n_b = s.lay.nbits;
     p.bond_ncls = bc.ncls;
     p.bond_real = bc.real ? 1 : 0;
+    p.bond_one = bc.common_amplitude(n_b, p.bond_a0) ? 1 : 0;
     p.o_bcomp = alloc((size_t)bc.ncls * BOND_MAXC * 4 * wsz);
     p.o_binfo = alloc((size_t)bc.ncls * 4);
     p.o_bflip = alloc((size_t)bc.ncls * n_b * wsz);
@@ -2489,7 +2507,7 @@ int edgpu_op_build_slabs(edgpu_op oh, int64_t slab_bytes, int64_t max_bytes, int
         }
         // padded or with masks
         constexpr int PAD = 2 * 128;   // entries after a padded pass: the product reads two groups ahead
-        S.padded = pad_id && (double)n_steps * 32.0 <= SLAB_PAD_MOST * (double)S.n &&
+        S.padded = pad_id && ((double)n_steps * 32.0 <= SLAB_PAD_MOST * (double)S.n || n_steps < SLAB_PAD_SMALL) &&
                    (double)meta + ((double)n_steps * 32.0 + (double)PAD * n_pass) * 4.0 <= (double)max_bytes;
         S.tile_steps = (int)(n_steps / ((int64_t)n_pass * n_tiles));
         S.base.assign((size_t)n_pass + 1, 0);

@@ -249,6 +249,8 @@ struct HxParams {
     int bond_ncls;
     int o_bcomp, o_binfo, o_bflip, o_bamp;    // shared-memory offsets of the class tables
     int bond_real;                            // every pair amplitude is real
+    int bond_one;                             // every pair that can match has the real amplitude bond_a0
+    double bond_a0;
     int bond_nt;                              // targets per lane and step: 2, or 4 (parent-state map only)
     int bond_pf;                              // target tables: x prefetched this many steps ahead (0: none)
     int bond_uni;                             // target tables: warp-uniform pair steps (bond_tile UNI)
@@ -435,7 +437,9 @@ struct SlabRun {
 // target: the padded product takes a third of the instructions per step (4x8: 1.72 against 2.16 ms, 6x5:
 // 0.68 against 0.75 ms), and one pass over a sector needs 1.1 to 1.4; at 18 passes of a few entries per
 // row it is above 2, which would double the memory of the largest tables.
+// Tables below SLAB_PAD_SMALL steps (2 MB) are always padded.
 constexpr double SLAB_PAD_MOST = 1.5;
+constexpr int64_t SLAB_PAD_SMALL = 1 << 14;
 // One slab of short rows (at most this many steps per tile on average: chains): the rows' entries stay in
 // the target table's order, which fills the steps as well and costs little where few gathers per row wait
 // for each other anyway (chain L = 24, complex64: 4.9 us in order, 4.5 by bond; L = 28, complex128: 104 us

@@ -131,6 +131,47 @@ __device__ __forceinline__ int bond_row_count(W b, const BondTables<W, PREC>& bt
     return cnt;
 }
 
+// acc (or sum) += element x of one target in FP64, with as few double-precision operations as its form
+// needs: the FP64 pipe takes 16 cycles of an SM for each of a warp's, and sets the pace of the FP64
+// products that look their targets up (chain L = 25, k = 3, 208,012 rows: 85 us a product with nine
+// operations a target, 70 us with these four; 61 us with the unrolled ring search of odd lengths).  An amplitude that all pairs share is applied to the row's sum; the ratio of
+// the orbit sizes is 1 for nearly all targets, whose lanes then skip it together.
+template <int GK>
+__device__ __forceinline__ void bond_add_fp64(const HxParams& p, const RowsSector<0>& sc, double2 a, const double* rrow,
+                                              int ri, int sx, int g, double2 x, double2& acc, double2& sum) {
+    const bool equal = GK == GK_TRIVIAL || sx == ri;
+    const bool arg = GK != GK_TRIVIAL && sc.want_arg;
+    if (p.bond_one && !arg) {
+        if (equal) {
+            sum.x += x.x;
+            sum.y += x.y;
+        } else {
+            const double f = rrow[sx];
+            sum.x = fma_r(f, x.x, sum.x);
+            sum.y = fma_r(f, x.y, sum.y);
+        }
+        return;
+    }
+    if (p.bond_real && !arg) {
+        double f = a.x;
+        if (!equal) f *= rrow[sx];
+        acc.x = fma_r(f, x.x, acc.x);
+        acc.y = fma_r(f, x.y, acc.y);
+        return;
+    }
+    double2 c = a;
+    if (arg) {
+        const double2 ph = sc.ph[sc.num[g]];
+        c = p.bond_one ? ph : p.bond_real ? cscale(ph, a.x) : cmul(a, ph);
+    }
+    if (!equal) c = cscale(c, rrow[sx]);
+    double2& t = p.bond_one ? sum : acc;
+    t.x = fma_r(c.x, x.x, t.x);
+    t.x = fma_r(-c.y, x.y, t.x);
+    t.y = fma_r(c.x, x.y, t.y);
+    t.y = fma_r(c.y, x.x, t.y);
+}
+
 // One warp tile of rows (32 / lpr consecutive rows of the sector, lpr lanes each) of the pair-flip
 // schedule; lane sub of a row takes the pairs whose start bit i has i % lpr == sub.  NT targets per
 // lane and step (2 or 4): their lookups, then their gathers, are issued together.
@@ -171,6 +212,7 @@ __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W,
     const W b = kr >> sb;
     const int ri = (int)(kr & smask);
     V acc = czero<V>();
+    V sum = czero<V>();  // FP64: the targets' sum without the amplitude they share (p.bond_one)
     V gv = czero<V>();   // GRAD: gy of the row
     if (!FILL && ADJ == 0) {
         const V xr = act ? x[row] : czero<V>();
@@ -354,7 +396,9 @@ __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W,
                     a += gv.x * t.x + gv.y * t.y;
                 }
             }
-            if (c[h] >= 0) {
+            if constexpr (PREC == 0) {
+                if (c[h] >= 0) bond_add_fp64<GK>(p, sc, bt.amp[ti[h]], rrow, ri, sx[h], g[h], xv[h], acc, sum);
+            } else if (c[h] >= 0) {
                 const V a = bt.amp[ti[h]];
                 if (GK == GK_TRIVIAL) {
                     acc = cadd(acc, cmul(a, xv[h]));
@@ -378,6 +422,12 @@ __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W,
         }
     }
     if (FILL || ADJ != 0) return;
+    if constexpr (PREC == 0) {
+        if (p.bond_one) {
+            acc.x = fma_r(p.bond_a0, sum.x, acc.x);
+            acc.y = fma_r(p.bond_a0, sum.y, acc.y);
+        }
+    }
     // partial sums of the row's lanes (fixed butterfly order)
     for (int d = 1; d < lpr; d <<= 1) acc = cadd(acc, shfl_xor_v(acc, d));
     if (act && sub == 0) {

@@ -40,7 +40,7 @@ def _sector(E, shape, q, k, scaling, slab_bytes):
 # (shape, 2Sz, momentum): sectors of 1, 3, 32 and 33 rows (one tile, one row more), ragged ones, and
 # several tiles; many passes: 1024 columns per slab
 CASES = [((4, 1), 2, (0, 0)), ((6, 1), 0, (1, 0)), ((13, 1), 5, (3, 0)), ((11, 1), 3, (2, 0)), ((12, 1), 0, (0, 0)),
-         ((4, 3), 0, (1, 2)), ((17, 1), 1, (5, 0)), ((5, 4), 0, (0, 0))]
+         ((4, 3), 0, (1, 2)), ((17, 1), 1, (5, 0)), ((5, 4), 0, (0, 0)), ((20, 1), 0, (3, 0))]
 
 
 @pytest.mark.parametrize("slab_bytes", [1 << 20, 8192])
