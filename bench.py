@@ -1016,7 +1016,8 @@ def main():
     ap.add_argument("--batch-launch", type=int, default=7, choices=[0, 1, 2, 3, 5, 6, 7],
                     help="batched workload with --tiling: the batch launch mode (edgpu_batch_set_launch)")
     ap.add_argument("--slab-mode", type=int, default=1, choices=[1, 2, 3, 4, 5, 6],
-                    help="with --tiling: use the slab product (any value)")
+                    help="with --tiling: use the slab product; one kernel serves all codes (5 and 6 took two and "
+                         "four lanes per row)")
     ap.add_argument("--slab-scaling", type=int, default=0, choices=[0, 1, 2],
                     help="slab table layout (edgpu_op_slab_scaling): 0 scaled on sectors of 2^22 rows or more "
                          "where that saves passes or the coefficients are complex, 1 never, 2 always")
