@@ -225,6 +225,7 @@ struct edgpu_op_s {
         DevBuf<double> lut64;               // the same in FP64
         int lut_real = 1;
         int lut_mode = 0;                   // SlabRun::lut_mode
+        int occ[2] = {0, 0};                // [precision] SlabRun::occ
         // scaled table: ids carry no orbit-size indices; x is scaled by sqrt(|O_c|) into xsc before the
         // passes and row r of the result by 1 / sqrt(|O_r|) in the last pass
         int scaled = 0;
@@ -1188,6 +1189,7 @@ void launch_slab_passes(edgpu_op_s* op, int prec, const Blob& B, const void* x, 
     r.acc_c128 = acc_c128;
     r.accumulate = y_c128 ? 0 : accumulate;
     r.padded = S.padded;
+    r.occ = &S.occ[prec];
     r.two_sums = S.in_order && r.n_rows >= SLAB_TWO_SUMS;
     r.tile_steps = S.tile_steps;
     const long long n_tiles = r.n_tiles;

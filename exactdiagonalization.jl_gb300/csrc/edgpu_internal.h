@@ -431,6 +431,7 @@ struct SlabRun {
     int nd;
     long long tile0;                // the launch covers the tiles [tile0, tile0 + n_tiles)
     int chunk;                      // consecutive tiles of a warp (set by hx_slab_launch)
+    int* occ;                       // host: resident blocks per SM of the table's kernel (0: not known yet)
     int blocks_per_sm;              // 0: as many as fit; > 0: at most that many; < 0: leave -blocks_per_sm free
 };
 // A table is padded (32 entries in every step, no masks) where that takes at most this many entries per

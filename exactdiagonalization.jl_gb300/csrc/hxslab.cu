@@ -600,12 +600,16 @@ void slab_pdl_launch(K kern, const SlabRun& r, int blocks, size_t smem, cudaStre
     EDGPU_CUDA(cudaLaunchKernelEx(&cfg, kern, r));
 }
 
-// Blocks of a launch over n_warps warps of work.
+// Blocks of a launch over n_warps warps of work.  *occ: the blocks that fit on an SM, 0 until a table's
+// first launch (the query costs a microsecond of the host's five per launch).
 template <typename K>
-int slab_blocks(K kern, size_t smem, long long n_warps, int per_sm = 0) {
-    raise_smem_limit((const void*)kern, smem);
-    int n = 0;
-    EDGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kern, HX_THREADS, smem));
+int slab_blocks(K kern, size_t smem, long long n_warps, int* occ, int per_sm = 0) {
+    if (*occ == 0) {
+        raise_smem_limit((const void*)kern, smem);
+        EDGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, HX_THREADS, smem));
+        *occ = std::max(1, *occ);
+    }
+    int n = *occ;
     if (per_sm > 0) n = std::min(n, per_sm);
     else if (per_sm < 0) n = std::max(1, n + per_sm);
     const long long need = (n_warps + HX_THREADS / 32 - 1) / (HX_THREADS / 32);
@@ -670,13 +674,13 @@ template <int PREC, bool REAL, int LUTM>
 void slab_launch_k(const SlabRun& r, size_t smem, cudaStream_t st) {
     const long long warps = (r.n_tiles + r.chunk - 1) / r.chunk;
     if (r.padded) {
-        auto go = [&](auto k) { slab_pdl_launch(k, r, slab_blocks(k, smem, warps, r.blocks_per_sm), smem, st); };
+        auto go = [&](auto k) { slab_pdl_launch(k, r, slab_blocks(k, smem, warps, r.occ, r.blocks_per_sm), smem, st); };
         if constexpr (PREC == 0) go(hx_slab_pad_kernel<PREC, REAL, LUTM, 1>);
         else if (r.two_sums) go(hx_slab_pad_kernel<PREC, REAL, LUTM, 2>);
         else go(hx_slab_pad_kernel<PREC, REAL, LUTM, 4>);
     } else {
         auto k = hx_slab_kernel<PREC, REAL, LUTM>;
-        slab_pdl_launch(k, r, slab_blocks(k, smem, warps, r.blocks_per_sm), smem, st);
+        slab_pdl_launch(k, r, slab_blocks(k, smem, warps, r.occ, r.blocks_per_sm), smem, st);
     }
 }
 
