@@ -755,6 +755,48 @@ void build_blob(edgpu_op_s* op, int prec, int dir, int mode) {
     p.o_pdb = p.o_pdv = -1;
     p.n_pdb = grad_pair ? n_pdb : -1;
     p.bunit_real = 0;
+    // One unit amplitude u for all pairs, antiparallel matches only, trivial characters, and every diagonal
+    // term d(b_i, b_j) of a pair with its own coupling, equal on both parallel and on both antiparallel
+    // patterns, with the same change k on a match: then g_c = sum over matches of (Re(conj(gy_r) x_c') u +
+    // k z_r) + base_c sum z_r, with z_r = Re(conj(gy_r) x_r) (hx_bond.cuh, GRAD).
+    p.grad_one = 0;
+    p.no_y = 0;
+    p.o_gbase = -1;
+    p.grad_u = p.grad_kz = 0.0;
+    std::vector<double> gbase;
+    if (grad_pair && prec == EDGPU_FP64 && g.den == 1 && bcu.real && n_pdb >= 0) {
+        double u = 0.0, kap = 0.0;
+        bool ok = bcu.common_amplitude(n_b, u) && u != 0.0, any = false;
+        gbase.assign((size_t)op->n_coupl, 0.0);
+        size_t used = 0;
+        for (int c = 0; c < bc.ncls && ok; ++c) {
+            for (int k = 0; k < BOND_MAXC; ++k) ok = ok && bc.comp[((size_t)c * BOND_MAXC + k) * 4 + 2] == 0;
+            for (int i = 0; i < n_b && ok; ++i) {
+                const uint64_t f = bc.flip[(size_t)c * n_b + i];
+                if (!f) continue;
+                const int32_t* cid = &bc.cid[((size_t)c * n_b + i) * 4];
+                ok = cid[0] >= 0 && cid[0] == cid[1];
+                double kp = 0.0;
+                for (const DiagPair& d : dpairs) {
+                    if (d.cid != cid[0] || d.i == d.j || ((1ull << d.i) | (1ull << d.j)) != f) continue;
+                    for (int pat = 0; pat < 4; ++pat) ok = ok && d.u[pat][1] == 0.0;
+                    ok = ok && d.u[0][0] == d.u[3][0] && d.u[1][0] == d.u[2][0];
+                    kp += d.u[1][0] - d.u[0][0];
+                    gbase[cid[0]] += d.u[0][0];
+                    ++used;
+                }
+                ok = ok && (!any || kp == kap);
+                kap = kp;
+                any = true;
+            }
+        }
+        if (ok && any && used == dpairs.size() && op->n_coupl <= 128) {   // (more have another kernel)
+            p.grad_one = 1;
+            p.grad_u = u;
+            p.grad_kz = kap / u;
+            p.o_gbase = alloc((size_t)op->n_coupl * 8);
+        }
+    }
     if (grad_pair) {
         p.o_bunit = alloc((size_t)bc.ncls * n_b * 4 * vsz);
         p.o_bcid = alloc((size_t)bc.ncls * n_b * 4 * 4);
@@ -880,6 +922,7 @@ void build_blob(edgpu_op_s* op, int prec, int dir, int mode) {
         for (size_t i = 0; i < bc.flip.size(); ++i) putw(p.o_bflip, i, bc.flip[i]);
         for (size_t i = 0; i < bc.flip.size() * 4; ++i) putv(p.o_bamp, i, bc.amp[2 * i], bc.amp[2 * i + 1]);
     }
+    if (p.grad_one) memcpy(&h[p.o_gbase], gbase.data(), gbase.size() * 8);
     if (grad_pair) {
         p.bunit_real = bcu.real ? 1 : 0;
         for (size_t i = 0; i < bcu.flip.size() * 4; ++i) putv(p.o_bunit, i, bcu.amp[2 * i], bcu.amp[2 * i + 1]);
@@ -1263,7 +1306,7 @@ static size_t pair_grad_acc_bytes(const edgpu_op_s* op, int prec) {
 void launch_product(edgpu_op_s* op, int prec, int dir, int mode, const void* x, void* y, int accumulate,
                     const void* gy, double* grad_partial, cudaStream_t st, int* blocks_used = nullptr,
                     int rows_override = 0, void* y_c128 = nullptr, int acc_c128 = 0, bool* wrote_c128 = nullptr,
-                    int max_blocks_cap = 0) {
+                    int max_blocks_cap = 0, bool y_unused = false) {
     if (wrote_c128) *wrote_c128 = false;
     // the space's parent-state map is read below and by the launched kernel: hold the space's lock
     // while enqueueing so that the map is not freed in between
@@ -1393,6 +1436,7 @@ void launch_product(edgpu_op_s* op, int prec, int dir, int mode, const void* x, 
             q.gy = gy;
             q.grad_partial = grad_partial;
             q.accumulate = accumulate;
+            q.no_y = y_unused ? 1 : 0;   // (FP64: the product's operations are left out)
             if (table) {
                 q.tab = op->d_tab;
                 q.tile_off = op->d_tile_off;
@@ -3322,7 +3366,8 @@ int edgpu_coupling_grad_device(edgpu_op oh, int32_t precision, const void* x, co
     op->grad_partial.ensure((size_t)max_blocks * op->n_coupl);
     op->grad_dev.ensure(op->n_coupl);
     int blocks = 0;
-    launch_product(op, precision, 0, 1, x, yy, 0, gy, op->grad_partial.p, st, &blocks);
+    launch_product(op, precision, 0, 1, x, yy, 0, gy, op->grad_partial.p, st, &blocks, 0, nullptr, 0, nullptr, 0,
+                   y == nullptr);
     launch_reduce_grad(blocks, op->n_coupl, op->grad_partial.p, op->grad_dev.p, st);
     EDGPU_CUDA(cudaMemcpyAsync(grad_out, op->grad_dev.p, op->n_coupl * sizeof(double), cudaMemcpyDeviceToHost, st));
     EDGPU_CUDA(cudaStreamSynchronize(st));

@@ -261,6 +261,10 @@ struct HxParams {
     // the diagonal records by site pair (n_pdb entries; -1: a record has a mask of more than two bits):
     // i | j << 8 | coupling id << 16, and per entry the unit amplitudes of the pair's four bit patterns
     int o_pdb, o_pdv, n_pdb;
+    // FP64 gradient with one unit amplitude (build_blob): amplitude, the diagonal terms' change on a match over
+    // it, offset of their value without one by coupling; no_y: only the gradient is wanted
+    int grad_one, o_gbase, no_y;
+    double grad_u, grad_kz;
     // adjoint target table (column-sorted; built by the ADJ passes of bond_tile): per column the
     // count, the offset of its run, a fill cursor, and the entries (row << 32 | slot << 19 |
     // row's orbit-size index << 14 | group element)

@@ -135,11 +135,10 @@ __device__ __forceinline__ int bond_row_count(W b, const BondTables<W, PREC>& bt
 // needs: the FP64 pipe takes 16 cycles of an SM for each of a warp's, and sets the pace of the FP64
 // products that look their targets up (chain L = 25, k = 3, 208,012 rows: 85 us a product with nine
 // operations a target, 70 us with these four; 61 us with the unrolled ring search of odd lengths).  An amplitude that all pairs share is applied to the row's sum; the ratio of
-// the orbit sizes is 1 for nearly all targets, whose lanes then skip it together.
+// the orbit sizes is 1 for nearly all targets (equal) and skipped there.
 template <int GK>
 __device__ __forceinline__ void bond_add_fp64(const HxParams& p, const RowsSector<0>& sc, double2 a, const double* rrow,
-                                              int ri, int sx, int g, double2 x, double2& acc, double2& sum) {
-    const bool equal = GK == GK_TRIVIAL || sx == ri;
+                                              bool equal, int sx, int g, double2 x, double2& acc, double2& sum) {
     const bool arg = GK != GK_TRIVIAL && sc.want_arg;
     if (p.bond_one && !arg) {
         if (equal) {
@@ -192,13 +191,17 @@ __device__ __forceinline__ void bond_add_fp64(const HxParams& p, const RowsSecto
 //             reproducible), and every diagonal term matching the row adds Re(u_t z_r) with
 //             z_r = conj(gy_r) x_r.  The accumulators have the product's arithmetic type R (FP32 in
 //             mixed precision: a thread adds a few dozen terms before the block sums them in FP64).
+//             In FP64, where every pair has the same real unit amplitude and its own diagonal terms
+//             follow from the match (p.grad_one), a target takes three double-precision operations (the
+//             diagonal's share rides in the first) and the amplitude is applied to the block's sums; with
+//             p.no_y the product is left out (per-bond couplings on chain L = 28: 477 -> 227 us);
 //   ADJ       (1 or 2, with GK_TABLE) the passes that build the adjoint target table: 1 counts every
 //             target on its column, 2 writes row, slot, the row's orbit-size index and the group
 //             element into the column's run.
 template <typename W, int GK, int PREC, int NT, bool FILL = false, bool UNI = false, bool GRAD = false, int ADJ = 0>
 __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W, PREC>& tb,
                                           const BondTables<W, PREC>& bt, const RowsSector<PREC>& sc, long long tile,
-                                          int lane, typename Cx<PREC>::R* sgrad = nullptr) {
+                                          int lane, typename Cx<PREC>::R* sgrad = nullptr, double* zsum = nullptr) {
     typedef typename Cx<PREC>::V V;
     typedef typename Cx<PREC>::R R;
     const W* __restrict__ keys = (const W*)sc.keys;
@@ -214,12 +217,21 @@ __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W,
     V acc = czero<V>();
     V sum = czero<V>();  // FP64: the targets' sum without the amplitude they share (p.bond_one)
     V gv = czero<V>();   // GRAD: gy of the row
+    // GRAD in FP64, one unit amplitude (p.grad_one): kz = grad_kz Re(conj(gy_r) x_r), the diagonal terms'
+    // share of every pair the row matches, in units of the amplitude
+    const bool grad_one = GRAD && PREC == 0 && p.grad_one;
+    const bool want_y = !(GRAD && PREC == 0 && p.no_y);
+    R kz = 0;
     if (!FILL && ADJ == 0) {
         const V xr = act ? x[row] : czero<V>();
-        if (act && sub == 0) acc = cmul(sc.diag[row], xr);
+        if (act && sub == 0 && want_y) acc = cmul(sc.diag[row], xr);
         if (GRAD) {
             gv = act ? ((const V*)p.gy)[row] : czero<V>();
-            if (act && sub == 0) {
+            if (grad_one) {
+                const R z = fma_r(gv.x, xr.x, gv.y * xr.y);
+                *zsum += (double)z;
+                kz = (R)p.grad_kz * z;
+            } else if (act && sub == 0) {
                 const unsigned char* smb = (const unsigned char*)bt.comp - p.o_bcomp;
                 const W* dm = (const W*)(smb + p.o_pdm);
                 const W* dr = (const W*)(smb + p.o_pdr);
@@ -377,7 +389,23 @@ __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W,
         for (int h = 0; h < NT; ++h) xv[h] = (c[h] >= 0) ? x[c[h]] : czero<V>();
 #pragma unroll
         for (int h = 0; h < NT; ++h) {
-            if (GRAD && c[h] >= 0) {
+            if (grad_one) {
+                // (a warp branch: per lane, the compiler runs both forms' double-precision operations; a
+                // slot without a target has x = 0)
+                R t;
+                if (__any_sync(0xffffffffu, c[h] >= 0 && sx[h] != ri)) {
+                    const R r = c[h] >= 0 ? rrow[sx[h]] : (R)0;
+                    t = fma_r(r, fma_r(gv.x, xv[h].x, gv.y * xv[h].y), kz);
+                } else {
+                    t = fma_r(gv.x, xv[h].x, fma_r(gv.y, xv[h].y, kz));
+                }
+                if (on[h]) {
+                    if (c[h] < 0) t = kz;   // (also where gy_r is not finite)
+                    const unsigned char* smb = (const unsigned char*)bt.comp - p.o_bcomp;
+                    const int cid = ((const int*)(smb + p.o_bcid))[ti[h]];
+                    sgrad[cid * HX_THREADS + threadIdx.x] += t;
+                }
+            } else if (GRAD && c[h] >= 0) {
                 const unsigned char* smb = (const unsigned char*)bt.comp - p.o_bcomp;
                 const V u0 = ((const V*)(smb + p.o_bunit))[ti[h]];
                 const int cid = ((const int*)(smb + p.o_bcid))[ti[h]];
@@ -397,7 +425,11 @@ __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W,
                 }
             }
             if constexpr (PREC == 0) {
-                if (c[h] >= 0) bond_add_fp64<GK>(p, sc, bt.amp[ti[h]], rrow, ri, sx[h], g[h], xv[h], acc, sum);
+                // equal: this target's ratio of the orbit sizes is 1; in the fused gradient, all of the warp's (a
+                // warp branch there, where the FP64 pipe is all that counts)
+                const bool equal = GK == GK_TRIVIAL || (GRAD ? !__any_sync(0xffffffffu, c[h] >= 0 && sx[h] != ri) : sx[h] == ri);
+                if (c[h] >= 0 && want_y)
+                    bond_add_fp64<GK>(p, sc, bt.amp[ti[h]], rrow, equal, sx[h], g[h], xv[h], acc, sum);
             } else if (c[h] >= 0) {
                 const V a = bt.amp[ti[h]];
                 if (GK == GK_TRIVIAL) {
@@ -430,7 +462,7 @@ __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W,
     }
     // partial sums of the row's lanes (fixed butterfly order)
     for (int d = 1; d < lpr; d <<= 1) acc = cadd(acc, shfl_xor_v(acc, d));
-    if (act && sub == 0) {
+    if (act && sub == 0 && want_y) {
         if (PREC == 1 && p.y_c128) {
             // complex128 output (the host-buffer product, written to the caller's buffer): the
             // complex64 result widened, plus the old value for apply!, as the separate conversion does
@@ -558,6 +590,7 @@ __global__ void __launch_bounds__(HX_THREADS) hx_bond_grad_kernel(const HxParams
     typedef typename Cx<PREC>::R R;
     R* sgrad = (R*)(sm + p.o_grad);
     for (int i = threadIdx.x; i < p.n_coupl * HX_THREADS; i += blockDim.x) sgrad[i] = (R)0;
+    double zsum = 0.0;
     __syncthreads();
     const RowsTables<W, PREC> tb(p, sm);
     const BondTables<W, PREC> bt(p, sm);
@@ -583,7 +616,15 @@ __global__ void __launch_bounds__(HX_THREADS) hx_bond_grad_kernel(const HxParams
     const int rpw = 32 / p.lpr;
     const long long n_tiles = (p.n_rows + rpw - 1) / rpw;
     for (long long tile = (long long)blockIdx.x * wpb + warp; tile < n_tiles; tile += (long long)gridDim.x * wpb)
-        bond_tile<W, GK, PREC, NT, false, false, true>(p, tb, bt, sc, tile, lane, sgrad);
+        bond_tile<W, GK, PREC, NT, false, false, true>(p, tb, bt, sc, tile, lane, sgrad, &zsum);
+    // grad_one: the accumulators are in units of the amplitude, and without the diagonal terms' value on
+    // bits a row does not match (grad_base per coupling and unit of z)
+    __shared__ double zw[HX_THREADS / 32];
+    if (PREC == 0 && p.grad_one) {
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) zsum += __shfl_xor_sync(0xffffffffu, zsum, d);
+        if (lane == 0) zw[warp] = zsum;
+    }
     __syncthreads();
     // block sums in FP64, one warp per coupling: lane l adds the accumulators of threads l, l + 32, ...
     // in turn, then a butterfly over the lanes (a fixed order)
@@ -592,6 +633,11 @@ __global__ void __launch_bounds__(HX_THREADS) hx_bond_grad_kernel(const HxParams
         for (int t = lane; t < HX_THREADS; t += 32) sum += (double)sgrad[i * HX_THREADS + t];
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+        if (PREC == 0 && p.grad_one) {
+            double z = 0.0;
+            for (int q = 0; q < wpb; ++q) z += zw[q];
+            sum = p.grad_u * sum + ((const double*)(sm + p.o_gbase))[i] * z;
+        }
         if (lane == 0) p.grad_partial[(size_t)blockIdx.x * p.n_coupl + i] = sum;
     }
 }

@@ -342,6 +342,31 @@ __global__ void __launch_bounds__(HX_THREADS) hx_adj_kernel(const HxParams p) {
         const int sxc = (int)(keys[c] & smask);
         V acc = cmul(cconj(diag[c]), x[c]);
         const long long a = p.adj_off[c], b = p.adj_off[c + 1];
+        if (PREC == 0 && real_fast) {
+            // real amplitudes, trivial characters: the element is its own conjugate.  Two double-precision
+            // operations an entry, which the FP64 pipe sets the pace for; the ratio of the orbit sizes is
+            // 1 for nearly all entries.  Four entries, then their gathers, at a time.
+            for (long long i = a; i < b; i += 4) {
+                unsigned long long e[4];
+                V xr[4];
+#pragma unroll
+                for (int h = 0; h < 4; ++h) e[h] = i + h < b ? p.adj_tab[i + h] : ~0ull;
+#pragma unroll
+                for (int h = 0; h < 4; ++h) xr[h] = e[h] != ~0ull ? x[(long long)(e[h] >> 32)] : czero<V>();
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    if (e[h] == ~0ull) continue;
+                    const int sxr = (int)((e[h] >> 14) & 0x1fu);
+                    R f = bt.amp[(int)((e[h] >> 19) & 0x1fffu)].x;
+                    if (sxr != sxc) f *= tb.ratio[sxr * p.nd + sxc];
+                    acc.x = fma_r(f, xr[h].x, acc.x);
+                    acc.y = fma_r(f, xr[h].y, acc.y);
+                }
+            }
+            if (p.accumulate) acc = cadd(acc, y[c]);
+            y[c] = acc;
+            continue;
+        }
         for (long long i = a; i < b; ++i) {
             const unsigned long long e = p.adj_tab[i];
             const long long r = (long long)(e >> 32);

@@ -130,12 +130,15 @@ __global__ void k_dot_stage2(int nparts, const double2* partial, double* out, in
     }
 }
 
+// out[c] = sum over the blocks of partial[b][c]: a warp per coupling, lane l adds the blocks l, l + 32, ...,
+// then a butterfly (a fixed order; one thread per coupling took 24 us for 304 blocks).
 __global__ void k_reduce_grad(int nblocks, int ncoupl, const double* partial, double* out) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (c >= ncoupl) return;
     double s = 0.0;
-    for (int b = 0; b < nblocks; ++b) s += partial[(size_t)b * ncoupl + c];
-    out[c] = s;
+    for (int b = lane; b < nblocks; b += 32) s += partial[(size_t)b * ncoupl + c];
+    for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+    if (lane == 0) out[c] = s;
 }
 
 // ---- one Lanczos step (launch_lanczos_*): alpha, recurrence and projections, correction, next vector ----
@@ -516,7 +519,7 @@ void launch_norm2_c128(int64_t n, const double* a, double* scratch, double* out_
 
 void launch_reduce_grad(int nblocks, int ncoupl, const double* partial, double* out_dev, cudaStream_t st) {
     if (ncoupl <= 0) return;
-    k_reduce_grad<<<(ncoupl + 127) / 128, 128, 0, st>>>(nblocks, ncoupl, partial, out_dev);
+    k_reduce_grad<<<(ncoupl + 3) / 4, 128, 0, st>>>(nblocks, ncoupl, partial, out_dev);
     EDGPU_CUDA(cudaGetLastError());
 }
 
