@@ -1999,7 +1999,6 @@ int edgpu_reduce(edgpu_space parent_h, int32_t n_elems, const int32_t* site_maps
         EDGPU_CUDA(cudaMalloc(&s->d_keys, 16));
     } else {
         enumerate_reps(*s, *parent, s->hs.stream());
-        embed_orbit_index(*s, s->hs.stream());
     }
     build_search_directory(*s, s->hs.stream());
     *out = s.release();

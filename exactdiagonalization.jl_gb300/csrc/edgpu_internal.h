@@ -126,10 +126,8 @@ struct SectorDev {
 // Device copy of a Group (owned).
 struct GroupBuffers {
     GroupDev dev{};
-    int32_t* d_num = nullptr;
-    unsigned long long* d_keep = nullptr;
-    unsigned long long* d_lut = nullptr;
-    unsigned long long* d_flips = nullptr;
+    unsigned long long* d_all = nullptr;
+    const int32_t* divi = nullptr;   // [d]: index of d among the divisors of G
     void upload(const Group& g, const Layout& lay);
     void release();
     ~GroupBuffers() { release(); }
@@ -176,9 +174,7 @@ void orbit_sizes(const Space& red, int32_t* out_host, cudaStream_t st);
 void lookup_keys(const Space& s, const uint64_t* keys_host, int64_t n, int64_t* out_host, cudaStream_t st);
 // Number of index bits for the divisors of G, and the divisor index of every stabiliser size.
 int orbit_index_bits(int G);
-// Rewrite a freshly enumerated representative table as keys (state << sb) | orbit-size index, and
-// build the shared-memory search tree of any table.
-void embed_orbit_index(Space& red, cudaStream_t st);
+// Builds the search directory of any table.
 void build_search_directory(Space& s, cudaStream_t st);
 void get_states(const Space& s, uint64_t* out_host, cudaStream_t st);
 // Vectors between a reduced space and its parent on the device (symmetry_unreduce / symmetry_reduce):

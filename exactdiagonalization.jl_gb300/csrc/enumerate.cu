@@ -2,7 +2,7 @@
 //
 // Replaces hs_get_basis_list(::HilbertSpaceSector) (hilbert_space_representation.jl:127-206) and the
 // representative sweep of symmetry_reduce (symmetry_reduce_generic.jl:22-106).  Candidates are
-// scanned in increasing order, 32 per thread (one bitmap word per thread, written coalesced);
+// scanned in increasing order, 1024 per warp (one bitmap word per thread, written coalesced);
 // a predicate marks the kept ones, per-block popcounts are scanned into offsets, and a second pass
 // regenerates the candidates and writes the kept ones in order: the output is sorted by
 // construction.  Candidate sources:
@@ -112,13 +112,50 @@ __device__ __forceinline__ bool sector_ok(W s, const SectorDev& d) {
     return false;
 }
 
+// Stages the row-rotation masks of a torus group in shared memory (keep[64]); the block synchronises.
 template <typename W>
-__device__ __forceinline__ bool rep_ok(W s, const GroupDev& g) {
-    if (g.kind == GK_TORUS) {
-        W keep[64];
-        for (int a = 0; a < g.L1; ++a) keep[a] = (W)g.keep[a];
-        return is_rep_torus<W>(s, g.L1, g.L2, g.w, g.rowbits, g.nbits, (W)g.full, keep, g.num);
+__device__ __forceinline__ void stage_keep(W* keep, const GroupDev& g) {
+    if (threadIdx.x < 64) keep[threadIdx.x] = g.kind == GK_TORUS && (int)threadIdx.x < g.L1 ? (W)g.keep[threadIdx.x] : (W)0;
+    __syncthreads();
+}
+
+// A ring of 1-bit (or wider) sites in a 32-bit word, whose rotations are funnel shifts.
+template <typename W>
+__device__ __forceinline__ bool ring32(const GroupDev& g) {
+    return sizeof(W) == 4 && g.kind == GK_TORUS && g.L2 == 1 && g.nbits <= 31;
+}
+
+// Whether a rotation other than the identity leaves the ring state q unchanged: then one by L1 / p sites
+// does, p a prime divisor of L1.
+__device__ __forceinline__ bool ring_periodic(unsigned q, const GroupDev& g) {
+    const unsigned full = (unsigned)g.full;
+    int m = g.L1;
+    for (int p = 2; p * p <= m; ++p) {
+        if (m % p) continue;
+        const int s = g.L1 / p * g.w;
+        if ((((q << s) | (q >> (g.nbits - s))) & full) == q) return true;
+        while (m % p == 0) m /= p;
     }
+    if (m > 1 && g.L1 > 1) {
+        const int s = g.L1 / m * g.w;
+        if (s < g.nbits ? (((q << s) | (q >> (g.nbits - s))) & full) == q : false) return true;
+    }
+    return false;
+}
+
+template <typename W>
+__device__ __forceinline__ bool rep_ok(W s, const GroupDev& g, const W* keep) {
+    if (ring32<W>(g)) {
+        // the smallest rotation by unrolled shifts, two instructions each; the characters on the
+        // stabiliser only for a representative that has one
+        unsigned rep;
+        int e;
+        canon_ring((unsigned)s, g.nbits, g.L1, g.w, 0, false, rep, e);
+        if (rep != (unsigned)s) return false;
+        return !ring_periodic((unsigned)s, g) ||
+               is_rep_torus<W>(s, g.L1, g.L2, g.w, g.rowbits, g.nbits, (W)g.full, keep, g.num);
+    }
+    if (g.kind == GK_TORUS) return is_rep_torus<W>(s, g.L1, g.L2, g.w, g.rowbits, g.nbits, (W)g.full, keep, g.num);
     if (g.kind == GK_GENERIC) {
         for (int e = 1; e < g.G; ++e) {
             W t = 0;
@@ -147,19 +184,41 @@ __device__ __forceinline__ W next_candidate(const EnumParams& p, W v, long long 
     return p.list_w32 ? (W)((const unsigned*)p.list)[r] : (W)((const unsigned long long*)p.list)[r];
 }
 
+// Bit j of bitmap word t: candidate 32 t + j is kept.  A listed candidate is read by the lane that tests
+// it, 32 neighbours at a time (a word is a ballot); the others are generated one after the other.  Bound by
+// the rotations' instructions: 10.4 million states of the chain L = 26 take 66 us, 212 with 32 consecutive
+// states per thread, rotations in a loop and the masks in local memory.
 template <typename W>
 __global__ void __launch_bounds__(ENUM_THREADS) k_mark(EnumParams p) {
     __shared__ long long tmp[32];
+    __shared__ W keep[64];
+    if (p.check_rep) stage_keep<W>(keep, p.grp);
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const long long r0 = t * 32;
     unsigned word = 0;
-    if (r0 < p.total) {
+    if (p.src == SRC_LIST) {
+        const int lane = threadIdx.x & 31;
+        const long long w0 = (t - lane) * 32;   // the warp's 1024 candidates
+#pragma unroll 2
+        for (int j = 0; j < 32; ++j) {
+            const long long r = w0 + 32 * j + lane;
+            bool ok = r < p.total;
+            if (ok) {
+                const W v = first_candidate<W>(p, r);
+                if (p.check_sector) ok = sector_ok<W>(v, p.sec);
+                if (ok && p.check_rep) ok = rep_ok<W>(v, p.grp, keep);
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, ok);
+            if (lane == j) word = m;
+        }
+        if (r0 < p.total) p.bitmap[t] = word;
+    } else if (r0 < p.total) {
         const int cnt = (int)min(32LL, p.total - r0);
         W v = first_candidate<W>(p, r0);
         for (int j = 0; j < cnt; ++j) {
             bool ok = true;
             if (p.check_sector) ok = sector_ok<W>(v, p.sec);
-            if (ok && p.check_rep) ok = rep_ok<W>(v, p.grp);
+            if (ok && p.check_rep) ok = rep_ok<W>(v, p.grp, keep);
             if (ok) word |= 1u << j;
             if (j + 1 < cnt) v = next_candidate<W>(p, v, r0 + j + 1);
         }
@@ -203,16 +262,26 @@ __global__ void __launch_bounds__(ENUM_THREADS) k_compact(EnumParams p) {
     }
 }
 
+// The words of a popcount, ascending: a thread unranks one in sixteen, the block writes them in order
+// (10.4 million words: 30 us, 81 with each thread writing its own run).
+constexpr int COMBO_RUN = 16;
 template <typename W>
-__global__ void k_combo_write(long long total, int n, int k, const unsigned long long* C, W* out) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long r0 = t * 32;
-    if (r0 >= total) return;
-    W v = unrank_combo<W>((unsigned long long)r0, n, k, C);
-    const int cnt = (int)min(32LL, total - r0);
-    for (int j = 0; j < cnt; ++j) {
-        out[r0 + j] = v;
-        if (j + 1 < cnt) v = gosper_next<W>(v);
+__global__ void __launch_bounds__(256) k_combo_write(long long total, int n, int k, const unsigned long long* C, W* out) {
+    __shared__ W st[256 * COMBO_RUN + 256 * COMBO_RUN / 32];   // (one word in 33 spare: no bank conflicts)
+    const long long base = (long long)blockIdx.x * (256 * COMBO_RUN);
+    const long long i0 = base + (long long)threadIdx.x * COMBO_RUN;
+    W v = i0 < total ? unrank_combo<W>((unsigned long long)i0, n, k, C) : (W)0;
+#pragma unroll
+    for (int j = 0; j < COMBO_RUN; ++j) {
+        const int at = threadIdx.x * COMBO_RUN + j;
+        st[at + at / 32] = v;
+        if (i0 + j + 1 < total) v = gosper_next<W>(v);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < COMBO_RUN; ++j) {
+        const int at = j * 256 + threadIdx.x;
+        if (base + at < total) out[base + at] = st[at + at / 32];
     }
 }
 
@@ -256,16 +325,14 @@ int64_t run_filtered(EnumParams p, void** out_keys, bool write, cudaStream_t st)
     const long long n_words = (p.total + 31) / 32;
     const long long n_blocks = (n_words + ENUM_THREADS - 1) / ENUM_THREADS;
     if (n_blocks > 0x7fffffffLL) throw Error(EDGPU_ERR_ARG, "enumeration too large");
-    unsigned* d_bitmap = nullptr;
+    // one allocation: block counts, block offsets, the total, the bitmap
     long long* d_counts = nullptr;
-    long long* d_offsets = nullptr;
-    long long* d_total = nullptr;
     int64_t total = 0;
     try {
-        EDGPU_CUDA(cudaMalloc(&d_bitmap, std::max<long long>(n_words, 1) * sizeof(unsigned)));
-        EDGPU_CUDA(cudaMalloc(&d_counts, std::max<long long>(n_blocks, 1) * sizeof(long long)));
-        EDGPU_CUDA(cudaMalloc(&d_offsets, std::max<long long>(n_blocks, 1) * sizeof(long long)));
-        EDGPU_CUDA(cudaMalloc(&d_total, sizeof(long long)));
+        EDGPU_CUDA(cudaMalloc(&d_counts, (size_t)(2 * n_blocks + 1) * sizeof(long long) + (size_t)n_words * sizeof(unsigned)));
+        long long* d_offsets = d_counts + n_blocks;
+        long long* d_total = d_offsets + n_blocks;
+        unsigned* d_bitmap = (unsigned*)(d_total + 1);
         p.bitmap = d_bitmap;
         p.block_counts = d_counts;
         p.block_offsets = d_offsets;
@@ -295,16 +362,10 @@ int64_t run_filtered(EnumParams p, void** out_keys, bool write, cudaStream_t st)
             *out_keys = keys;
         }
     } catch (...) {
-        cudaFree(d_bitmap);
         cudaFree(d_counts);
-        cudaFree(d_offsets);
-        cudaFree(d_total);
         throw;
     }
-    cudaFree(d_bitmap);
     cudaFree(d_counts);
-    cudaFree(d_offsets);
-    cudaFree(d_total);
     return total;
 }
 
@@ -316,10 +377,10 @@ void enumerate_parent_t(Space& s, cudaStream_t st) {
         s.dim = total;
         if (s.lazy) return;
         EDGPU_CUDA(cudaMalloc(&s.d_keys, std::max<long long>(total, 1) * sizeof(W)));
-        const long long threads = (total + 31) / 32;
-        if (threads > 0) {
-            k_combo_write<W><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(total, lay.nbits, lay.popcount,
-                                                                             binomial_table(), (W*)s.d_keys);
+        if (total > 0) {
+            const long long blocks = (total + 256 * COMBO_RUN - 1) / (256 * COMBO_RUN);
+            k_combo_write<W><<<(unsigned)blocks, 256, 0, st>>>(total, lay.nbits, lay.popcount, binomial_table(),
+                                                              (W*)s.d_keys);
             EDGPU_CUDA(cudaGetLastError());
             EDGPU_CUDA(cudaStreamSynchronize(st));
         }
@@ -336,6 +397,32 @@ void enumerate_parent_t(Space& s, cudaStream_t st) {
     p.sec = sb.dev;
     p.check_rep = 0;
     s.dim = run_filtered<W>(p, &s.d_keys, !s.lazy, st);
+}
+
+// key = (state << sb) | index of the stabiliser size among the divisors of G
+template <typename W>
+__global__ void k_embed(W* keys, long long n, int sb, GroupDev g, const int32_t* divi) {
+    __shared__ W keep[64];
+    stage_keep<W>(keep, g);
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const W q = keys[i];
+    int stab = 1;
+    if (g.kind == GK_TORUS) {
+        W rep;
+        int gb;
+        canon_torus<W>(q, g.L1, g.L2, g.w, g.rowbits, g.nbits, (W)g.full, keep, false, true, rep, gb, stab);
+    } else if (g.kind == GK_GENERIC) {
+        stab = 0;
+        for (int e = 0; e < g.G; ++e) {
+            W t = 0;
+            const unsigned long long* L = g.lut + (size_t)e * g.nchunks * 16;
+            for (int c = 0; c < g.nchunks; ++c) t |= (W)L[c * 16 + (int)((q >> (4 * c)) & 15u)];
+            t ^= (W)g.flips[e];
+            stab += (t == q);
+        }
+    }
+    keys[i] = (W)((q << sb) | (W)divi[stab]);
 }
 
 template <typename W>
@@ -367,6 +454,11 @@ void enumerate_reps_t(Space& red, const Space& parent, cudaStream_t st) {
         p.check_sector = 1;
         p.sec = sb.dev;
         red.dim = run_filtered<W>(p, &red.d_keys, true, st);
+    }
+    if (red.sb > 0 && red.dim > 0) {
+        k_embed<W><<<(unsigned)((red.dim + 255) / 256), 256, 0, st>>>((W*)red.d_keys, red.dim, red.sb, gb.dev, gb.divi);
+        EDGPU_CUDA(cudaGetLastError());
+        EDGPU_CUDA(cudaStreamSynchronize(st));
     }
 }
 
@@ -408,13 +500,13 @@ __global__ void k_mapping(const PW* parent, long long n_parent, const W* reps, l
 
 template <typename W>
 __global__ void k_orbit_sizes(const W* reps, long long n, int sb, GroupDev g, int32_t* out) {
+    __shared__ W keep[64];
+    stage_keep<W>(keep, g);
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const W q = reps[i] >> sb;
     int stab = 1;
     if (g.kind == GK_TORUS) {
-        W keep[64];
-        for (int a = 0; a < g.L1; ++a) keep[a] = (W)g.keep[a];
         W rep;
         int gb;
         canon_torus<W>(q, g.L1, g.L2, g.w, g.rowbits, g.nbits, (W)g.full, keep, false, true, rep, gb, stab);
@@ -446,116 +538,181 @@ __global__ void k_get_states(const W* keys, long long n, int sb, unsigned long l
     if (i < n) out[i] = (unsigned long long)(keys[i] >> sb);
 }
 
-// key = (state << sb) | index of the stabiliser size among the divisors of G
-template <typename W>
-__global__ void k_embed(W* keys, long long n, int sb, GroupDev g, const int32_t* divi) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const W q = keys[i];
-    int stab = 1;
-    if (g.kind == GK_TORUS) {
-        W keep[64];
-        for (int a = 0; a < g.L1; ++a) keep[a] = (W)g.keep[a];
-        W rep;
-        int gb;
-        canon_torus<W>(q, g.L1, g.L2, g.w, g.rowbits, g.nbits, (W)g.full, keep, false, true, rep, gb, stab);
-    } else if (g.kind == GK_GENERIC) {
-        stab = 0;
-        for (int e = 0; e < g.G; ++e) {
-            W t = 0;
-            const unsigned long long* L = g.lut + (size_t)e * g.nchunks * 16;
-            for (int c = 0; c < g.nchunks; ++c) t |= (W)L[c * 16 + (int)((q >> (4 * c)) & 15u)];
-            t ^= (W)g.flips[e];
-            stab += (t == q);
-        }
-    }
-    keys[i] = (W)((q << sb) | (W)divi[stab]);
-}
-
 // Bucket width of a search directory: for every candidate shift s in [s_lo, s_lo + n_shift) count
 // the keys whose bucket (state >> s) holds at most K(s) keys, K(s) = min(4, 28 / (s + sb)) (the keys
 // a bucket summary can carry).  A bucket holds more than K keys exactly when some K+1 consecutive
-// keys around key i share its bucket, so each key reads its K neighbours on either side.
+// keys around key i share its bucket.
+// Two keys share a bucket of width 2^s exactly when their difference has at most s bits, so a window's lane
+// needs one difference per K; which keys lie in a shared window follows from a ballot's bits.  A warp
+// loads 32 keys, SURVEY_LOADS groups ahead, and counts the middle 24 (bound by the latency of the loads
+// and the instructions per shift: 10.4 million keys, two shifts, 61 us; 92 with every thread comparing all
+// windows at each shift).
+constexpr int SURVEY_RUN = 8, SURVEY_LOADS = 4;   // 24-key groups per warp and load phase, load phases
+
 template <typename W>
-__global__ void k_dir_survey(const W* keys, long long n, int sb, int s_lo, int n_shift, unsigned long long* counts) {
-    __shared__ unsigned long long part[64];
-    for (int j = threadIdx.x; j < n_shift; j += blockDim.x) part[j] = 0ull;
-    __syncthreads();
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const bool act = i < n;
-    const unsigned lane = threadIdx.x & 31u;
-    unsigned long long v[9];   // states of keys i-4 .. i+4 (v valid where 0 <= index < n)
-#pragma unroll
-    for (int j = 0; j < 9; ++j) {
-        const long long w = i - 4 + j;
-        v[j] = (act && w >= 0 && w < n) ? (unsigned long long)(keys[w] >> sb) : 0ull;
+__global__ void __launch_bounds__(256) k_dir_survey(const W* keys, long long n, int sb, int s_lo, int n_shift,
+                                                    unsigned long long* counts) {
+    __shared__ unsigned part[64];
+    __shared__ int members[64];   // K of shift s_lo + j
+    if (threadIdx.x < 64) {
+        const int mb = s_lo + (int)threadIdx.x + sb;
+        part[threadIdx.x] = 0u;
+        members[threadIdx.x] = mb == 0 ? 4 : min(4, 28 / mb);
     }
-    for (int j = 0; j < n_shift; ++j) {
-        const int sh = s_lo + j, mb = sh + sb;
-        const int K = mb == 0 ? 4 : min(4, 28 / mb);
-        bool ok = act;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const long long g0 = ((long long)blockIdx.x * 8 + threadIdx.x / 32) * SURVEY_RUN;
+    unsigned mine[2] = {0u, 0u};   // counts of shifts s_lo + lane and s_lo + lane + 32
+#pragma unroll 1
+    for (int c = 0; c < SURVEY_RUN; c += SURVEY_LOADS) {
+        W v[SURVEY_LOADS];
 #pragma unroll
-        for (int a = 0; a <= 4; ++a) {   // the K+1 keys from w = i-4+a (windows through i: a >= 4-K)
-            const long long w = i - 4 + a;
-            if (a >= 4 - K && w >= 0 && w + K < n && (v[a] >> sh) == (v[a + K] >> sh)) ok = false;
+        for (int h = 0; h < SURVEY_LOADS; ++h) {   // the lane's window starts at key w and, as a key, is key w
+            const long long w = (g0 + c + h) * 24 - 4 + lane;
+            v[h] = w >= 0 && w < n ? (W)(keys[w] >> sb) : (W)0;
         }
-        ok = ok && act;
-        const unsigned cnt = __popc(__ballot_sync(0xffffffffu, ok));
-        if (lane == 0 && cnt) atomicAdd(&part[j], (unsigned long long)cnt);
+#pragma unroll
+        for (int h = 0; h < SURVEY_LOADS; ++h) {
+            const long long w0 = (g0 + c + h) * 24 - 4, w = w0 + lane;
+            const bool inner = w0 >= 0 && w0 + 36 <= n;   // every window of the warp lies in the table
+            if (w0 + 4 >= n) break;
+            const unsigned valid = inner ? 0x0ffffff0u : __ballot_sync(0xffffffffu, lane >= 4 && lane < 28 && w < n);
+            int K = -1, len = 0;   // bits of the difference of the window's ends (64: no window)
+            for (int j = 0; j < n_shift; ++j) {
+                if (members[j] != K) {
+                    // (K = 0: buckets too wide for any member; a window of one key is always shared)
+                    K = members[j];
+                    const W x = v[h] ^ __shfl_down_sync(0xffffffffu, v[h], K);
+                    len = sizeof(W) == 8 ? 64 - __clzll((long long)x) : 32 - __clz((int)x);
+                    if (!inner && (w < 0 || w + K >= n)) len = 64;
+                }
+                const unsigned f = __ballot_sync(0xffffffffu, len <= s_lo + j);
+                unsigned bad = f;
+                if (K == 4) {
+                    bad |= bad << 1;
+                    bad |= bad << 2;
+                    bad |= f << 4;
+                } else {
+                    for (int d = 1; d <= K; ++d) bad |= f << d;
+                }
+                const unsigned cnt = __popc(valid & ~bad);
+                if (lane == (j & 31)) mine[j >> 5] += cnt;
+            }
+        }
     }
+    if (mine[0]) atomicAdd(&part[lane], mine[0]);
+    if (mine[1]) atomicAdd(&part[lane + 32], mine[1]);
     __syncthreads();
-    for (int j = threadIdx.x; j < n_shift; j += blockDim.x)
-        if (part[j]) atomicAdd(&counts[j], part[j]);
+    if ((int)threadIdx.x < n_shift && part[threadIdx.x]) atomicAdd(&counts[threadIdx.x], (unsigned long long)part[threadIdx.x]);
 }
 
 // Search directory, one entry per bucket b in [0, nb) plus the sentinel dir[nb] = n:
 // dir[b] = start | min(count, 15) << 32 | the low mb bits of each key << (36 + k*mb) when the bucket
 // holds at most K keys (start = index of the bucket's first key, or of the next key when empty).
-// Each thread builds DIR_CHUNK consecutive buckets: one binary search for the first key of its
-// chunk, then a walk over the chunk's keys.  stats[0] receives the largest bucket and stats[1] the
-// number of keys answered by their bucket summary.
-constexpr int DIR_CHUNK = 128;
+// A block builds DIR_CHUNK consecutive buckets, DIR_STEP at a time: the keys from the step's first on are
+// staged in shared memory (one search in the table per block), counted by bucket, the counts scanned into
+// starts, and neighbouring threads write neighbouring entries.  Bound by instructions: 33.5 million buckets of
+// 10.4 million keys (chain L = 26) take 90 us, 180 with a thread per 128 buckets, whose writes lay 1 KB apart
+// within a warp.  stats[0] receives the largest bucket and
+// stats[1] the number of keys answered by their bucket summary.
+constexpr int DIR_STEP = 2048, DIR_TILE = 4096, DIR_CHUNK = 4 * DIR_STEP;
 
 template <typename W>
-__global__ void k_dir_build(const W* keys, long long n, int sb, int shift, long long nb, int mb, int K,
-                            unsigned long long* dir, unsigned long long* stats) {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long b0 = t * DIR_CHUNK;
-    unsigned long long mx = 0ull, inl = 0ull;
-    if (b0 <= nb) {
-        long long lo = 0, len = n;   // first key with bucket >= b0
-        while (len > 0) {
-            const long long half = len >> 1;
-            if ((long long)((keys[lo + half] >> sb) >> shift) < b0) {
+__global__ void __launch_bounds__(256) k_dir_build(const W* keys, long long n, int sb, int shift, long long nb, int mb,
+                                                   int K, unsigned long long* dir, unsigned long long* stats) {
+    constexpr int E = DIR_STEP / 256;
+    __shared__ W tile[DIR_TILE];
+    __shared__ unsigned cell[DIR_STEP + 256];   // bucket r's count, then start | count << 16, at r + r / E
+    __shared__ unsigned sums[8];
+    const unsigned mbmask = mb >= 32 ? ~0u : (1u << mb) - 1u;   // (a summary's fields have 28 bits at most)
+    auto bucket = [&](W key) { return (long long)((unsigned long long)(key >> sb) >> shift); };
+    // first of the m keys at k with a bucket >= b
+    auto lower = [&](const W* k, long long m, long long b) {
+        long long lo = 0;
+        while (m > 0) {
+            const long long half = m >> 1;
+            if (bucket(k[lo + half]) < b) {
                 lo += half + 1;
-                len -= half + 1;
+                m -= half + 1;
             } else {
-                len = half;
+                m = half;
             }
         }
-        long long i = lo;
-        const unsigned long long mbmask = (mb >= 64) ? ~0ull : ((1ull << mb) - 1ull);
-        const long long b1 = min(b0 + DIR_CHUNK, nb + 1);
-        for (long long bb = b0; bb < b1; ++bb) {
-            if (bb == nb) {
-                dir[bb] = (unsigned long long)n;
-                break;
+        return lo;
+    };
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    unsigned mx = 0u, inl = 0u;
+    const long long c0 = (long long)blockIdx.x * DIR_CHUNK, c1 = min(c0 + DIR_CHUNK, nb);
+    long long cur = lower(keys, n, c0), b1;   // the step's first key and the end of its buckets, alike in all threads
+    for (long long b0 = c0; b0 < c1; b0 = b1) {
+        b1 = min(b0 + DIR_STEP, c1);
+        const int have = (int)min((long long)DIR_TILE, n - cur);
+        __syncthreads();
+        for (int i = threadIdx.x; i < have; i += 256) tile[i] = keys[cur + i];
+#pragma unroll
+        for (int j = 0; j < E + 1; ++j) cell[j * 256 + threadIdx.x] = 0u;
+        __syncthreads();
+        if (cur + have < n) {
+            const long long last = bucket(tile[have - 1]);
+            if (last == b0) {
+                // one bucket fills the tile: count it in the table
+                const long long m = lower(keys + cur, n - cur, b0 + 1);
+                if (threadIdx.x == 0) {
+                    mx = max(mx, (unsigned)m);
+                    dir[b0] = (unsigned long long)cur | (15ull << 32);   // (more than K keys: no members)
+                }
+                cur += m;
+                b1 = b0 + 1;
+                continue;
             }
-            const long long st = i;
-            unsigned long long mem = 0ull;
-            int k = 0;
-            while (i < n && (long long)((keys[i] >> sb) >> shift) == bb) {
-                if (k < K) mem |= ((unsigned long long)keys[i] & mbmask) << (36 + k * mb);
-                ++k;
-                ++i;
-            }
-            const unsigned long long cnt = (unsigned long long)k;
-            if ((long long)cnt <= K) inl += cnt;
-            else mem = 0ull;
-            if (cnt > mx) mx = cnt;
-            dir[bb] = (unsigned long long)st | (min(cnt, 15ull) << 32) | mem;
+            b1 = min(b1, last);   // the buckets before the last key's are whole
         }
+        const unsigned nbk = (unsigned)(b1 - b0);
+        for (int i = threadIdx.x; i < have; i += 256) {
+            const W r = (W)((W)(tile[i] >> sb) >> shift) - (W)b0;
+            if (r < nbk) atomicAdd(&cell[(unsigned)r + (unsigned)r / E], 1u);
+        }
+        __syncthreads();
+        unsigned c[E], sum = 0;
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            c[j] = cell[threadIdx.x * (E + 1) + j];
+            sum += c[j];
+        }
+        unsigned inc = sum;
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned o = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += o;
+        }
+        if (lane == 31) sums[wid] = inc;
+        __syncthreads();
+        unsigned at = inc - sum, all = 0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const unsigned o = sums[j];
+            if (j < wid) at += o;
+            all += o;
+        }
+#pragma unroll
+        for (int j = 0; j < E; ++j) {
+            cell[threadIdx.x * (E + 1) + j] = at | (c[j] << 16);
+            at += c[j];
+        }
+        __syncthreads();
+#pragma unroll 2
+        for (unsigned r = threadIdx.x; r < nbk; r += 256) {
+            const unsigned v = cell[r + r / E], first = v & 0xffffu, cnt = v >> 16;
+            unsigned hi = min(cnt, 15u);   // the entry's upper word; the start is its lower one
+            if ((int)cnt <= K) {
+                for (unsigned k = 0; k < cnt; ++k) hi |= ((unsigned)tile[first + k] & mbmask) << (4 + (int)k * mb);
+                inl += cnt;
+            }
+            mx = max(mx, cnt);
+            dir[b0 + r] = (unsigned long long)((unsigned)cur + first) | ((unsigned long long)hi << 32);
+        }
+        cur += all;
     }
+    if (c1 == nb && threadIdx.x == 0) dir[nb] = (unsigned long long)n;
     for (int d = 16; d > 0; d >>= 1) {
         mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, d));
         inl += __shfl_xor_sync(0xffffffffu, inl, d);
@@ -687,38 +844,42 @@ void GroupBuffers::upload(const Group& g, const Layout& lay) {
     dev.rowbits = g.L1 * g.w;
     dev.nbits = lay.nbits;
     dev.full = (lay.nbits >= 64) ? ~0ull : ((1ull << lay.nbits) - 1ull);
-    EDGPU_CUDA(cudaMalloc(&d_num, std::max<size_t>(g.num.size(), 1) * sizeof(int32_t)));
-    EDGPU_CUDA(cudaMemcpy(d_num, g.num.data(), g.num.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-    dev.num = d_num;
+    // one allocation: 64-bit tables, then the character numerators and divisor indices
+    std::vector<unsigned long long> h;
+    size_t o_flips = 0;
     if (g.kind == GK_TORUS) {
-        auto keep = torus_keep_masks(g, lay.nbits);
-        EDGPU_CUDA(cudaMalloc(&d_keep, keep.size() * sizeof(unsigned long long)));
-        EDGPU_CUDA(cudaMemcpy(d_keep, keep.data(), keep.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice));
-        dev.keep = d_keep;
+        h = torus_keep_masks(g, lay.nbits);
     } else if (g.kind == GK_GENERIC) {
         int nc = 0;
-        auto lut = generic_luts(g, lay, &nc);
+        h = generic_luts(g, lay, &nc);
         dev.nchunks = nc;
-        EDGPU_CUDA(cudaMalloc(&d_lut, lut.size() * sizeof(unsigned long long)));
-        EDGPU_CUDA(cudaMemcpy(d_lut, lut.data(), lut.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice));
-        EDGPU_CUDA(cudaMalloc(&d_flips, g.G * sizeof(unsigned long long)));
-        std::vector<unsigned long long> fl(g.flips.begin(), g.flips.end());
-        fl.resize(g.G, 0ull);
-        EDGPU_CUDA(cudaMemcpy(d_flips, fl.data(), g.G * sizeof(unsigned long long), cudaMemcpyHostToDevice));
-        dev.lut = d_lut;
-        dev.flips = d_flips;
+        o_flips = h.size();
+        h.insert(h.end(), g.flips.begin(), g.flips.end());
+        h.resize(o_flips + g.G, 0ull);
+    }
+    const size_t o_num = h.size();
+    h.resize(o_num + (g.num.size() + 1) / 2 + 1, 0ull);
+    memcpy(h.data() + o_num, g.num.data(), g.num.size() * sizeof(int32_t));
+    const size_t o_divi = h.size();
+    std::vector<int32_t> di(g.G + 1, 0);
+    for (int d = 1, k = 0; d <= g.G; ++d)
+        if (g.G % d == 0) di[d] = k++;
+    h.resize(o_divi + di.size() / 2 + 1, 0ull);
+    memcpy(h.data() + o_divi, di.data(), di.size() * sizeof(int32_t));
+    EDGPU_CUDA(cudaMalloc(&d_all, h.size() * sizeof(unsigned long long)));
+    EDGPU_CUDA(cudaMemcpy(d_all, h.data(), h.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice));
+    dev.num = (const int32_t*)(d_all + o_num);
+    divi = (const int32_t*)(d_all + o_divi);
+    if (g.kind == GK_TORUS) dev.keep = d_all;
+    if (g.kind == GK_GENERIC) {
+        dev.lut = d_all;
+        dev.flips = d_all + o_flips;
     }
 }
 
 void GroupBuffers::release() {
-    cudaFree(d_num);
-    cudaFree(d_keep);
-    cudaFree(d_lut);
-    cudaFree(d_flips);
-    d_num = nullptr;
-    d_keep = nullptr;
-    d_lut = nullptr;
-    d_flips = nullptr;
+    cudaFree(d_all);
+    d_all = nullptr;
 }
 
 Space::~Space() {
@@ -908,26 +1069,6 @@ int orbit_index_bits(int G) {
 
 namespace {
 template <typename W>
-void embed_t(Space& red, cudaStream_t st) {
-    GroupBuffers gb;
-    gb.upload(red.group, red.lay);
-    std::vector<int32_t> divi(red.group.G + 1, 0);
-    int k = 0;
-    for (int d = 1; d <= red.group.G; ++d)
-        if (red.group.G % d == 0) divi[d] = k++;
-    int32_t* d_divi = nullptr;
-    EDGPU_CUDA(cudaMalloc(&d_divi, divi.size() * sizeof(int32_t)));
-    cudaError_t e = cudaMemcpy(d_divi, divi.data(), divi.size() * sizeof(int32_t), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && red.dim > 0) {
-        k_embed<W><<<(unsigned)((red.dim + 255) / 256), 256, 0, st>>>((W*)red.d_keys, red.dim, red.sb, gb.dev, d_divi);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    }
-    cudaFree(d_divi);
-    if (e != cudaSuccess) throw Error(EDGPU_ERR_CUDA, std::string("embed: ") + cudaGetErrorString(e));
-}
-
-template <typename W>
 void dir_t(Space& s, cudaStream_t st) {
     const long long n = s.dim;
     if (n >= (1ll << 32)) throw Error(EDGPU_ERR_ARG, "tables of 2^32 or more rows are not supported");
@@ -959,7 +1100,8 @@ void dir_t(Space& s, cudaStream_t st) {
     std::vector<unsigned long long> cnt(n_shift + 2, 0ull);
     cudaError_t e = cudaMemsetAsync(d_stats, 0, (n_shift + 2) * sizeof(unsigned long long), st);
     if (e == cudaSuccess && n > 0) {
-        k_dir_survey<W><<<(unsigned)((n + 255) / 256), 256, 0, st>>>((const W*)s.d_keys, n, s.sb, s_lo, n_shift, d_stats);
+        const long long per_block = 8 * SURVEY_RUN * 24;
+        k_dir_survey<W><<<(unsigned)((n + per_block - 1) / per_block), 256, 0, st>>>((const W*)s.d_keys, n, s.sb, s_lo, n_shift, d_stats);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(cnt.data(), d_stats, n_shift * sizeof(unsigned long long),
@@ -987,9 +1129,8 @@ void dir_t(Space& s, cudaStream_t st) {
     s.d_dir = nullptr;
     e = cudaMalloc(&s.d_dir, (nb + 1) * sizeof(unsigned long long));
     if (e == cudaSuccess) {
-        const long long threads = nb / DIR_CHUNK + 1;
-        k_dir_build<W><<<(unsigned)((threads + 255) / 256), 256, 0, st>>>((const W*)s.d_keys, n, s.sb, shift, nb, mb, K,
-                                                                          s.d_dir, d_stats + n_shift);
+        k_dir_build<W><<<(unsigned)((nb + DIR_CHUNK - 1) / DIR_CHUNK), 256, 0, st>>>((const W*)s.d_keys, n, s.sb, shift,
+                                                                                   nb, mb, K, s.d_dir, d_stats + n_shift);
         e = cudaGetLastError();
     }
     unsigned long long hs[2] = {0, 0};
@@ -1043,12 +1184,6 @@ DirSearch dir_search_of(const Space& s) {
         d.top |= (1u << (d.mb - 1)) << o;
     }
     return d;
-}
-
-void embed_orbit_index(Space& red, cudaStream_t st) {
-    if (red.sb == 0 || red.dim == 0) return;
-    if (red.w32) embed_t<uint32_t>(red, st);
-    else embed_t<unsigned long long>(red, st);
 }
 
 void build_search_directory(Space& s, cudaStream_t st) {
