@@ -21,13 +21,14 @@
 //
 // What bounds the product, and what the steps gave (complex64, H x in device time, before -> now;
 // before, every lane walked its own row's run of entries): triangular 6x5, 5.2 million rows, one pass,
-// 1167 -> 685 us; square 4x8, 18.8 million rows, two passes, 2960 -> 1750 us; square 6x6, 252 million
-// rows, 18 passes, 70.6 -> 63.9 ms; chain L = 24, 112,720 rows, 5.5 -> 5.1 us.  It was bound by the L1
+// 1167 -> 687 us; square 4x8, 18.8 million rows, two passes, 2960 -> 1750 us; square 6x6, 252 million
+// rows, 18 passes, 70.6 -> 63.9 ms; chain L = 24, 112,720 rows, 5.5 -> 4.9 us.  It was bound by the L1
 // data pipe (every entry load and every gather a line of its own); now a gather touches 0.2 (chains) to
-// 0.4 (tori) lines per entry, and the L1 tag lookups of those lines and the L2 requests behind them
-// share the limit.  In FP64 the FP64 pipe sets the pace, before and now (chain L = 28 107.6 -> 107.8 us,
-// 6x6 130 -> 131.5 ms): a double-precision FMA occupies it for 16 cycles of an SM per warp, so the mean
-// filling of the steps counts there.
+// 0.5 (tori) lines per entry, and the L1 tag lookups of those lines and the L2 requests behind them
+// share the limit (24 sectors of the triangular 6x4, 113,000 rows each: 352 us of tag lookups in 394 us;
+// one launch over all of them, or more padding, gained nothing).  In FP64 the FP64 pipe sets the pace,
+// before and now (chain L = 28 107.6 -> 104.3 us, 6x6 130 -> 131.5 ms): a double-precision FMA occupies
+// it for 16 cycles of an SM per warp, so the mean filling of the steps counts there.
 #include "hx_bond.cuh"
 
 #include <algorithm>
@@ -526,8 +527,8 @@ __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_kernel(
         ld_entries(tab, m, below, e0, e);
         for (; tile < t1; ++tile) {
             const unsigned kn = tile + 1 < t1 ? r.moff[tile + 2] : kt;
-            V acc = czero<V>();
-            unsigned rows_on = 0;   // rows of the tile with entries in this pass
+            V sums[PREC == 0 ? 1 : 4] = {};   // partial sums, as hx_slab_pad_kernel's
+            unsigned rows_on = 0;             // rows of the tile with entries in this pass
             for (; k < kt; k += 4) {
                 V xv[4];
                 unsigned id[4], mc[4];
@@ -544,9 +545,11 @@ __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_kernel(
 #pragma unroll
                 for (int h = 0; h < 4; ++h) {
                     if (PREC == 0 && h > 0 && mc[h] == 0u) continue;
-                    fma_if(acc, lut(id[h]), xv[h], ~mc[h] & bit, 1u);
+                    fma_if(sums[PREC == 0 ? 0 : h], lut(id[h]), xv[h], ~mc[h] & bit, 1u);
                 }
             }
+            V acc = sums[0];
+            if constexpr (PREC != 0) acc = cadd(cadd(acc, sums[1]), cadd(sums[2], sums[3]));
             finish_row<PREC>(r, (long long)tile * 32 + lane, acc, (rows_on & bit) != 0u);
             kt = kn;
         }
