@@ -261,7 +261,7 @@ struct edgpu_op_s {
             blk_ev.push_back(e);
         }
     }
-    int slab_hint[2] = {0, 0};        // [precision]: the slab product's cache hints (chosen by the autotuner)
+    int slab_hint[2] = {0, 0};        // [precision]: edgpu_op_slab_use's value less one, kept for its queries
     // Lanczos: pinned host memory the steps write their alpha, beta and norm to (three doubles a step and
     // three more), and the events after which those of the even and odd steps are there
     double* lz_slots = nullptr;

@@ -487,11 +487,9 @@ int record_api_error(int code, const std::string& msg);
 void launch_random_c128(int64_t n, uint64_t seed, double* dst, cudaStream_t st);
 void launch_c128_to_c64(int64_t n, const double* src, float* dst, cudaStream_t st);
 void launch_c64_to_c128(int64_t n, const float* src, double* dst, int accumulate, cudaStream_t st);
-void launch_scale_c128(int64_t n, double s, double* v, cudaStream_t st);
 void launch_conj_c128(int64_t n, double* v, cudaStream_t st);
 // Deterministic FP64 reductions through a per-call scratch buffer of at least dot_scratch_doubles().
 size_t dot_scratch_doubles();
-void launch_dot_c128(int64_t n, const double* a, const double* b, double* scratch, double* out_dev, cudaStream_t st);
 // (a norm: |a|, 1 / |a|)
 void launch_norm2_c128(int64_t n, const double* a, double* scratch, double* out_dev, cudaStream_t st);
 void launch_reduce_grad(int nblocks, int ncoupl, const double* partial, double* out_dev, cudaStream_t st);

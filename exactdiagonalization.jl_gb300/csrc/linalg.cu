@@ -62,13 +62,6 @@ __global__ void k_c64_to_c128(long long n, const float2* src, double2* dst, int 
     }
 }
 
-__global__ void k_scale_c128(long long n, double s, double2* v) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        double2 a = v[i];
-        v[i] = make_double2(a.x * s, a.y * s);
-    }
-}
-
 __global__ void k_conj_c128(long long n, double2* v) {
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         v[i].y = -v[i].y;
@@ -92,41 +85,27 @@ __device__ __forceinline__ double2 block_sum2(double2 v, double2* sh) {
     return r;
 }
 
-// Stage 1: <a, b> = sum conj(a_i) b_i over a grid-stride slice; partial per block.
-__global__ void k_dot_stage1(long long n, const double2* a, const double2* b, double2* partial, int norm_only) {
+// Norm, stage 1: |a_i|^2 over a grid-stride slice; partial per block.
+__global__ void k_norm_stage1(long long n, const double2* a, double2* partial) {
     __shared__ double2 sh[32];
     double2 s = make_double2(0.0, 0.0);
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const double2 u = a[i];
-        if (norm_only) {
-            s.x += u.x * u.x + u.y * u.y;
-        } else {
-            const double2 v = b[i];
-            s.x += u.x * v.x + u.y * v.y;
-            s.y += u.x * v.y - u.y * v.x;
-        }
+        s.x += u.x * u.x + u.y * u.y;
     }
     const double2 r = block_sum2(s, sh);
     if (threadIdx.x == 0) partial[blockIdx.x] = r;
 }
 
-// Stage 2: fixed-order sum of the partials; out = sum (or sqrt of its real part for a norm).
-__global__ void k_dot_stage2(int nparts, const double2* partial, double* out, int take_sqrt) {
+// Stage 2: fixed-order sum of the partials; out = the norm and its inverse.
+__global__ void k_norm_stage2(int nparts, const double2* partial, double* out) {
     __shared__ double2 sh[32];
     double2 s = make_double2(0.0, 0.0);
-    for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
-        s.x += partial[i].x;
-        s.y += partial[i].y;
-    }
+    for (int i = threadIdx.x; i < nparts; i += blockDim.x) s.x += partial[i].x;
     const double2 r = block_sum2(s, sh);
     if (threadIdx.x == 0) {
-        if (take_sqrt) {
-            out[0] = sqrt(r.x);
-            out[1] = 1.0 / out[0];
-        } else {
-            out[0] = r.x;
-            out[1] = r.y;
-        }
+        out[0] = sqrt(r.x);
+        out[1] = 1.0 / out[0];
     }
 }
 
@@ -491,12 +470,6 @@ void launch_c64_to_c128(int64_t n, const float* src, double* dst, int accumulate
     EDGPU_CUDA(cudaGetLastError());
 }
 
-void launch_scale_c128(int64_t n, double s, double* v, cudaStream_t st) {
-    if (n <= 0) return;
-    k_scale_c128<<<grid_for(n), 256, 0, st>>>(n, s, (double2*)v);
-    EDGPU_CUDA(cudaGetLastError());
-}
-
 void launch_conj_c128(int64_t n, double* v, cudaStream_t st) {
     if (n <= 0) return;
     k_conj_c128<<<grid_for(n), 256, 0, st>>>(n, (double2*)v);
@@ -505,15 +478,9 @@ void launch_conj_c128(int64_t n, double* v, cudaStream_t st) {
 
 size_t dot_scratch_doubles() { return 2 * (size_t)RED_BLOCKS; }
 
-void launch_dot_c128(int64_t n, const double* a, const double* b, double* scratch, double* out_dev, cudaStream_t st) {
-    k_dot_stage1<<<RED_BLOCKS, RED_THREADS, 0, st>>>(n, (const double2*)a, (const double2*)b, (double2*)scratch, 0);
-    k_dot_stage2<<<1, 1024, 0, st>>>(RED_BLOCKS, (const double2*)scratch, out_dev, 0);
-    EDGPU_CUDA(cudaGetLastError());
-}
-
 void launch_norm2_c128(int64_t n, const double* a, double* scratch, double* out_dev, cudaStream_t st) {
-    k_dot_stage1<<<RED_BLOCKS, RED_THREADS, 0, st>>>(n, (const double2*)a, nullptr, (double2*)scratch, 1);
-    k_dot_stage2<<<1, 1024, 0, st>>>(RED_BLOCKS, (const double2*)scratch, out_dev, 1);
+    k_norm_stage1<<<RED_BLOCKS, RED_THREADS, 0, st>>>(n, (const double2*)a, (double2*)scratch);
+    k_norm_stage2<<<1, 1024, 0, st>>>(RED_BLOCKS, (const double2*)scratch, out_dev);
     EDGPU_CUDA(cudaGetLastError());
 }
 
