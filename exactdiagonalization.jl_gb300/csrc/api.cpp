@@ -1233,6 +1233,7 @@ void launch_slab_passes(edgpu_op_s* op, int prec, const Blob& B, const void* x, 
     r.accumulate = y_c128 ? 0 : accumulate;
     r.padded = S.padded;
     r.occ = &S.occ[prec];
+    r.in_order = S.in_order;
     r.two_sums = S.in_order && r.n_rows >= SLAB_TWO_SUMS;
     r.tile_steps = S.tile_steps;
     const long long n_tiles = r.n_tiles;
@@ -1282,7 +1283,7 @@ void launch_slab_passes(edgpu_op_s* op, int prec, const Blob& B, const void* x, 
 
 // Row blocks of a host-buffer slab product (launch_slab_passes): EDGPU_SLAB_ROW_BLOCKS when set (1 to
 // 64); else 2 for mixed precision on sectors of 2^22 rows or more with at least 4 passes (on 6x6 k=0,
-// 252M rows: 101.8 -> 96.9 ms per H x with pinned complex128 buffers; 4 and 8 blocks gain no more,
+// 252M rows: 95.2 -> 89.5 ms per H x with pinned complex128 buffers; 4 blocks gain little more,
 // and the FP64 product is slower in blocks), 1 otherwise.
 int slab_row_blocks(const edgpu_op_s* op, int prec, int64_t n) {
     const char* v = std::getenv("EDGPU_SLAB_ROW_BLOCKS");
@@ -2744,7 +2745,7 @@ int edgpu_op_autotune(edgpu_op oh, int32_t precision, int32_t* rows_per_tile_out
     // rows per warp tile when there is no parent-state map); where the pair-flip schedule applies
     // (and the caller allows it), that schedule with 2 or 4 targets per step (4 with a map or a
     // target table) and 1, 2 or 4 lanes per row, and its target-table flavour (one lane per row).
-    // With a slab table (mixed precision), also its multi-pass product.
+    // With a slab table, also its multi-pass product.
     struct Cand { int pair, nt, table, rows, pf, uni, slab = 0, hint = 0; };
     std::vector<Cand> cands;
     build_blob(op, precision, 0, 0);

@@ -259,6 +259,7 @@ struct HxParams {
     int o_pdb, o_pdv, n_pdb;
     // FP64 gradient with one unit amplitude (build_blob): amplitude, the diagonal terms' change on a match over
     // it, offset of their value without one by coupling; no_y: only the gradient is wanted
+    int early;                 // the next launch may start with this one (set by the launch, see pdl_early)
     int grad_one, o_gbase, no_y;
     double grad_u, grad_kz;
     // adjoint target table (column-sorted; built by the ADJ passes of bond_tile): per column the
@@ -410,6 +411,9 @@ struct SlabRun {
     const unsigned* mask;           // this pass's steps (null on a padded table)
     int padded;
     int two_sums;                   // mixed precision, padded: two partial sums per row (else four)
+    int in_order;                   // the rows' entries are in the target table's order
+    int split;                      // several warps per tile (set by hx_slab_launch)
+    int early;                      // the next launch may start with this one (set by hx_slab_launch)
     const void* xs;                 // x from the slab's first column
     const void* x;                  // x (first pass: the diagonal's product)
     void* y;
@@ -448,6 +452,16 @@ constexpr int64_t SLAB_PAD_SMALL = 1 << 14;
 // on: the sums, bit for bit, that four and two lanes per row gave these sectors.
 constexpr int SLAB_IN_ORDER = 32;
 constexpr int64_t SLAB_TWO_SUMS = 1 << 16;
+// Tiles up to which several warps share one (padded tables; in mixed precision not on in-order ones, whose sums
+// are fixed above): four in mixed precision, eight in FP64.  Such a sector leaves most of the chip empty, and
+// its time is a row's chain of gathers: triangular 4x4 (28 tiles) complex64 3.6 -> 2.3 us, complex128
+// 11.5 -> 3.9; 5x4 (290) 5.4 -> 3.6 and 23 -> 11; chain L = 20 (290) complex128 5.0 -> 3.5.  At 525 tiles
+// (chain L = 21) complex128 takes 5.3 without and 6.2 with it, at 3520 (triangular 6x4) 69 and 74.
+constexpr int64_t SLAB_SPLIT = 400;
+// FP64, by-bond tables: four partial sums per row up to this many tiles (triangular 6x4, 3520 tiles: 69 us, 80
+// with one sum; 7x4, 44600 tiles: 491 and 487).  In-order tables have one (chain L = 26: 30 us, 36 with four,
+// whose registers leave room for fewer warps).
+constexpr int64_t SLAB_FP64_SUMS = 1 << 14;
 // Coefficient tables of at most this many entries go to registers (real) or to one copy per shared-
 // memory bank group (SLAB_REP_BYTES in all, which keeps eight blocks of the slab kernel per SM).
 constexpr int SLAB_REG_LUT = 4;

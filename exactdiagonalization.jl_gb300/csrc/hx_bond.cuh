@@ -131,16 +131,14 @@ __device__ __forceinline__ int bond_row_count(W b, const BondTables<W, PREC>& bt
     return cnt;
 }
 
-// acc (or sum) += element x of one target in FP64, with as few double-precision operations as its form
-// needs: the FP64 pipe takes 16 cycles of an SM for each of a warp's, and sets the pace of the FP64
-// products that look their targets up (chain L = 25, k = 3, 208,012 rows: 85 us a product with nine
-// operations a target, 70 us with these four; 61 us with the unrolled ring search of odd lengths).  An amplitude that all pairs share is applied to the row's sum; the ratio of
-// the orbit sizes is 1 for nearly all targets (equal) and skipped there.
-template <int GK>
-__device__ __forceinline__ void bond_add_fp64(const HxParams& p, const RowsSector<0>& sc, double2 a, const double* rrow,
-                                              bool equal, int sx, int g, double2 x, double2& acc, double2& sum) {
-    const bool arg = GK != GK_TRIVIAL && sc.want_arg;
-    if (p.bond_one && !arg) {
+// acc (or sum) += element x of one target in FP64 with trivial characters, with as few double-precision
+// operations as its form needs: the FP64 pipe takes 16 cycles of an SM for each of a warp's.  An amplitude
+// that all pairs share is applied to the row's sum; the ratio of the orbit sizes is 1 for nearly all
+// targets (equal) and skipped there.  (With characters this form gained on long rings, chain L = 25, k = 3,
+// but lost on tori, triangular 5x4, k = (1, 2): 86 -> 102 us; and maps, tables and all groups add alike.)
+__device__ __forceinline__ void bond_add_fp64(const HxParams& p, double2 a, const double* rrow, bool equal, int sx,
+                                              double2 x, double2& acc, double2& sum) {
+    if (p.bond_one) {
         if (equal) {
             sum.x += x.x;
             sum.y += x.y;
@@ -151,24 +149,18 @@ __device__ __forceinline__ void bond_add_fp64(const HxParams& p, const RowsSecto
         }
         return;
     }
-    if (p.bond_real && !arg) {
+    if (p.bond_real) {
         double f = a.x;
         if (!equal) f *= rrow[sx];
         acc.x = fma_r(f, x.x, acc.x);
         acc.y = fma_r(f, x.y, acc.y);
         return;
     }
-    double2 c = a;
-    if (arg) {
-        const double2 ph = sc.ph[sc.num[g]];
-        c = p.bond_one ? ph : p.bond_real ? cscale(ph, a.x) : cmul(a, ph);
-    }
-    if (!equal) c = cscale(c, rrow[sx]);
-    double2& t = p.bond_one ? sum : acc;
-    t.x = fma_r(c.x, x.x, t.x);
-    t.x = fma_r(-c.y, x.y, t.x);
-    t.y = fma_r(c.x, x.y, t.y);
-    t.y = fma_r(c.y, x.x, t.y);
+    if (!equal) a = cscale(a, rrow[sx]);
+    acc.x = fma_r(a.x, x.x, acc.x);
+    acc.x = fma_r(-a.y, x.y, acc.x);
+    acc.y = fma_r(a.x, x.y, acc.y);
+    acc.y = fma_r(a.y, x.x, acc.y);
 }
 
 // One warp tile of rows (32 / lpr consecutive rows of the sector, lpr lanes each) of the pair-flip
@@ -424,13 +416,15 @@ __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W,
                     a += gv.x * t.x + gv.y * t.y;
                 }
             }
-            if constexpr (PREC == 0) {
-                // equal: this target's ratio of the orbit sizes is 1; in the fused gradient, all of the warp's (a
-                // warp branch there, where the FP64 pipe is all that counts)
-                const bool equal = GK == GK_TRIVIAL || (GRAD ? !__any_sync(0xffffffffu, c[h] >= 0 && sx[h] != ri) : sx[h] == ri);
-                if (c[h] >= 0 && want_y)
-                    bond_add_fp64<GK>(p, sc, bt.amp[ti[h]], rrow, equal, sx[h], g[h], xv[h], acc, sum);
-            } else if (c[h] >= 0) {
+            if (PREC == 0 && !(GK != GK_TRIVIAL && sc.want_arg)) {
+                if constexpr (PREC == 0) {
+                    // equal: this target's ratio of the orbit sizes is 1; in the fused gradient, all of the warp's
+                    // (a warp branch there, where the FP64 pipe is all that counts)
+                    const bool equal = GK == GK_TRIVIAL ||
+                                       (GRAD ? !__any_sync(0xffffffffu, c[h] >= 0 && sx[h] != ri) : sx[h] == ri);
+                    if (c[h] >= 0 && want_y) bond_add_fp64(p, bt.amp[ti[h]], rrow, equal, sx[h], xv[h], acc, sum);
+                }
+            } else if (c[h] >= 0 && want_y) {
                 const V a = bt.amp[ti[h]];
                 if (GK == GK_TRIVIAL) {
                     acc = cadd(acc, cmul(a, xv[h]));
@@ -455,7 +449,7 @@ __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W,
     }
     if (FILL || ADJ != 0) return;
     if constexpr (PREC == 0) {
-        if (p.bond_one) {
+        if (p.bond_one && !(GK != GK_TRIVIAL && sc.want_arg)) {
             acc.x = fma_r(p.bond_a0, sum.x, acc.x);
             acc.y = fma_r(p.bond_a0, sum.y, acc.y);
         }
@@ -485,10 +479,11 @@ template <typename W, int GK, int PREC, int NT, bool UNI = false>
 __global__ void __launch_bounds__(HX_THREADS) hx_bond_kernel(const HxParams p) {
     typedef typename Cx<PREC>::V V;
     extern __shared__ __align__(16) unsigned char sm[];
-    // programmatic dependent launch: the next kernel in the stream may start its own prologue now;
-    // this kernel copies its (constant) tables, then waits for the previous kernel in the stream to
-    // complete before touching any vector or table it may have written
-    pdl_launch_dependents();
+    // programmatic dependent launch: the next kernel in the stream may start its own prologue now (a small
+    // grid) or once this one's blocks are done (see pdl_early); this kernel copies its (constant) tables,
+    // then waits for the previous kernel in the stream to complete before touching any vector or table
+    // it may have written
+    if (p.early) pdl_launch_dependents();
     {
         const int4* src = (const int4*)p.blob;
         int4* dst = (int4*)sm;
@@ -644,8 +639,17 @@ __global__ void __launch_bounds__(HX_THREADS) hx_bond_grad_kernel(const HxParams
 
 // Launch with programmatic stream serialisation: the kernel may begin while the previous kernel in
 // the stream finishes (it waits for it with griddepcontrol.wait before reading any vector).
+// Whether a launch lets the next one's blocks in at its start.  They then sit in whatever slots it leaves
+// free, which are unevenly spread, and the next launch runs so: with 440 blocks on 152 SMs of four slots
+// each as if on 110 SMs.  So only grids that leave half of the SMs empty do (chain L = 20, one slab, complex64
+// 2.48 against 2.58 us); the others let them in as their blocks exit (back to back, products without
+// tables, triangular 6x4, k = (1, 2): complex128 230 -> 180 us, complex64 123 -> 105).
+inline bool pdl_early(int blocks) { return 2 * blocks <= sm_count(); }
+
 template <typename K>
-void pdl_launch(K kern, const HxParams& p, int blocks, size_t smem, cudaStream_t st) {
+void pdl_launch(K kern, const HxParams& params, int blocks, size_t smem, cudaStream_t st) {
+    HxParams p = params;
+    p.early = pdl_early(blocks);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
     cfg.blockDim = dim3(HX_THREADS);

@@ -450,13 +450,14 @@ __device__ __forceinline__ void fma_if(double2& a, double2 c, double2 x, unsigne
 // group's gathers are under way, the entries of the group after the next are read, on through the
 // warp's tiles.  SUMS: partial sums per row, by the entry's place in its group; mixed precision takes
 // four (a row of 93 terms is half as far from its 64-bit sum as with one) or two (SlabRun::two_sums).
-// FP64: a step without entries (the last ones of a tile may be) is not added up, since the FP64 pipe sets
-// the pace (a warp's double-precision FMA takes 16 cycles of an SM).
+// FP64 takes four on small by-bond tables (SLAB_FP64_SUMS), else one, and does not add up a step without
+// entries (the last ones of a tile may be), since the FP64 pipe sets the pace (a warp's double-precision FMA
+// takes 16 cycles of an SM).
 template <int PREC, bool REAL, int LUTM, int SUMS>
 __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_pad_kernel(const SlabRun r) {
     typedef typename Cx<PREC>::V V;
     extern __shared__ __align__(16) unsigned char sm[];
-    pdl_launch_dependents();
+    if (r.early) pdl_launch_dependents();
     const SlabLut<PREC, REAL, LUTM> lut(r, sm);
     pdl_wait();
     const V* __restrict__ xs = (const V*)r.xs;
@@ -482,10 +483,11 @@ __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_pad_ker
                 const V x2 = xs[e.z & r.colmask], x3 = xs[e.w & r.colmask];
                 tp += 32;
                 const uint4 e2 = ld_stream(tp + 32);
+                const bool tail = q + 1 == qt;   // (only a tile's last group may have empty steps)
                 add(acc, e.x, x0, false);
-                add(SUMS == 1 ? acc : acc1, e.y, x1, true);
-                add(SUMS == 4 ? acc2 : acc, e.z, x2, true);
-                add(SUMS == 4 ? acc3 : SUMS == 2 ? acc1 : acc, e.w, x3, true);
+                add(SUMS == 1 ? acc : acc1, e.y, x1, tail);
+                add(SUMS == 4 ? acc2 : acc, e.z, x2, tail);
+                add(SUMS == 4 ? acc3 : SUMS == 2 ? acc1 : acc, e.w, x3, tail);
                 e = en;
                 en = e2;
             }
@@ -494,6 +496,50 @@ __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_pad_ker
             finish_row<PREC>(r, (long long)tile * 32 + lane, acc, true);
             qt = qn;
         }
+    }
+    if (!r.early) pdl_launch_dependents();
+}
+
+// Small sectors (SLAB_SPLIT): WAYS warps share a tile, each taking every WAYS-th group of steps, so that a row's
+// chain of gathers and additions is that much shorter; their sums are added in order.
+template <int PREC, bool REAL, int LUTM, int WAYS>
+__global__ void __launch_bounds__(HX_THREADS, 2) hx_slab_split_kernel(const SlabRun r) {
+    typedef typename Cx<PREC>::V V;
+    extern __shared__ __align__(16) unsigned char sm[];
+    __shared__ V part[HX_THREADS];
+    pdl_launch_dependents();
+    const SlabLut<PREC, REAL, LUTM> lut(r, sm);
+    pdl_wait();
+    const V* __restrict__ xs = (const V*)r.xs;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lim = (unsigned)r.n_lut << r.colbits;
+    const unsigned tile = (unsigned)r.tile0 + blockIdx.x * (HX_THREADS / 32 / WAYS) + warp / WAYS;
+    const bool act = tile < (unsigned)(r.tile0 + r.n_tiles);
+    V sum[4] = {};
+    if (act) {
+        const unsigned q1 = r.moff[tile + 1] >> 2;
+        unsigned q = (r.moff[tile] >> 2) + warp % WAYS;
+        const uint4* __restrict__ tp = (const uint4*)r.tab + ((size_t)q * 32 + lane);
+        uint4 e = q < q1 ? ld_stream(tp) : make_uint4(0u, 0u, 0u, 0u);
+        while (q < q1) {
+            const V x0 = xs[e.x & r.colmask], x1 = xs[e.y & r.colmask];
+            const V x2 = xs[e.z & r.colmask], x3 = xs[e.w & r.colmask];
+            tp += 32 * WAYS;
+            q += WAYS;
+            const uint4 en = q < q1 ? ld_stream(tp) : e;
+            fma_if(sum[0], lut(e.x >> r.colbits), x0, e.x, lim);
+            fma_if(sum[1], lut(e.y >> r.colbits), x1, e.y, lim);
+            fma_if(sum[2], lut(e.z >> r.colbits), x2, e.z, lim);
+            fma_if(sum[3], lut(e.w >> r.colbits), x3, e.w, lim);
+            e = en;
+        }
+    }
+    part[threadIdx.x] = cadd(cadd(sum[0], sum[1]), cadd(sum[2], sum[3]));
+    __syncthreads();
+    if (act && warp % WAYS == 0) {
+        V acc = part[threadIdx.x];
+        for (int w = 1; w < WAYS; ++w) acc = cadd(acc, part[threadIdx.x + 32 * w]);
+        finish_row<PREC>(r, (long long)tile * 32 + lane, acc, true);
     }
 }
 
@@ -505,7 +551,7 @@ template <int PREC, bool REAL, int LUTM>
 __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_kernel(const SlabRun r) {
     typedef typename Cx<PREC>::V V;
     extern __shared__ __align__(16) unsigned char sm[];
-    pdl_launch_dependents();
+    if (r.early) pdl_launch_dependents();
     const SlabLut<PREC, REAL, LUTM> lut(r, sm);
     pdl_wait();
     const V* __restrict__ xs = (const V*)r.xs;
@@ -554,6 +600,7 @@ __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_kernel(
             kt = kn;
         }
     }
+    if (!r.early) pdl_launch_dependents();
 }
 
 // x_c -> sqrt(|O_c|) x_c over the columns [c0, c1)
@@ -589,10 +636,10 @@ int xscale_blocks(long long n) {
 }
 
 template <typename K>
-void slab_pdl_launch(K kern, const SlabRun& r, int blocks, size_t smem, cudaStream_t st) {
+void slab_pdl_launch(K kern, const SlabRun& r, int blocks, int threads, size_t smem, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)blocks);
-    cfg.blockDim = dim3(HX_THREADS);
+    cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -603,20 +650,25 @@ void slab_pdl_launch(K kern, const SlabRun& r, int blocks, size_t smem, cudaStre
     EDGPU_CUDA(cudaLaunchKernelEx(&cfg, kern, r));
 }
 
-// Blocks of a launch over n_warps warps of work.  *occ: the blocks that fit on an SM, 0 until a table's
-// first launch (the query costs a microsecond of the host's five per launch).
+// A launch over n_warps warps of work.  With blocks_per_sm the block has half its usual size, so that an SM's
+// share can be cut finely: four blocks of 256 fit, and one of them is too much to leave free (6x6 from host
+// buffers, two row blocks: 89.5 ms, 103 with blocks of 256).
 template <typename K>
-int slab_blocks(K kern, size_t smem, long long n_warps, int* occ, int per_sm = 0) {
+void slab_go(K kern, SlabRun r, size_t smem, long long n_warps, cudaStream_t st) {
+    const int threads = r.blocks_per_sm ? HX_THREADS / 2 : HX_THREADS;
+    int own = 0, *occ = r.blocks_per_sm ? &own : r.occ;   // (the query costs a microsecond of the host's five per launch)
     if (*occ == 0) {
         raise_smem_limit((const void*)kern, smem);
-        EDGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, HX_THREADS, smem));
+        EDGPU_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, kern, threads, smem));
         *occ = std::max(1, *occ);
     }
     int n = *occ;
-    if (per_sm > 0) n = std::min(n, per_sm);
-    else if (per_sm < 0) n = std::max(1, n + per_sm);
-    const long long need = (n_warps + HX_THREADS / 32 - 1) / (HX_THREADS / 32);
-    return (int)std::max<long long>(1, std::min<long long>(need, (long long)std::max(1, n) * sm_count()));
+    if (r.blocks_per_sm > 0) n = std::min(n, r.blocks_per_sm);
+    else if (r.blocks_per_sm < 0) n = std::max(1, n + r.blocks_per_sm);
+    const long long need = (n_warps + threads / 32 - 1) / (threads / 32);
+    const int blocks = (int)std::max<long long>(1, std::min<long long>(need, (long long)n * sm_count()));
+    r.early = pdl_early(blocks);
+    slab_pdl_launch(kern, r, blocks, threads, smem, st);
 }
 
 template <typename W, int PREC>
@@ -677,13 +729,25 @@ template <int PREC, bool REAL, int LUTM>
 void slab_launch_k(const SlabRun& r, size_t smem, cudaStream_t st) {
     const long long warps = (r.n_tiles + r.chunk - 1) / r.chunk;
     if (r.padded) {
-        auto go = [&](auto k) { slab_pdl_launch(k, r, slab_blocks(k, smem, warps, r.occ, r.blocks_per_sm), smem, st); };
-        if constexpr (PREC == 0) go(hx_slab_pad_kernel<PREC, REAL, LUTM, 1>);
+        if (r.split) {
+                        constexpr int WAYS = PREC == 0 ? 8 : 4;
+            auto k = hx_slab_split_kernel<PREC, REAL, LUTM, WAYS>;
+            if (*r.occ == 0) {
+                raise_smem_limit((const void*)k, smem);
+                *r.occ = 1;
+            }
+            slab_pdl_launch(k, r, (int)((r.n_tiles * 32 * WAYS + HX_THREADS - 1) / HX_THREADS), HX_THREADS, smem, st);
+            return;
+        }
+        auto go = [&](auto k) { slab_go(k, r, smem, warps, st); };
+        if constexpr (PREC == 0) {
+            if (!r.in_order && r.n_rows <= SLAB_FP64_SUMS * 32) go(hx_slab_pad_kernel<PREC, REAL, LUTM, 4>);
+            else go(hx_slab_pad_kernel<PREC, REAL, LUTM, 1>);
+        }
         else if (r.two_sums) go(hx_slab_pad_kernel<PREC, REAL, LUTM, 2>);
         else go(hx_slab_pad_kernel<PREC, REAL, LUTM, 4>);
     } else {
-        auto k = hx_slab_kernel<PREC, REAL, LUTM>;
-        slab_pdl_launch(k, r, slab_blocks(k, smem, warps, r.occ, r.blocks_per_sm), smem, st);
+        slab_go(hx_slab_kernel<PREC, REAL, LUTM>, r, smem, warps, st);
     }
 }
 
@@ -703,6 +767,8 @@ void hx_slab_launch(int prec, const SlabRun& run, cudaStream_t st) {
     SlabRun r = run;
     // Consecutive tiles of a warp: about 128 steps together (the pipeline fills once for them), but at
     // least four chunks for every warp that fits, so that none is left with the last long one.
+    // (by the table's tiles, not the launch's: row blocks add up alike)
+    r.split = r.padded && r.n_rows <= SLAB_SPLIT * 32 && (prec == 0 || !r.in_order);
     r.chunk = (int)std::max<long long>(1, std::min<long long>({16, 128 / std::max(1, r.tile_steps),
                                                               r.n_tiles / ((long long)sm_count() * 48 * 4)}));
     const size_t csize = (size_t)(r.lut_real ? 1 : 2) * (prec == 0 ? 8 : 4);

@@ -686,8 +686,8 @@ class OperatorRepresentation:
 
     def build_slabs(self, slab_bytes: int = 54 << 20, max_bytes: Optional[int] = None) -> bool:
         """Build the column-slab table from the target table (which must exist): the product then runs
-        one pass per slab of slab_bytes of complex64 x, each gathering only from its slab (mixed
-        precision).  max_bytes defaults to a quarter of the free device memory.  Returns whether it
+        one pass per slab of slab_bytes of complex64 x, each gathering only from its slab (both
+        precisions).  max_bytes defaults to a quarter of the free device memory.  Returns whether it
         was built."""
         if max_bytes is None:
             import torch
