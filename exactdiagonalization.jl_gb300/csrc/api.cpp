@@ -437,21 +437,23 @@ struct BondClasses {
     bool cid_ok = true;               // the terms of every slot share one coupling id
     bool real = true;
 
-    // Whether every slot that a row can match has the same real amplitude a0 (n bits).
-    bool common_amplitude(int n, double& a0) const {
-        bool any = false;
-        a0 = 0.0;
+    // A slot (index (class n + start) 4 + pattern) whose real amplitude all slots that a row can match share for
+    // any values of the couplings: one coupling id, and one amplitude at the present values, which is neither 0 nor
+    // so small that different terms may round to it.  -1: none.  (n bits)
+    int common_slot(int n) const {
+        int slot = -1;
         for (int c = 0; c < ncls; ++c)
             for (int k = 0; k < BOND_MAXC; ++k)
                 for (int i = 0; i < n; ++i)
                     for (int v = 0; v < 4; ++v) {
                         if (!((comp[((size_t)c * BOND_MAXC + k) * 4 + 1 + (v >> 1)] >> i) & 1ull)) continue;
-                        const double* a = &amp[(((size_t)c * n + i) * 4 + v) * 2];
-                        if (a[1] != 0.0 || (any && a[0] != a0)) return false;
-                        a0 = a[0];
-                        any = true;
+                        const int at = (c * n + i) * 4 + v;
+                        const double* a = &amp[(size_t)at * 2];
+                        if (slot < 0) slot = at;
+                        if (a[1] != 0.0 || a[0] != amp[(size_t)slot * 2] || cid[at] != cid[slot]) return -1;
                     }
-        return any;
+        return slot >= 0 && cid_ok && std::fabs(amp[(size_t)slot * 2]) > 1e-280 &&
+                       std::isfinite(amp[(size_t)slot * 2]) ? slot : -1;
     }
 };
 
@@ -744,7 +746,7 @@ void build_blob(edgpu_op_s* op, int prec, int dir, int mode) {
     const int n_b = s.lay.nbits;
     p.bond_ncls = bc.ncls;
     p.bond_real = bc.real ? 1 : 0;
-    p.bond_one = bc.common_amplitude(n_b, p.bond_a0) ? 1 : 0;
+    p.bond_slot = bc.common_slot(n_b);
     p.o_bcomp = alloc((size_t)bc.ncls * BOND_MAXC * 4 * wsz);
     p.o_binfo = alloc((size_t)bc.ncls * 4);
     p.o_bflip = alloc((size_t)bc.ncls * n_b * wsz);
@@ -766,7 +768,9 @@ void build_blob(edgpu_op_s* op, int prec, int dir, int mode) {
     std::vector<double> gbase;
     if (grad_pair && prec == EDGPU_FP64 && g.den == 1 && bcu.real && n_pdb >= 0) {
         double u = 0.0, kap = 0.0;
-        bool ok = bcu.common_amplitude(n_b, u) && u != 0.0, any = false;
+        const int slot = bcu.common_slot(n_b);   // (the unit classes carry no coupling ids)
+        bool ok = slot >= 0, any = false;
+        if (ok) u = bcu.amp[(size_t)slot * 2];
         gbase.assign((size_t)op->n_coupl, 0.0);
         size_t used = 0;
         for (int c = 0; c < bc.ncls && ok; ++c) {

@@ -245,8 +245,9 @@ struct HxParams {
     int bond_ncls;
     int o_bcomp, o_binfo, o_bflip, o_bamp;    // shared-memory offsets of the class tables
     int bond_real;                            // every pair amplitude is real
-    int bond_one;                             // every pair that can match has the real amplitude bond_a0
-    double bond_a0;
+    int bond_slot;                            // >= 0: every pair that can match has this slot's amplitude, whatever
+                                              // the couplings (its value is read from the image, which a change of
+                                              // couplings rewrites under launches already captured)
     int bond_nt;                              // targets per lane and step: 2, or 4 (parent-state map only)
     int bond_pf;                              // target tables: x prefetched this many steps ahead (0: none)
     int bond_uni;                             // target tables: warp-uniform pair steps (bond_tile UNI)

@@ -138,7 +138,7 @@ __device__ __forceinline__ int bond_row_count(W b, const BondTables<W, PREC>& bt
 // but lost on tori, triangular 5x4, k = (1, 2): 86 -> 102 us; and maps, tables and all groups add alike.)
 __device__ __forceinline__ void bond_add_fp64(const HxParams& p, double2 a, const double* rrow, bool equal, int sx,
                                               double2 x, double2& acc, double2& sum) {
-    if (p.bond_one) {
+    if (p.bond_slot >= 0) {
         if (equal) {
             sum.x += x.x;
             sum.y += x.y;
@@ -207,7 +207,7 @@ __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W,
     const W b = kr >> sb;
     const int ri = (int)(kr & smask);
     V acc = czero<V>();
-    V sum = czero<V>();  // FP64: the targets' sum without the amplitude they share (p.bond_one)
+    V sum = czero<V>();  // FP64: the targets' sum without the amplitude they share (p.bond_slot)
     V gv = czero<V>();   // GRAD: gy of the row
     // GRAD in FP64, one unit amplitude (p.grad_one): kz = grad_kz Re(conj(gy_r) x_r), the diagonal terms'
     // share of every pair the row matches, in units of the amplitude
@@ -449,9 +449,10 @@ __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W,
     }
     if (FILL || ADJ != 0) return;
     if constexpr (PREC == 0) {
-        if (p.bond_one && !(GK != GK_TRIVIAL && sc.want_arg)) {
-            acc.x = fma_r(p.bond_a0, sum.x, acc.x);
-            acc.y = fma_r(p.bond_a0, sum.y, acc.y);
+        if (p.bond_slot >= 0 && !(GK != GK_TRIVIAL && sc.want_arg)) {
+            const double a0 = bt.amp[p.bond_slot].x;
+            acc.x = fma_r(a0, sum.x, acc.x);
+            acc.y = fma_r(a0, sum.y, acc.y);
         }
     }
     // partial sums of the row's lanes (fixed butterfly order)
