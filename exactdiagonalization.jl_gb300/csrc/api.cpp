@@ -745,7 +745,15 @@ void build_blob(edgpu_op_s* op, int prec, int dir, int mode) {
     }
     const int n_b = s.lay.nbits;
     p.bond_ncls = bc.ncls;
-    p.bond_real = bc.real ? 1 : 0;
+    // real for any values of the couplings, as launches already captured keep it: no imaginary term, or the terms'
+    // imaginary parts cancel within one coupling, which is then not 0
+    bool imag = false, hidden = !bc.cid_ok;
+    for (int t : offd)
+        if (op->unit[2 * t + 1] != 0.0) {
+            imag = true;
+            hidden = hidden || op->coupl[op->cid[t]] == 0.0;
+        }
+    p.bond_real = bc.real && !(imag && hidden) ? 1 : 0;
     p.bond_slot = bc.common_slot(n_b);
     p.o_bcomp = alloc((size_t)bc.ncls * BOND_MAXC * 4 * wsz);
     p.o_binfo = alloc((size_t)bc.ncls * 4);

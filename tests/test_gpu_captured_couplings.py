@@ -72,3 +72,28 @@ def test_replay_after_new_couplings(path, per_bond, prec):
     settings = [np.full(n_c, 0.7), 0.5 + rng.random(n_c), np.full(n_c, -1.3), np.ones(n_c)]
     _check_replays(E, opr, ora, ids, m, r, c, a, settings, prec)
 
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("path,span", [(p, s) for p in ("full", "direct", "map", "table", "momentum") for s in (1, 2)] +
+                                      [("slab", 2)])
+def test_replay_after_an_imaginary_coupling(path, span, prec):
+    """A Dzyaloshinskii-Moriya term (imaginary amplitudes) whose coupling is 0 at the capture, on the bonds of
+    the other coupling or on bonds of its own (a slab table needs the latter)."""
+    import edgpu as E
+    from edgpu import lattice
+    from edgpu.operators import pauli_matrix, simplify
+    space, ora, (m, r, c, a, ids) = _problem(E, path)
+    hs, _ = E.spin_half_system(L)
+    m, r, c, a = (list(v) for v in (m, r, c, a))
+    ids = [0] * len(m)
+    for i, j in [(i, (i + span) % L) for i in range(L)]:
+        t = simplify(0.25 * (pauli_matrix(hs, i, "x") * pauli_matrix(hs, j, "y") +
+                             (-1.0) * (pauli_matrix(hs, i, "y") * pauli_matrix(hs, j, "x"))))
+        for p in t.terms:
+            m.append(p.bitmask), r.append(p.bitrow), c.append(p.bitcol), a.append(p.amplitude), ids.append(1)
+    m, r, c = (np.array(v, dtype=np.uint64) for v in (m, r, c))
+    a, ids = np.array(a, dtype=complex), np.array(ids, dtype=np.int32)
+    assert np.abs(a[ids == 1].imag).min() > 0
+    opr = E.OperatorRepresentation.from_terms(space, m, r, c, a, coupling_ids=ids, couplings=[1.0, 0.0])
+    _prepare(opr, path)
+    _check_replays(E, opr, ora, ids, m, r, c, a, np.array([[1.0, 0.4], [0.6, 0.0], [0.6, -0.8]]), prec)
