@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "edgpu_internal.h"
+#include "lanczos_layout.h"
 
 using namespace edgpu;
 
@@ -4016,13 +4017,12 @@ int edgpu_lanczos(edgpu_op oh, int32_t precision, int32_t n_steps, int32_t reort
     DevBuf<double> V64, ww, small, psi, vstart;
     DevBuf<float> V32, y32;
     // one allocation for the small buffers, one for w and (with reorthogonalisation) w1
-    const size_t n_scratch = std::max(dot_scratch_doubles(), lanczos_scratch_doubles(m + 1));
-    const size_t n_h = 2 * (size_t)(m + 1), n_groups = (size_t)m / 16 + 2;
-    small.ensure(16 + n_scratch + n_h + 2 * n_groups);
-    struct { double* p; } scal{small.p}, scratch{scal.p + 16}, h{scratch.p + n_scratch};
-    double* d_hmax = h.p + n_h;
-    struct { unsigned* p; } tickets{(unsigned*)(d_hmax + n_groups)};
-    EDGPU_CUDA(cudaMemsetAsync(tickets.p, 0, n_groups * sizeof(unsigned), st));
+    const LanczosSmall sm = lanczos_small(m, g_sm_count);
+    small.ensure(sm.total);
+    struct { double* p; } scal{small.p + sm.scal}, scratch{small.p + sm.scratch}, h{small.p + sm.h};
+    double* d_hmax = small.p + sm.hmax;
+    struct { unsigned* p; } tickets{(unsigned*)(small.p + sm.tickets)};
+    EDGPU_CUDA(cudaMemsetAsync(tickets.p, 0, sm.n_groups * sizeof(unsigned), st));
     ww.ensure((reorth ? 4 : 2) * (size_t)N);
     struct { double* p; } w{ww.p}, w1{reorth ? ww.p + 2 * (size_t)N : nullptr};
     double* d_alpha = scal.p;      // [0]=re [1]=im of <v, w>

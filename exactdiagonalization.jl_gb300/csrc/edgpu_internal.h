@@ -508,10 +508,9 @@ size_t dot_scratch_doubles();
 // (a norm: |a|, 1 / |a|)
 void launch_norm2_c128(int64_t n, const double* a, double* scratch, double* out_dev, cudaStream_t st);
 void launch_reduce_grad(int nblocks, int ncoupl, const double* partial, double* out_dev, cudaStream_t st);
-// One Lanczos step.  scratch: lanczos_scratch_doubles(largest k); tickets: one zeroed counter per 16 basis
-// vectors (each launch leaves them zero).  Every null vector or scalar drops its term.
+// One Lanczos step.  scratch, tickets (one zeroed counter per 16 basis vectors, which each launch leaves
+// zero): lanczos_layout.h.  Every null vector or scalar drops its term.
 // alpha = <v, w> (re, im); with y32, w is first written as the widened complex64 vector y32.
-size_t lanczos_scratch_doubles(int kmax);
 void launch_lanczos_alpha(int64_t n, const double* v, double* w, const float* y32, double* scratch, unsigned* tickets,
                           double* alpha_dev, cudaStream_t st);
 // w1 = w - alpha v - beta u, h = V^H w1 (k vectors, complex128 or complex64), hmax = largest |Re h|, |Im h| of

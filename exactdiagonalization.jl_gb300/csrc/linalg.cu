@@ -8,12 +8,12 @@
 #include <utility>
 
 #include "edgpu_internal.h"
+#include "lanczos_layout.h"
 
 namespace edgpu {
 
 namespace {
 
-constexpr int RED_BLOCKS = 1024;
 constexpr int RED_THREADS = 256;
 
 unsigned grid_for(int64_t n, int threads = 256) {
@@ -129,11 +129,6 @@ __global__ void k_reduce_grad(int nblocks, int ncoupl, const double* partial, do
 // blocks' partial sums (a ticket counter tells it; no block waits).  Sector of 112,720 rows, 100 steps:
 // 42.8 -> 11.1 ms a run (before: two passes of a dot kernel with a block row per vector and a subtraction
 // kernel, separate reductions, a synchronisation per step).
-constexpr int LZ_THREADS = 256;
-constexpr int LZ_G = 16;         // basis vectors per block of the projections (accumulators in registers)
-constexpr int LZ_AXPY_THREADS = 128;
-constexpr int LZ_MAX_BLOCKS = 4096;
-
 __device__ __forceinline__ double2 lz_load(const double2* p) { return *p; }
 __device__ __forceinline__ double2 lz_load(const float2* p) {
     const float2 v = *p;
@@ -490,23 +485,8 @@ void launch_reduce_grad(int nblocks, int ncoupl, const double* partial, double* 
     EDGPU_CUDA(cudaGetLastError());
 }
 
-// Row blocks of the projections of K vectors: two blocks per SM (all that fit) over all groups of vectors.
-static int lz_row_blocks(int64_t n, int groups) {
-    const int64_t need = (n + LZ_THREADS - 1) / LZ_THREADS;
-    return (int)std::max<int64_t>(1, std::min<int64_t>(need, 2ll * std::max(1, sm_count()) / groups));
-}
-
-static int lz_groups(int k) { return std::max(1, (k + LZ_G - 1) / LZ_G); }
-
 static unsigned lz_correct_blocks(int64_t n) {
     return (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + LZ_AXPY_THREADS - 1) / LZ_AXPY_THREADS, LZ_MAX_BLOCKS));
-}
-
-size_t lanczos_scratch_doubles(int kmax) {
-    // partial sums of the projections (2 LZ_G doubles a block, at most two blocks per SM or one row block
-    // per group, and a norm per row block) and of the other kernels
-    const size_t blocks = std::max<size_t>((size_t)lz_groups(kmax), 2 * (size_t)std::max(1, sm_count()));
-    return std::max<size_t>(2 * LZ_G * blocks + blocks, 2 * LZ_MAX_BLOCKS);
 }
 
 void launch_lanczos_alpha(int64_t n, const double* v, double* w, const float* y32, double* scratch, unsigned* tickets,
@@ -531,7 +511,7 @@ void launch_lanczos_project(int64_t n, int k, const void* V, bool c64, int64_t l
                             double* scratch, unsigned* tickets, double* h_dev, double* hmax_dev, double* nrm2_dev,
                             cudaStream_t st) {
     const int groups = lz_groups(k);
-    const dim3 grid((unsigned)lz_row_blocks(n, groups), (unsigned)groups);
+    const dim3 grid((unsigned)lz_row_blocks(n, groups, sm_count()), (unsigned)groups);
     auto go = [&](auto kern, auto* basis) {
         kern<<<grid, LZ_THREADS, 0, st>>>(n, k, basis, ldv, (const double2*)w, (const double2*)v, (const double2*)u,
                                           alpha_dev, beta_dev, (double2*)w1, (double2*)scratch, (double2*)h_dev, hmax_dev,

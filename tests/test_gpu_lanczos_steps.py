@@ -7,6 +7,8 @@ all its steps; a run that stops when the eigenvalue has settled says nothing abo
 import numpy as np
 import pytest
 
+from oracle import oracle as O
+
 pytestmark = pytest.mark.gpu
 
 
@@ -52,3 +54,32 @@ def test_nearly_invariant_start(noise):
     r = E.lanczos(opr, 120, precision="fp64", reorth=True, v0=v0, tol=0.0, want_vector=True)
     _check(r, w)
     assert np.linalg.norm(M @ r.ground_state - r.e0 * r.ground_state) < 1e-7
+
+
+def test_more_vectors_than_blocks():
+    """More groups of 16 basis vectors than row blocks that fit on the GPU: each group has one row block, in
+    every step from there on.  The lowest Ritz values of the full-length run are eigenvalues, each once
+    (1e-9 of a sparse eigensolver's; copies would show a lost orthogonality); a run that stops early too."""
+    import scipy.linalg
+    import scipy.sparse.linalg
+    import torch
+    import edgpu as E
+    from edgpu import lattice
+    hs, _ = E.spin_half_system(15)
+    hsr = E.represent(E.HilbertSpaceSector(hs, 1))
+    rng = np.random.default_rng(4)
+    H = lattice.xxz_hamiltonian(hs, lattice.chain_bonds(15), 0.5 + rng.random(15), 0.5 + rng.random(15))
+    opr = E.represent(hsr, H)
+    steps = 32 * torch.cuda.get_device_properties(0).multi_processor_count + 5
+    assert steps < opr.dimension
+    basis = O.hs_get_basis_list(O.spin_half_sites(15), [(1,)])
+    terms = [(t.bitmask, t.bitrow, t.bitcol, t.amplitude) for t in H.terms]
+    A = scipy.sparse.linalg.LinearOperator((len(basis),) * 2, dtype=complex,
+                                           matvec=lambda v: O.apply_rows(basis, terms, np.ravel(v)))
+    w = np.sort(scipy.sparse.linalg.eigsh(A, k=8, which="SA", tol=1e-12, return_eigenvectors=False))
+    r = E.lanczos(opr, steps, precision="fp64", reorth=True, seed=3, tol=1e-12)
+    assert r.steps < 400 and abs(r.e0 - w[0]) < 1e-9 * abs(w[0])
+    r = E.lanczos(opr, steps, precision="fp64", reorth=True, seed=3, tol=0.0)
+    assert r.steps == steps
+    t = scipy.linalg.eigvalsh_tridiagonal(r.alphas, r.betas[:-1], select="i", select_range=(0, 7))
+    assert np.abs(t - w).max() < 1e-9 * np.abs(w).max()
