@@ -1,10 +1,17 @@
 // Sizes and places of the small device buffers of a Lanczos run (one allocation), by the largest number of
-// basis vectors and the number of SMs.  Plain C++: the host tests compile it without CUDA.
+// basis vectors and the number of SMs, and the rule for the precision of its correction.  Plain C++ too: the
+// host tests compile it without CUDA.
 #pragma once
 
 #include <algorithm>
 #include <cstddef>
 #include <cstdint>
+
+#ifdef __CUDACC__
+#define EDGPU_HOST_DEVICE __host__ __device__ inline
+#else
+#define EDGPU_HOST_DEVICE inline
+#endif
 
 namespace edgpu {
 
@@ -46,6 +53,18 @@ inline LanczosSmall lanczos_small(int m, int sms) {
     o.tickets = o.hmax + o.n_groups;
     o.total = o.tickets + o.n_groups;
     return o;
+}
+
+// Whether the sum of K basis vectors of norm 1 with coefficients h_k, taken off a vector of squared norm nrm2, may
+// be formed in single precision: |Re h_k|, |Im h_k| <= hmax.  Each component is a chain of at most two FMAs per
+// vector and LZ_CHUNK vectors (the chunks add up in FP64), of coefficients rounded to 24 bits and vectors cut to
+// 24 bits: a relative error of at most (2 min(K, LZ_CHUNK) + 4) 2^-24 in every term, so 2 (that) K hmax in the norm
+// of the sum.  The rule keeps it below 2^-54 of the vector's norm, half of a double's rounding.  Not for NaN,
+// infinities, or coefficients below 2^-900 (whose scale is not a double).
+constexpr int LZ_CHUNK = 256;
+EDGPU_HOST_DEVICE bool lz_single_precision(int K, double hmax, double nrm2) {
+    const double reach = hmax * (double)K * (double)(2 * (K < LZ_CHUNK ? K : LZ_CHUNK) + 4) * 2147483648.0;
+    return reach * reach <= nrm2 && hmax >= 0x1p-900;
 }
 
 }  // namespace edgpu

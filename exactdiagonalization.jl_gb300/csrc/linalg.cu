@@ -306,26 +306,24 @@ __device__ __forceinline__ float2 lz_top(const float2& v) { return v; }
 
 // w = w1 - alpha v - beta u - sum_k h_k V_k, beta_out = |w|; slot != null: alpha, beta_out and nrm2 for the
 // host.  After the recurrence the projections are at the level of rounding errors (1e-15 |w1|), so the
-// sum over k needs no more than a few digits to be exact beside w1: with hmax given and K hmax <= 2^-31
-// |w1|, it is taken in single precision (its error is then below 2^-54 |w1|, that of storing w), with h
-// scaled by a power of two near 1 / hmax; otherwise in FP64.  Basis vectors have elements of at most 1.
+// sum over k needs no more than a few digits beside w1: with hmax given and small enough for that
+// (lz_single_precision: its error is then below 2^-54 |w1|), it is taken in single precision, with h scaled by a
+// power of two near 1 / hmax; otherwise in FP64.  Basis vectors have elements of at most 1.
 // At K = 90 on 112,720 rows: 88 us in FP64, 28 us so.
 template <typename VT>
 __global__ void __launch_bounds__(LZ_AXPY_THREADS, 8)
 k_lz_correct(long long n, int K, const VT* V, long long ldv, const double2* h, const double* hmax, const double2* w1,
              const double2* v, const double2* u, const double* alpha, const double* beta, double2* w, double* partial, double* beta_out,
              const double* nrm2, double* slot, unsigned* ticket) {
-    __shared__ double2 hs[256];
-    __shared__ float2 hf[256];
+    __shared__ double2 hs[LZ_CHUNK];
+    __shared__ float2 hf[LZ_CHUNK];
     __shared__ double red[LZ_AXPY_THREADS / 32];
     __shared__ double sc[2];   // the scale of the single-precision sum and its inverse; 0: in FP64
     if (threadIdx.x == 0) {
         double big = 0.0;
         if (hmax)
             for (int g = 0; g < (K + LZ_G - 1) / LZ_G; ++g) big = fmax(big, hmax[g]);
-        const double reach = big * (double)K * 2147483648.0;
-        // (not for NaN, infinities, or projections below 2^-900)
-        const bool ok = hmax && reach * reach <= nrm2[0] && big >= 0x1p-900;
+        const bool ok = hmax && lz_single_precision(K, big, nrm2[0]);
         const int e = ok ? ilogb(big) : 0;
         sc[0] = ok ? scalbn(1.0, -e) : 0.0;
         sc[1] = scalbn(1.0, e);
@@ -349,9 +347,9 @@ k_lz_correct(long long n, int K, const VT* V, long long ldv, const double2* h, c
             x.x = fma(-b, t.x, x.x);
             x.y = fma(-b, t.y, x.y);
         }
-        for (int k0 = 0; k0 < K; k0 += 256) {
-            const int nk = min(256, K - k0);
-            if (K > 256 || i0 == (long long)blockIdx.x * LZ_AXPY_THREADS) {
+        for (int k0 = 0; k0 < K; k0 += LZ_CHUNK) {
+            const int nk = min(LZ_CHUNK, K - k0);
+            if (K > LZ_CHUNK || i0 == (long long)blockIdx.x * LZ_AXPY_THREADS) {
                 __syncthreads();
                 for (int k = threadIdx.x; k < nk; k += LZ_AXPY_THREADS) {
                     const double2 c = h[k0 + k];

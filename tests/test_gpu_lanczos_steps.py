@@ -83,3 +83,71 @@ def test_more_vectors_than_blocks():
     assert r.steps == steps
     t = scipy.linalg.eigvalsh_tridiagonal(r.alphas, r.betas[:-1], select="i", select_range=(0, 7))
     assert np.abs(t - w).max() < 1e-9 * np.abs(w).max()
+
+
+@pytest.mark.parametrize("L,q", [(10, 0), (11, 1)])   # 252 and 462 rows: steps on both sides of 256 vectors
+def test_full_spectrum(L, q):
+    """As many steps as rows: the tridiagonal matrix has the operator's eigenvalues (1e-10), which it has only
+    while the basis stays orthogonal."""
+    import scipy.linalg
+    import edgpu as E
+    from edgpu import lattice
+    hs, _ = E.spin_half_system(L)
+    rng = np.random.default_rng(L)
+    H = lattice.xxz_hamiltonian(hs, lattice.chain_bonds(L), 0.5 + rng.random(L), 0.5 + rng.random(L))
+    opr = E.represent(E.represent(E.HilbertSpaceSector(hs, q)), H)
+    w = np.linalg.eigvalsh(opr.todense())
+    r = E.lanczos(opr, opr.dimension, precision="fp64", reorth=True, seed=5, tol=0.0)
+    assert r.steps == opr.dimension
+    t = scipy.linalg.eigvalsh_tridiagonal(r.alphas, r.betas[:-1])
+    assert np.abs(t - w).max() < 1e-10 * np.abs(w).max()
+
+
+@pytest.mark.parametrize("refine", [False, True])
+def test_complex64_basis(refine):
+    """A mixed-precision run whose basis fits as complex64 only, reorthogonalised."""
+    import edgpu as E
+    opr = _operator(E, 16, 0, 1)
+    w = np.linalg.eigvalsh(opr.todense())
+    steps = 300
+    E.set_krylov_limit(12 * (steps + 1) * opr.dimension)
+    try:
+        r = E.lanczos(opr, steps, precision="mixed", reorth=True, seed=3, refine=refine, tol=1e-12 if refine else 0.0)
+        assert abs(r.e0 - w[0]) < (1e-10 if refine else 1e-5) * abs(w[0])
+        if not refine:
+            t = np.linalg.eigvalsh(np.diag(r.alphas) + np.diag(r.betas[:-1], 1) + np.diag(r.betas[:-1], -1))
+            assert np.abs(t[:4] - w[:4]).max() < 1e-5 * abs(w[0])
+    finally:
+        E.set_krylov_limit(0)
+
+
+def test_large_sector_second_projection():
+    """More than 2^20 rows (steps are then not issued ahead), from a start whose Krylov space is invariant up to
+    1e-7, against the same recurrence on the host with two projections in every step."""
+    import edgpu as E
+    from edgpu import lattice
+    L = 23
+    hs, _ = E.spin_half_system(L)
+    rng = np.random.default_rng(8)
+    H = lattice.xxz_hamiltonian(hs, lattice.chain_bonds(L), 1e-7 * (1.0 + rng.random(L)), 1.0 + rng.random(L))
+    opr = E.represent(E.represent(E.HilbertSpaceSector(hs, 1)), H)
+    N = opr.dimension
+    assert N > 1 << 20
+    v0 = np.zeros(N, dtype=complex)
+    v0[rng.integers(N, size=3)] = [0.8, 0.5, 0.3j]
+    steps = 8
+    r = E.lanczos(opr, steps, precision="fp64", reorth=True, v0=v0, tol=0.0)
+    basis = O.hs_get_basis_list(O.spin_half_sites(L), [(1,)])
+    terms = [(t.bitmask, t.bitrow, t.bitcol, t.amplitude) for t in H.terms]
+    V, alphas, betas = [v0 / np.linalg.norm(v0)], [], []
+    for j in range(steps):
+        w = O.apply_rows(basis, terms, V[j])
+        alphas.append(np.vdot(V[j], w).real)
+        for _ in range(2):
+            for u in V:
+                w = w - np.vdot(u, w) * u
+        betas.append(np.linalg.norm(w))
+        V.append(w / betas[-1])
+    assert betas[2] < 1e-5 < betas[1]
+    assert np.abs(r.alphas - alphas).max() < 1e-6 * np.abs(alphas).max()
+    assert np.abs(r.betas[:-1] / betas[:-1] - 1.0).max() < 1e-6
