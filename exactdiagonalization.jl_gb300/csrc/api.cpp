@@ -4014,17 +4014,16 @@ int edgpu_lanczos(edgpu_op oh, int32_t precision, int32_t n_steps, int32_t reort
     auto fits64 = [&](int k) { return (double)(k + 1) * (double)N * 16.0 <= limit; };
     auto fits32 = [&](int k) { return (double)(k + 1) * (double)N * 8.0 <= limit; };
 
-    DevBuf<double> V64, ww, small, psi, vstart;
+    DevBuf<double> V64, w, small, psi, vstart;
     DevBuf<float> V32, y32;
-    // one allocation for the small buffers, one for w and (with reorthogonalisation) w1
+    // one allocation for the small buffers (beside w, the run's vectors are those the Krylov limit counts)
     const LanczosSmall sm = lanczos_small(m, g_sm_count);
     small.ensure(sm.total);
     struct { double* p; } scal{small.p + sm.scal}, scratch{small.p + sm.scratch}, h{small.p + sm.h};
     double* d_hmax = small.p + sm.hmax;
     struct { unsigned* p; } tickets{(unsigned*)(small.p + sm.tickets)};
     EDGPU_CUDA(cudaMemsetAsync(tickets.p, 0, sm.n_groups * sizeof(unsigned), st));
-    ww.ensure((reorth ? 4 : 2) * (size_t)N);
-    struct { double* p; } w{ww.p}, w1{reorth ? ww.p + 2 * (size_t)N : nullptr};
+    w.ensure(2 * N);
     double* d_alpha = scal.p;      // [0]=re [1]=im of <v, w>
     double* d_beta[2] = {scal.p + 2, scal.p + 4};   // |w| and 1 / |w| of the even and odd steps
     double* d_tmp = scal.p + 6;
@@ -4098,10 +4097,11 @@ int edgpu_lanczos(edgpu_op oh, int32_t precision, int32_t n_steps, int32_t reort
             const double* u = j > 0 ? vec64(j - 1) : nullptr;
             const double* bu = j > 0 ? d_beta[(j - 1) & 1] : nullptr;
             if (cur_reorth) {
-                launch_lanczos_project(N, j + 1, basis, c64, N, w.p, vj, u, d_alpha, bu, w1.p, scratch.p, tickets.p,
-                                       h.p, d_hmax, d_nrm2, st);
-                launch_lanczos_correct(N, j + 1, basis, c64, N, h.p, d_hmax, w1.p, nullptr, nullptr, d_alpha, nullptr, w.p,
-                                       scratch.p, tickets.p, d_beta[j & 1], d_nrm2, slots + 3 * j, st);
+                // (both form w - alpha v - beta u: keeping it would take one more vector)
+                launch_lanczos_project(N, j + 1, basis, c64, N, w.p, vj, u, d_alpha, bu, scratch.p, tickets.p, h.p,
+                                       d_hmax, d_nrm2, st);
+                launch_lanczos_correct(N, j + 1, basis, c64, N, h.p, d_hmax, w.p, vj, u, d_alpha, bu, w.p, scratch.p,
+                                       tickets.p, d_beta[j & 1], d_nrm2, slots + 3 * j, st);
             } else {
                 launch_lanczos_correct(N, 0, basis, c64, N, nullptr, nullptr, w.p, vj, u, d_alpha, bu, w.p, scratch.p, tickets.p,
                                        d_beta[j & 1], nullptr, slots + 3 * j, st);
@@ -4121,9 +4121,9 @@ int edgpu_lanczos(edgpu_op oh, int32_t precision, int32_t n_steps, int32_t reort
                 // the projections took most of w away, so rounding errors of their size are left in it: once
                 // more, on v_{j+1} (the criterion of Daniel, Gragg, Kaufman and Stewart)
                 double* vn = vec64(j + 1);
-                launch_lanczos_project(N, j + 1, basis, c64, N, vn, nullptr, nullptr, nullptr, nullptr, w1.p, scratch.p,
+                launch_lanczos_project(N, j + 1, basis, c64, N, vn, nullptr, nullptr, nullptr, nullptr, scratch.p,
                                        tickets.p, h.p, d_hmax, d_nrm2, st);
-                launch_lanczos_correct(N, j + 1, basis, c64, N, h.p, d_hmax, w1.p, nullptr, nullptr, nullptr, nullptr, w.p,
+                launch_lanczos_correct(N, j + 1, basis, c64, N, h.p, d_hmax, vn, nullptr, nullptr, nullptr, nullptr, w.p,
                                        scratch.p, tickets.p, d_tmp, d_nrm2, slots + 3 * m, st);
                 launch_normalize(N, w.p, d_tmp, vn, cur_prec == EDGPU_MIXED ? vin32(j + 1) : nullptr, st);
                 EDGPU_CUDA(cudaStreamSynchronize(st));

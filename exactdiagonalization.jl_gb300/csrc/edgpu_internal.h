@@ -513,14 +513,13 @@ void launch_reduce_grad(int nblocks, int ncoupl, const double* partial, double* 
 // alpha = <v, w> (re, im); with y32, w is first written as the widened complex64 vector y32.
 void launch_lanczos_alpha(int64_t n, const double* v, double* w, const float* y32, double* scratch, unsigned* tickets,
                           double* alpha_dev, cudaStream_t st);
-// w1 = w - alpha v - beta u, h = V^H w1 (k vectors, complex128 or complex64), hmax = largest |Re h|, |Im h| of
-// every group of vectors (room for one per 16 vectors), nrm2 = |w1|^2
+// h = V^H w1 for w1 = w - alpha v - beta u (k vectors, complex128 or complex64), hmax = largest |Re h|, |Im h| of
+// every group of vectors (room for one per 16 vectors), nrm2 = |w1|^2; w1 itself is not kept
 void launch_lanczos_project(int64_t n, int k, const void* V, bool c64, int64_t ldv, const double* w, const double* v,
-                            const double* u, const double* alpha_dev, const double* beta_dev, double* w1,
-                            double* scratch, unsigned* tickets, double* h_dev, double* hmax_dev, double* nrm2_dev,
-                            cudaStream_t st);
-// w = w1 - alpha v - beta u - V h, beta_out = |w|, 1 / |w| (hmax, nrm2: those of the projections of w1, null for other
-// coefficients h); slot (host memory the device can address): alpha, |w| and
+                            const double* u, const double* alpha_dev, const double* beta_dev, double* scratch,
+                            unsigned* tickets, double* h_dev, double* hmax_dev, double* nrm2_dev, cudaStream_t st);
+// w = w1 - alpha v - beta u - V h (w1 may be w), beta_out = |w|, 1 / |w| (hmax, nrm2: those of the projections, null
+// for other coefficients h); slot (host memory the device can address): alpha, |w| and
 // nrm2 (without one: |w|^2)
 void launch_lanczos_correct(int64_t n, int k, const void* V, bool c64, int64_t ldv, const double* h_dev,
                             const double* hmax_dev, const double* w1, const double* v, const double* u, const double* alpha_dev,

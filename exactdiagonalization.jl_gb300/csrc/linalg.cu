@@ -189,14 +189,14 @@ __global__ void __launch_bounds__(LZ_THREADS) k_lz_alpha(long long n, const doub
     }
 }
 
-// w1 = w - alpha v - beta u, h_k = <V_k, w1> for the K vectors of the basis, hmax = the
-// largest of a group's |Re h|, |Im h|, nrm2 = |w1|^2.  Grid (row
-// blocks, groups of at most LZ_G vectors): every group forms w1 for itself, the first one stores it.
+// h_k = <V_k, w1> for the K vectors of the basis and w1 = w - alpha v - beta u, hmax = the largest of a group's
+// |Re h|, |Im h|, nrm2 = |w1|^2.  Grid (row blocks, groups of at most LZ_G vectors): every group forms w1 for
+// itself, and so does the correction.
 template <typename VT, int S>
 __global__ void __launch_bounds__(LZ_THREADS, 2)
 k_lz_project(long long n, int K, const VT* V, long long ldv, const double2* w, const double2* v, const double2* u,
-             const double* alpha, const double* beta, double2* w1, double2* partial, double2* h, double* hmax,
-             double* nrm2, unsigned* ticket) {
+             const double* alpha, const double* beta, double2* partial, double2* h, double* hmax, double* nrm2,
+             unsigned* ticket) {
     __shared__ double red[LZ_THREADS / 32][2 * LZ_G];
     __shared__ double nsum[LZ_THREADS / 32];
     const int KG = gridDim.y, RB = gridDim.x, grp = blockIdx.y;
@@ -222,10 +222,7 @@ k_lz_project(long long n, int K, const VT* V, long long ldv, const double2* w, c
             x.x = fma(-b, t.x, x.x);
             x.y = fma(-b, t.y, x.y);
         }
-        if (grp == 0) {
-            w1[i] = x;
-            nn = fma(x.x, x.x, fma(x.y, x.y, nn));
-        }
+        if (grp == 0) nn = fma(x.x, x.x, fma(x.y, x.y, nn));
         // (the groups have S or S - 1 vectors)
 #pragma unroll
         for (int g = 0; g < S - 1; ++g) cdot_acc(acc[g], lz_load(Vk + (size_t)g * ldv + i), x);
@@ -497,23 +494,21 @@ void launch_lanczos_alpha(int64_t n, const double* v, double* w, const float* y3
 
 template <typename VT, int... S>
 static constexpr std::array<void (*)(long long, int, const VT*, long long, const double2*, const double2*, const double2*,
-                                     const double*, const double*, double2*, double2*, double2*, double*, double*,
-                                     unsigned*),
+                                     const double*, const double*, double2*, double2*, double*, double*, unsigned*),
                             sizeof...(S)>
 lz_project_table(std::integer_sequence<int, S...>) {
     return {k_lz_project<VT, S + 1>...};
 }
 
 void launch_lanczos_project(int64_t n, int k, const void* V, bool c64, int64_t ldv, const double* w, const double* v,
-                            const double* u, const double* alpha_dev, const double* beta_dev, double* w1,
-                            double* scratch, unsigned* tickets, double* h_dev, double* hmax_dev, double* nrm2_dev,
-                            cudaStream_t st) {
+                            const double* u, const double* alpha_dev, const double* beta_dev, double* scratch,
+                            unsigned* tickets, double* h_dev, double* hmax_dev, double* nrm2_dev, cudaStream_t st) {
     const int groups = lz_groups(k);
     const dim3 grid((unsigned)lz_row_blocks(n, groups, sm_count()), (unsigned)groups);
     auto go = [&](auto kern, auto* basis) {
         kern<<<grid, LZ_THREADS, 0, st>>>(n, k, basis, ldv, (const double2*)w, (const double2*)v, (const double2*)u,
-                                          alpha_dev, beta_dev, (double2*)w1, (double2*)scratch, (double2*)h_dev, hmax_dev,
-                                          nrm2_dev, tickets);
+                                          alpha_dev, beta_dev, (double2*)scratch, (double2*)h_dev, hmax_dev, nrm2_dev,
+                                          tickets);
         EDGPU_CUDA(cudaGetLastError());
     };
     const int most = (k + groups - 1) / groups;   // vectors of the largest group

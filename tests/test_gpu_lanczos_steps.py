@@ -151,3 +151,30 @@ def test_large_sector_second_projection():
     assert betas[2] < 1e-5 < betas[1]
     assert np.abs(r.alphas - alphas).max() < 1e-6 * np.abs(alphas).max()
     assert np.abs(r.betas[:-1] / betas[:-1] - 1.0).max() < 1e-6
+
+
+def test_memory_beside_the_basis():
+    """A reorthogonalised run holds the basis that the Krylov limit counts, one vector more, and small
+    buffers (the device's free memory watched from another thread)."""
+    import threading
+    import torch
+    import edgpu as E
+    opr = _operator(E, 27, 1, 0)
+    steps, vector = 100, 16 * opr.dimension
+    E.lanczos(opr, 5, precision="fp64", reorth=True, seed=3, tol=0.0)   # (the product's own tables)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    lowest, stop = [before], threading.Event()
+
+    def watch():
+        while not stop.is_set():
+            lowest.append(torch.cuda.mem_get_info()[0])
+
+    t = threading.Thread(target=watch)
+    t.start()
+    E.lanczos(opr, steps, precision="fp64", reorth=True, seed=3, tol=0.0)
+    stop.set()
+    t.join()
+    used = before - min(lowest)
+    assert vector * (steps + 1) < used
+    assert used < vector * (steps + 1) + vector + (4 << 20)
