@@ -145,6 +145,7 @@ struct VectorTables {
         long long rank_hi;             // entries of the high part's table
         int rank_split, rank_wide;     // low bits (0: no tables), 64-bit entries
         int by_rank;                   // a parent index is the state's colex rank
+        int popcount;                  // by_rank: the parent's words are all those of this many set bits
         int elem_bits;                 // index bits beside a 32-bit ring state
     };
     GroupBuffers gb;

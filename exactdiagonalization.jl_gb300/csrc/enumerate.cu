@@ -1572,6 +1572,8 @@ __global__ void __launch_bounds__(256) k_reduce(const PW* parent, long long n_pa
             }
             long long i;
             if (t.by_rank) {
+                // (a flip may take a member out of the parent's sector)
+                if (__popcll((unsigned long long)m) != t.popcount) continue;
                 i = parent_rank<W>(m, t, C);
             } else {
                 long long lo = 0, len = n_parent;
@@ -1636,6 +1638,7 @@ const VectorTables& vector_tables(const Space& red, const Space& parent) {
     t.elem_bits = red.lay.nbits + pb <= 32 ? pb : 0;
     // the parent index is the colex rank where the parent is all words of a popcount
     t.by_rank = parent.lay.popcount >= 0 ? 1 : 0;
+    t.popcount = parent.lay.popcount;
     const int n = parent.lay.nbits;
     if (t.by_rank && n >= 2 && n <= RANK_SPLIT_BITS) {
         const std::vector<unsigned long long> T = split_rank_table(n, parent.lay.popcount);

@@ -59,3 +59,30 @@ def test_general_group(flip):
     want = np.where(idx >= 0, amp * small[np.maximum(idx, 0)], 0)
     assert np.max(np.abs(large.cpu().numpy() - want)) < 1e-13 * np.max(np.abs(small))
     assert np.max(np.abs(E.symmetry_reduce(rh, large).cpu().numpy() - small)) < 1e-12 * np.max(np.abs(small))
+
+
+@pytest.mark.parametrize("L,q", [(8, 2), (10, 2), (10, -4), (12, 0), (9, 1)])
+@pytest.mark.parametrize("lazy", [False, True])
+def test_flips_out_of_the_sector(L, q, lazy):
+    """Translations times the spin flip on a sector that the flip leaves (all but 2Sz = 0): members of an orbit
+    outside the parent have no entry of the large vector.  Against the sums written out (1e-13)."""
+    import torch
+    import edgpu as E
+    hs, _ = E.spin_half_system(L)
+    hsr = E.represent(E.HilbertSpaceSector(hs, q), lazy=lazy)
+    full = (1 << L) - 1
+    ops, elems = [], []
+    for a, (t, chi) in enumerate(E.translation_symops(L, 1)):
+        for f, par in ((False, 1), (True, -1)):
+            ops.append((t * E.GlobalBitFlip(f) if f else t, chi * par))
+            elems.append((list(t.map), full if f else 0, chi * par))
+    rh = E.symmetry_reduce(hsr, ops)
+    index = {int(b): i for i, b in enumerate(O.popcount_basis(L, (L - q) // 2))}
+    large = O.complex_gaussian(len(index), 5)
+    want = np.zeros(rh.dimension, dtype=complex)
+    for r, rep in enumerate(int(b) for b in rh.basis_list):
+        images = [(sum(((rep >> i) & 1) << m[i] for i in range(L)) ^ f, chi) for m, f, chi in elems]
+        stab = sum(im == rep for im, _ in images)
+        want[r] = sum(chi * large[index[im]] for im, chi in images if im in index) * np.sqrt(stab / len(elems)) / stab
+    got = E.symmetry_reduce(rh, torch.from_numpy(large).cuda()).cpu().numpy()
+    assert np.abs(got - want).max(initial=0.0) < 1e-13 * 2 * L * np.abs(large).max()
