@@ -93,6 +93,9 @@ struct Space {
     int rank_split = 0;              // > 0: split rank tables A (high bits) and B (rank_split low bits)
     uint64_t map_gen = 0;            // bumped whenever the map is built or freed
     mutable VectorTables* vec = nullptr;   // tables of the vector maps to and from the parent (on first use)
+    // a parent's split colex rank tables for the vector maps of all its reduced spaces (parent_rank_table)
+    mutable void* d_vec_rank = nullptr;
+    mutable std::mutex vec_rank_mu;
     ~Space();
 };
 // Build (or free) the parent-state map of a reduced space; false when it does not apply or would
@@ -134,14 +137,14 @@ struct GroupBuffers {
 };
 
 // Device tables of a reduced space's vector maps (reduce_vector): amplitudes chi sqrt(|stab| / |G|) by
-// (orbit-size index, character numerator), phases by numerator, sqrt(|stab| / |G|) / |stab| by orbit-size
-// index, and the split colex rank tables of a popcount parent.
+// (orbit-size index, character numerator), phases by numerator and sqrt(|stab| / |G|) / |stab| by orbit-size
+// index.
 struct VectorTables {
     struct Dev {
         const double2* ampl;
         const double2* phase;
         const double* inv_norm;
-        const void* rank;
+        const void* rank;              // the parent's split rank tables (set for a reduction only)
         long long rank_hi;             // entries of the high part's table
         int rank_split, rank_wide;     // low bits (0: no tables), 64-bit entries
         int by_rank;                   // a parent index is the state's colex rank
@@ -151,7 +154,6 @@ struct VectorTables {
     GroupBuffers gb;
     double2* d_ampl = nullptr;
     double* d_inv = nullptr;
-    void* d_rank = nullptr;
     Dev dev{};
     VectorTables() = default;
     VectorTables(const VectorTables&) = delete;

@@ -887,13 +887,13 @@ Space::~Space() {
     if (d_dir) cudaFree(d_dir);
     if (d_map) cudaFree(d_map);
     if (d_rank) cudaFree(d_rank);
+    if (d_vec_rank) cudaFree(d_vec_rank);
     delete vec;
 }
 
 VectorTables::~VectorTables() {
     if (d_ampl) cudaFree(d_ampl);
     if (d_inv) cudaFree(d_inv);
-    if (d_rank) cudaFree(d_rank);
 }
 
 void enumerate_parent(Space& s, cudaStream_t st) {
@@ -1639,20 +1639,38 @@ const VectorTables& vector_tables(const Space& red, const Space& parent) {
     // the parent index is the colex rank where the parent is all words of a popcount
     t.by_rank = parent.lay.popcount >= 0 ? 1 : 0;
     t.popcount = parent.lay.popcount;
-    const int n = parent.lay.nbits;
-    if (t.by_rank && n >= 2 && n <= RANK_SPLIT_BITS) {
-        const std::vector<unsigned long long> T = split_rank_table(n, parent.lay.popcount);
-        t.rank_split = n / 2;
-        t.rank_hi = 1ll << (n - n / 2);
-        t.rank_wide = host_binom(n, parent.lay.popcount) > 0xffffffffull ? 1 : 0;
-        const std::vector<unsigned> T32(T.begin(), T.end());
-        const size_t bytes = T.size() * (t.rank_wide ? 8 : 4);
-        EDGPU_CUDA(cudaMalloc(&v->d_rank, bytes));
-        EDGPU_CUDA(cudaMemcpy(v->d_rank, t.rank_wide ? (const void*)T.data() : (const void*)T32.data(), bytes, cudaMemcpyHostToDevice));
-        t.rank = v->d_rank;
-    }
     red.vec = v.release();
     return *red.vec;
+}
+
+// Fills in the rank tables of a popcount parent.  They depend on the parent alone (64 MB at 44 bits), so they are
+// built for the first reduction from it and kept with it; without room for them the kernel adds up the rank
+// bit by bit.
+void parent_rank_table(const Space& parent, VectorTables::Dev& t) {
+    const int n = parent.lay.nbits;
+    if (!t.by_rank || n < 2 || n > RANK_SPLIT_BITS) return;
+    const int wide = host_binom(n, parent.lay.popcount) > 0xffffffffull ? 1 : 0;
+    std::lock_guard<std::mutex> lk(parent.vec_rank_mu);
+    if (!parent.d_vec_rank) {
+        const std::vector<unsigned long long> T = split_rank_table(n, parent.lay.popcount);
+        const std::vector<unsigned> T32(T.begin(), T.end());
+        const size_t bytes = T.size() * (wide ? 8 : 4);
+        void* d = nullptr;
+        if (cudaMalloc(&d, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            return;
+        }
+        const cudaError_t e = cudaMemcpy(d, wide ? (const void*)T.data() : (const void*)T32.data(), bytes, cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) {
+            cudaFree(d);
+            throw Error(EDGPU_ERR_CUDA, std::string("rank table: ") + cudaGetErrorString(e));
+        }
+        parent.d_vec_rank = d;
+    }
+    t.rank_split = n / 2;
+    t.rank_hi = 1ll << (n - n / 2);
+    t.rank_wide = wide;
+    t.rank = parent.d_vec_rank;
 }
 
 template <typename W, typename PW, typename V>
@@ -1671,8 +1689,10 @@ void reduce_vector_t(const Space& red, const Space& parent, bool unreduce, const
                                                      (const V*)in, (V*)out);
     } else if (red.dim > 0) {
         const int blocks = (int)std::max<long long>(1, std::min<long long>((red.dim + 255) / 256, (long long)sm_count() * 16));
+        VectorTables::Dev t = vt.dev;
+        parent_rank_table(parent, t);
         k_reduce<W, PW, V><<<blocks, 256, 0, st>>>(pk, n_parent, binomial_table(), (const W*)red.d_keys, red.dim, red.sb,
-                                                   vt.gb.dev, vt.dev, (const V*)in, (V*)out);
+                                                   vt.gb.dev, t, (const V*)in, (V*)out);
     }
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);

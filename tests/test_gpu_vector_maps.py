@@ -86,3 +86,30 @@ def test_flips_out_of_the_sector(L, q, lazy):
         want[r] = sum(chi * large[index[im]] for im, chi in images if im in index) * np.sqrt(stab / len(elems)) / stab
     got = E.symmetry_reduce(rh, torch.from_numpy(large).cuda()).cpu().numpy()
     assert np.abs(got - want).max(initial=0.0) < 1e-13 * 2 * L * np.abs(large).max()
+
+
+def test_tables_are_kept_once():
+    """Sectors of one parent share its rank tables (32 MB at 44 bits), and symmetry_unreduce needs none."""
+    import torch
+    import edgpu as E
+    L, q = 44, 40
+    hs, _ = E.spin_half_system(L)
+    hsr = E.represent(E.HilbertSpaceSector(hs, q))
+    parent = O.popcount_basis(L, (L - q) // 2)
+    sectors = [E.symmetry_reduce(hsr, E.translation_symops(L, k)) for k in range(6)]
+    large = O.complex_gaussian(parent.size, 5)
+    lt = torch.from_numpy(large).cuda()
+    smalls = [E.random_state(s.dimension, 3, "fp64") for s in sectors]
+    torch.cuda.synchronize()
+    free = [torch.cuda.mem_get_info()[0]]
+    for s, v in zip(sectors, smalls):
+        E.symmetry_unreduce(s, v)
+    free.append(torch.cuda.mem_get_info()[0])
+    for k, s in enumerate(sectors):
+        maps, amps = O.translation_symops((L, 1), (k, 0))
+        red = O.symmetry_reduce(parent, *O.bit_layout(O.spin_half_sites(L)), maps, amps)
+        got = E.symmetry_reduce(s, lt).cpu().numpy()
+        assert np.abs(got - O.reduce_vector(red, large)).max() < 1e-13 * L * np.abs(large).max()
+    free.append(torch.cuda.mem_get_info()[0])
+    assert free[0] - free[1] < 16 << 20
+    assert free[1] - free[2] < (32 << 20) + (16 << 20)
