@@ -2589,7 +2589,7 @@ int edgpu_op_build_slabs(edgpu_op oh, int64_t slab_bytes, int64_t max_bytes, int
             const long long used = S.padded ? (long long)steps[q] * 32 : (long long)totals[q];
             const std::vector<unsigned> fill((size_t)(S.base[q + 1] - S.base[q] - used),
                                              S.padded ? (unsigned)n_ids << colbits : 0u);
-            EDGPU_CUDA(cudaMemcpy(S.tab + S.base[q] + used, fill.data(), fill.size() * 4, cudaMemcpyHostToDevice));
+            EDGPU_CUDA(cudaMemcpyAsync(S.tab + S.base[q] + used, fill.data(), fill.size() * 4, cudaMemcpyHostToDevice, st));
         }
         S.in_order = n_pass == 1 && S.tile_steps <= SLAB_IN_ORDER;
         sb.padded = S.padded;

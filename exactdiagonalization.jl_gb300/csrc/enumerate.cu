@@ -1639,6 +1639,7 @@ const VectorTables& vector_tables(const Space& red, const Space& parent) {
     // the parent index is the colex rank where the parent is all words of a popcount
     t.by_rank = parent.lay.popcount >= 0 ? 1 : 0;
     t.popcount = parent.lay.popcount;
+    EDGPU_CUDA(cudaStreamSynchronize(nullptr));   // copies from pageable memory may return before they end
     red.vec = v.release();
     return *red.vec;
 }
@@ -1660,7 +1661,8 @@ void parent_rank_table(const Space& parent, VectorTables::Dev& t) {
             cudaGetLastError();
             return;
         }
-        const cudaError_t e = cudaMemcpy(d, wide ? (const void*)T.data() : (const void*)T32.data(), bytes, cudaMemcpyHostToDevice);
+        cudaError_t e = cudaMemcpy(d, wide ? (const void*)T.data() : (const void*)T32.data(), bytes, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
         if (e != cudaSuccess) {
             cudaFree(d);
             throw Error(EDGPU_ERR_CUDA, std::string("rank table: ") + cudaGetErrorString(e));
