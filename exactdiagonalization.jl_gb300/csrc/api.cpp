@@ -212,8 +212,9 @@ struct edgpu_op_s {
         int padded = 0;                     // every step has 32 entries
         int tile_steps = 0;                 // mean steps of a tile in a pass
         int in_order = 0;                   // a row's entries in the target table's order
-        unsigned* off = nullptr;            // [n_pass][tiles + 1] first entries relative to the pass
-        unsigned* moff = nullptr;           // [n_pass][tiles + 1] first steps relative to the pass
+        unsigned char* cnt = nullptr;       // counted: [n_pass][dim] entries of each row in each pass
+        unsigned* off = nullptr;            // [n_pass][tiles + 1] first entries relative to the pass (counted: [n_pass][tiles])
+        unsigned* moff = nullptr;           // [n_pass][tiles + 1] first steps relative to the pass (null: counted)
         std::vector<long long> base;        // [n_pass + 1] first entry of each pass
         std::vector<long long> mbase;       // [n_pass + 1] first step of each pass
         int n_pass = 0, colbits = 0, n_ids = 0, den = 1, nd = 1;
@@ -289,6 +290,7 @@ struct edgpu_op_s {
         drop_host_graphs();
         if (slab.tab) cudaFree(slab.tab);
         if (slab.mask) cudaFree(slab.mask);
+        if (slab.cnt) cudaFree(slab.cnt);
         if (slab.off) cudaFree(slab.off);
         if (slab.moff) cudaFree(slab.moff);
         if (slab.cls) cudaFree(slab.cls);
@@ -1251,10 +1253,15 @@ void launch_slab_passes(edgpu_op_s* op, int prec, const Blob& B, const void* x, 
     r.tile_steps = S.tile_steps;
     const long long n_tiles = r.n_tiles;
     auto set_pass = [&](int q) {
-        r.off = S.off + (size_t)q * (n_tiles + 1);
-        r.moff = S.moff + (size_t)q * (n_tiles + 1);
         r.tab = S.tab + S.base[q];
-        r.mask = S.padded ? nullptr : S.mask + S.mbase[q];
+        if (S.cnt) {
+            r.off = S.off + (size_t)q * n_tiles;
+            r.cnt = S.cnt + (size_t)q * r.n_rows;
+        } else {
+            r.off = S.off + (size_t)q * (n_tiles + 1);
+            r.moff = S.moff + (size_t)q * (n_tiles + 1);
+            r.mask = S.padded ? nullptr : S.mask + S.mbase[q];
+        }
         r.xs = (const char*)x + (size_t)q * S.wc * esz;
         r.first = q == 0;
         r.last = q == S.n_pass - 1;
@@ -2532,8 +2539,10 @@ int edgpu_op_build_slabs(edgpu_op oh, int64_t slab_bytes, int64_t max_bytes, int
     sb.o_scratch = (int)align16(B.smem_bond);
     // tile offsets; a scaled table's orbit-size bytes and scaled-x buffer (complex128)
     const size_t n_off = (size_t)n_pass * (n_tiles + 1);
-    const size_t meta = n_off * 8 + (scaled ? (size_t)sp.dim * 17 : 0);
-    if ((double)meta > (double)max_bytes) {
+    const size_t scaled_bytes = scaled ? (size_t)sp.dim * 17 : 0;
+    const size_t meta = n_off * 8 + scaled_bytes;
+    const size_t meta_counted = (size_t)n_pass * (sp.dim + 4 * n_tiles) + scaled_bytes;   // the rows' counts instead of masks
+    if ((double)std::min(meta, meta_counted) > (double)max_bytes) {
         op->free_slabs();
         return EDGPU_OK;
     }
@@ -2564,7 +2573,7 @@ int edgpu_op_build_slabs(edgpu_op oh, int64_t slab_bytes, int64_t max_bytes, int
             require(totals[q] < ((unsigned long long)1 << 32) && steps[q] < ((unsigned long long)1 << 32),
                     EDGPU_ERR_ARG, "slab pass with 2^32 entries or more");
         }
-        // padded or with masks
+        // padded, with masks, or with the rows' counts
         constexpr int PAD = 2 * 128;   // entries after a padded pass: the product reads two groups ahead
         S.padded = pad_id && ((double)n_steps * 32.0 <= SLAB_PAD_MOST * (double)S.n || n_steps < SLAB_PAD_SMALL) &&
                    (double)meta + ((double)n_steps * 32.0 + (double)PAD * n_pass) * 4.0 <= (double)max_bytes;
@@ -2576,24 +2585,30 @@ int edgpu_op_build_slabs(edgpu_op oh, int64_t slab_bytes, int64_t max_bytes, int
             S.base[q + 1] = S.base[q] + (S.padded ? (long long)steps[q] * 32 + PAD : ((long long)totals[q] + 4) / 4 * 4);
             S.mbase[q + 1] = S.mbase[q] + (S.padded ? 0 : (long long)steps[q]);
         }
-        const long long n_entries = S.base[n_pass], n_masks = S.mbase[n_pass];
-        if ((double)meta + ((double)n_entries + (double)n_masks) * 4.0 > (double)max_bytes) {
+        const bool counted = (double)meta + ((double)S.base[n_pass] + (double)S.mbase[n_pass]) * 4.0 > (double)max_bytes;
+        if (counted && (double)meta_counted + (double)S.n * 4.0 > (double)max_bytes) {
             op->free_slabs();
             return EDGPU_OK;
         }
-        EDGPU_CUDA(cudaMalloc(&S.tab, std::max<size_t>((size_t)n_entries * 4, 16)));
-        if (!S.padded) {
-            EDGPU_CUDA(cudaMalloc(&S.mask, std::max<size_t>((size_t)n_masks * 4, 16)));
+        if (counted) {   // no entries between the passes
+            S.padded = 0;
+            for (int q = 0; q < n_pass; ++q) S.base[q + 1] = S.base[q] + (long long)totals[q];
         }
+        const long long n_entries = S.base[n_pass], n_masks = S.mbase[n_pass];
+        EDGPU_CUDA(cudaMalloc(&S.tab, std::max<size_t>((size_t)n_entries * 4, 16)));
+        if (counted) EDGPU_CUDA(cudaMalloc(&S.cnt, std::max<size_t>((size_t)n_pass * sp.dim, 16)));
+        else if (!S.padded) EDGPU_CUDA(cudaMalloc(&S.mask, std::max<size_t>((size_t)n_masks * 4, 16)));
         for (int q = 0; q < n_pass; ++q) {   // after a pass: entries without effect on the slab's first column
             const long long used = S.padded ? (long long)steps[q] * 32 : (long long)totals[q];
             const std::vector<unsigned> fill((size_t)(S.base[q + 1] - S.base[q] - used),
                                              S.padded ? (unsigned)n_ids << colbits : 0u);
             EDGPU_CUDA(cudaMemcpyAsync(S.tab + S.base[q] + used, fill.data(), fill.size() * 4, cudaMemcpyHostToDevice, st));
         }
-        S.in_order = n_pass == 1 && S.tile_steps <= SLAB_IN_ORDER;
+        S.in_order = !counted && n_pass == 1 && S.tile_steps <= SLAB_IN_ORDER;
         sb.padded = S.padded;
         sb.in_order = S.in_order;
+        sb.counted = counted ? 1 : 0;
+        sb.cnt = S.cnt;
         sb.n_ids = (int)n_ids;
         d_amp.ensure((size_t)n_slots);
         d_base.ensure(2 * (size_t)n_pass);
@@ -2608,6 +2623,18 @@ int edgpu_op_build_slabs(edgpu_op oh, int64_t slab_bytes, int64_t max_bytes, int
         sb.mask = S.mask;
         sb.amp_id = d_amp.p;
         hx_slab_build(sp.w32, prec, 2, p, sb, st);
+        if (counted) {   // the offsets without the passes' totals, and no step offsets
+            unsigned* off = nullptr;
+            EDGPU_CUDA(cudaMalloc(&off, (size_t)n_pass * n_tiles * 4));
+            std::swap(off, S.off);
+            const cudaError_t e = cudaMemcpy2DAsync(S.off, (size_t)n_tiles * 4, off, (size_t)(n_tiles + 1) * 4,
+                                                    (size_t)n_tiles * 4, n_pass, cudaMemcpyDeviceToDevice, st);
+            cudaStreamSynchronize(st);
+            cudaFree(off);
+            EDGPU_CUDA(e);
+            cudaFree(S.moff);
+            S.moff = nullptr;
+        }
         EDGPU_CUDA(cudaStreamSynchronize(st));
         S.n_pass = n_pass;
         S.wc = wc;

@@ -382,7 +382,10 @@ void hx_adj_launch(bool w32, int prec, const HxParams& p, size_t smem, cudaStrea
 // is (column - q wc) | id << colbits.  Two forms: padded, 32 entries per step (a row without one has a
 // padding entry of id n_ids), four steps of a row side by side; or per step a 32-bit mask of the rows that
 // have an entry, and their entries in row order.  Per pass and tile a 32-bit offset of its first step and
-// (with masks) of its first entry, relative to the pass ([n_tiles + 1], the last one the total).
+// (with masks) of its first entry, relative to the pass ([n_tiles + 1], the last one the total).  Where neither
+// fits the caller's limit, a third form: step k holds every row's k-th entry, so that a byte per row and pass, its
+// number of entries, takes the masks' place (one pass over long rows has more than eight steps a tile and
+// pass, whose masks take more than that); with an offset per tile and pass ([n_tiles]).
 // id indexes the coefficient table: id = ((amplitude id x den + character index) x nd +
 // orbit-size index of the row) x nd + orbit-size index of the column.
 struct SlabBuild {
@@ -404,6 +407,8 @@ struct SlabBuild {
     int scaled;                     // ids without the orbit-size indices (amplitude id x den + character)
     int padded;                     // every step has 32 entries (no masks)
     int in_order;                   // one slab: step k holds every row's k-th entry, in the target table's order
+    int counted;                    // the same for any number of slabs, and the rows' counts kept (no masks)
+    unsigned char* cnt;             // [n_pass][n_rows] entries of a row in a pass (fill pass, counted)
     int n_ids;                      // coefficient ids (a padding entry has the id n_ids)
     int cap;                        // steps a warp of the fill pass lays out at a time (>= the most of one tile)
     int o_scratch;                  // shared-memory offset of the passes' scratch
@@ -412,7 +417,8 @@ struct SlabRun {
     const unsigned* off;            // this pass's first entries by tile [n_tiles + 1]
     const unsigned* moff;           // this pass's first steps by tile [n_tiles + 1]
     const unsigned* tab;            // this pass's entries
-    const unsigned* mask;           // this pass's steps (null on a padded table)
+    const unsigned* mask;           // this pass's steps (null on a padded or counted table)
+    const unsigned char* cnt;       // this pass's rows' counts (counted table, whose off is [n_tiles])
     int padded;
     int two_sums;                   // mixed precision, padded: two partial sums per row (else four)
     int in_order;                   // the rows' entries are in the target table's order

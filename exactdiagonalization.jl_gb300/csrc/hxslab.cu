@@ -191,6 +191,16 @@ __global__ void __launch_bounds__(HX_THREADS) hx_slab_fill_kernel(const HxParams
                         continue;
                     }
                     unsigned pending = __ballot_sync(0xffffffffu, q >= qa && q < qb);
+                    if (s.counted) {
+                        if ((pending >> lane) & 1u) {
+                            unsigned k = first[q - qa];
+                            while ((occ[k] >> lane) & 1u) ++k;
+                            ent[k * 32 + lane] = entry;
+                            atomicOr(&occ[k], 1u << lane);
+                        }
+                        __syncwarp();
+                        continue;
+                    }
                     while (pending) {
                         const int q0 = __shfl_sync(0xffffffffu, q, __ffs((int)pending) - 1);
                         unsigned rest = __ballot_sync(0xffffffffu, q == q0);
@@ -240,8 +250,14 @@ __global__ void __launch_bounds__(HX_THREADS) hx_slab_fill_kernel(const HxParams
                     continue;
                 }
                 unsigned* tab = s.tab + s.base[q] + s.off[q * stride + tile];
-                unsigned* mask = s.mask + s.mbase[q] + s.moff[q * stride + tile];
-                for (unsigned k = lane; k < S; k += 32) mask[k] = occ[f0 + k];
+                if (s.counted) {
+                    unsigned c = 0;
+                    while (c < S && ((occ[f0 + c] >> lane) & 1u)) ++c;
+                    if (act) s.cnt[(size_t)q * p.n_rows + row] = (unsigned char)c;
+                } else {
+                    unsigned* mask = s.mask + s.mbase[q] + s.moff[q * stride + tile];
+                    for (unsigned k = lane; k < S; k += 32) mask[k] = occ[f0 + k];
+                }
                 for (unsigned k = 0; k < S; ++k) {
                     const unsigned o = occ[f0 + k];
                     if ((o >> lane) & 1u) tab[__popc(o & below)] = ent[(f0 + k) * 32 + lane];
@@ -603,6 +619,55 @@ __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_kernel(
     if (!r.early) pdl_launch_dependents();
 }
 
+// The same through a table with the rows' counts (where the caller's limit has no room for masks): step k's
+// rows are those with more than k entries, so the masks come from ballots.
+template <int PREC, bool REAL, int LUTM>
+__global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_counted_kernel(const SlabRun r) {
+    typedef typename Cx<PREC>::V V;
+    extern __shared__ __align__(16) unsigned char sm[];
+    if (r.early) pdl_launch_dependents();
+    const SlabLut<PREC, REAL, LUTM> lut(r, sm);
+    pdl_wait();
+    const V* __restrict__ xs = (const V*)r.xs;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
+    const unsigned bit = 1u << lane, below = bit - 1u;
+    const long long tile_end = r.tile0 + r.n_tiles, hop = (long long)gridDim.x * wpb;
+    for (long long tile = r.tile0 + (long long)blockIdx.x * wpb + warp; tile < tile_end; tile += hop) {
+        const long long row = tile * 32 + lane;
+        const unsigned cnt = row < r.n_rows ? ld_stream(r.cnt + row) : 0u;
+        const unsigned steps = __reduce_max_sync(0xffffffffu, cnt);
+        unsigned e0 = ld_stream(r.off + tile);
+        // this row's entry of step k, moving e0 past the step (0 without one)
+        auto next = [&](unsigned k) {
+            const unsigned m = __ballot_sync(0xffffffffu, k < cnt);
+            const unsigned e = k < cnt ? ld_stream(r.tab + e0 + (unsigned)__popc(m & below)) : 0u;
+            e0 += (unsigned)__popc(m);
+            return e;
+        };
+        V sums[PREC == 0 ? 1 : 4] = {};   // partial sums, as hx_slab_pad_kernel's
+        unsigned e[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) e[h] = next(h);
+        for (unsigned k = 0; k < steps; k += 4) {
+            V xv[4];
+            unsigned id[4];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                xv[h] = xs[e[h] & r.colmask];
+                id[h] = e[h] >> r.colbits;
+            }
+#pragma unroll
+            for (int h = 0; h < 4; ++h) e[h] = next(k + 4 + h);
+#pragma unroll
+            for (int h = 0; h < 4; ++h) fma_if(sums[PREC == 0 ? 0 : h], lut(id[h]), xv[h], k + h, cnt);
+        }
+        V acc = sums[0];
+        if constexpr (PREC != 0) acc = cadd(cadd(acc, sums[1]), cadd(sums[2], sums[3]));
+        finish_row<PREC>(r, row, acc, cnt != 0u);
+    }
+    if (!r.early) pdl_launch_dependents();
+}
+
 // x_c -> sqrt(|O_c|) x_c over the columns [c0, c1)
 template <typename V, typename R>
 __global__ void k_slab_xscale(const V* __restrict__ x, const unsigned char* __restrict__ cls,
@@ -730,7 +795,7 @@ void slab_launch_k(const SlabRun& r, size_t smem, cudaStream_t st) {
     const long long warps = (r.n_tiles + r.chunk - 1) / r.chunk;
     if (r.padded) {
         if (r.split) {
-                        constexpr int WAYS = PREC == 0 ? 8 : 4;
+            constexpr int WAYS = PREC == 0 ? 8 : 4;
             auto k = hx_slab_split_kernel<PREC, REAL, LUTM, WAYS>;
             if (*r.occ == 0) {
                 raise_smem_limit((const void*)k, smem);
@@ -746,6 +811,8 @@ void slab_launch_k(const SlabRun& r, size_t smem, cudaStream_t st) {
         }
         else if (r.two_sums) go(hx_slab_pad_kernel<PREC, REAL, LUTM, 2>);
         else go(hx_slab_pad_kernel<PREC, REAL, LUTM, 4>);
+    } else if (r.cnt) {
+        slab_go(hx_slab_counted_kernel<PREC, REAL, LUTM>, r, smem, r.n_tiles, st);
     } else {
         slab_go(hx_slab_kernel<PREC, REAL, LUTM>, r, smem, warps, st);
     }
