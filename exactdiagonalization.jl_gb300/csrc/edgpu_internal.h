@@ -422,7 +422,7 @@ struct SlabRun {
     int padded;
     int two_sums;                   // mixed precision, padded: two partial sums per row (else four)
     int in_order;                   // the rows' entries are in the target table's order
-    int split;                      // several warps per tile (set by hx_slab_launch)
+    int split;                      // several warps per tile: SLAB_BY_GROUP or SLAB_BY_PLACE (set by hx_slab_launch)
     int early;                      // the next launch may start with this one (set by hx_slab_launch)
     const void* xs;                 // x from the slab's first column
     const void* x;                  // x (first pass: the diagonal's product)
@@ -462,12 +462,25 @@ constexpr int64_t SLAB_PAD_SMALL = 1 << 14;
 // on: the sums, bit for bit, that four and two lanes per row gave these sectors.
 constexpr int SLAB_IN_ORDER = 32;
 constexpr int64_t SLAB_TWO_SUMS = 1 << 16;
-// Tiles up to which several warps share one (padded tables; in mixed precision not on in-order ones, whose sums
-// are fixed above): four in mixed precision, eight in FP64.  Such a sector leaves most of the chip empty, and
-// its time is a row's chain of gathers: triangular 4x4 (28 tiles) complex64 3.6 -> 2.3 us, complex128
-// 11.5 -> 3.9; 5x4 (290) 5.4 -> 3.6 and 23 -> 11; chain L = 20 (290) complex128 5.0 -> 3.5.  At 525 tiles
-// (chain L = 21) complex128 takes 5.3 without and 6.2 with it, at 3520 (triangular 6x4) 69 and 74.
+// Several warps share a tile of a padded table where the table leaves most of the chip empty and a row's chain
+// of gathers and additions sets the time.
+// By group, by-bond tables of up to SLAB_SPLIT tiles: each warp takes every fourth (mixed) or eighth (FP64) group of
+// steps (triangular 4x4, 28 tiles, complex64 3.6 -> 2.3 us, complex128 11.5 -> 3.9; 5x4, 290 tiles, 5.4 -> 3.6 and
+// 23 -> 11).
+// By place, in-order tables, whose sums it keeps: four warps, each one step of every group.  Complex128 up to 1024
+// tiles (chain L = 14 2.6 us, 4.1 with a warp per tile; L = 20 3.0 and 5.0, 22 4.8 and 5.4; at 1838 tiles, L = 23,
+// 7.3 and 7.2), complex64 from 4 to 600 (L = 12, three tiles, 1.95 us and 1.86; L = 18 2.1 and 2.3, 21 2.4 and 2.6;
+// at 1003, L = 22, 3.7 and 2.9).  A block copies the coefficients for two tiles: only up to 16 KB of them.
+// In FP64 with complex coefficients and more than 16 steps by group there too (triangular 4x3 at k = 1 3.6 us, 4.1
+// by place).
+enum { SLAB_BY_GROUP = 1, SLAB_BY_PLACE = 2 };
 constexpr int64_t SLAB_SPLIT = 400;
+inline int slab_split(int prec, bool in_order, int64_t tiles, int tile_steps, bool real, size_t lut_bytes) {
+    const bool few = lut_bytes <= 16 * 1024;
+    if (prec != 0 && in_order) return few && tiles >= 4 && tiles <= 600 ? SLAB_BY_PLACE : 0;
+    if (in_order && few && tiles <= 1024 && (real || tile_steps <= 16)) return SLAB_BY_PLACE;
+    return tiles <= SLAB_SPLIT ? SLAB_BY_GROUP : 0;
+}
 // FP64, by-bond tables: four partial sums per row up to this many tiles (triangular 6x4, 3520 tiles: 69 us, 80
 // with one sum; 7x4, 44600 tiles: 491 and 487).  In-order tables have one (chain L = 26: 30 us, 36 with four,
 // whose registers leave room for fewer warps).

@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hx_slab_split_kernel(const Slab
     typedef typename Cx<PREC>::V V;
     extern __shared__ __align__(16) unsigned char sm[];
     __shared__ V part[HX_THREADS];
-    pdl_launch_dependents();
+    if (r.early) pdl_launch_dependents();
     const SlabLut<PREC, REAL, LUTM> lut(r, sm);
     pdl_wait();
     const V* __restrict__ xs = (const V*)r.xs;
@@ -557,6 +557,45 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hx_slab_split_kernel(const Slab
         for (int w = 1; w < WAYS; ++w) acc = cadd(acc, part[threadIdx.x + 32 * w]);
         finish_row<PREC>(r, (long long)tile * 32 + lane, acc, true);
     }
+    if (!r.early) pdl_launch_dependents();
+}
+
+// Four warps share a tile, warp w of them taking every group's step w: the sums per row of hx_slab_pad_kernel with
+// four partial sums, bit for bit, in chains a quarter as long (small in-order tables: slab_split).
+template <int PREC, bool REAL, int LUTM>
+__global__ void __launch_bounds__(HX_THREADS, 2) hx_slab_place_kernel(const SlabRun r) {
+    typedef typename Cx<PREC>::V V;
+    extern __shared__ __align__(16) unsigned char sm[];
+    __shared__ V part[HX_THREADS];
+    if (r.early) pdl_launch_dependents();
+    const SlabLut<PREC, REAL, LUTM> lut(r, sm);
+    pdl_wait();
+    const V* __restrict__ xs = (const V*)r.xs;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const unsigned lim = (unsigned)r.n_lut << r.colbits;
+    const unsigned tile = (unsigned)r.tile0 + blockIdx.x * (HX_THREADS / 128) + warp / 4;
+    const bool act = tile < (unsigned)(r.tile0 + r.n_tiles);
+    V sum = czero<V>();
+    if (act) {
+        unsigned q = r.moff[tile] >> 2;
+        const unsigned q1 = r.moff[tile + 1] >> 2;
+        const unsigned* __restrict__ tp = r.tab + ((size_t)q * 32 + lane) * 4 + (warp & 3);
+        unsigned e = *tp;   // (a pass ends with two groups of padding entries)
+        for (; q < q1; ++q) {
+            const V x0 = xs[e & r.colmask];
+            tp += 128;
+            const unsigned en = *tp;
+            fma_if(sum, lut(e >> r.colbits), x0, e, lim);
+            e = en;
+        }
+    }
+    part[threadIdx.x] = sum;
+    __syncthreads();
+    if (act && (warp & 3) == 0) {
+        const V* p = part + threadIdx.x;
+        finish_row<PREC>(r, (long long)tile * 32 + lane, cadd(cadd(p[0], p[32]), cadd(p[64], p[96])), true);
+    }
+    if (!r.early) pdl_launch_dependents();
 }
 
 // The same through a table with masks (large sectors in many passes, where padding would double the
@@ -794,22 +833,31 @@ template <int PREC, bool REAL, int LUTM>
 void slab_launch_k(const SlabRun& r, size_t smem, cudaStream_t st) {
     const long long warps = (r.n_tiles + r.chunk - 1) / r.chunk;
     if (r.padded) {
-        if (r.split) {
-            constexpr int WAYS = PREC == 0 ? 8 : 4;
-            auto k = hx_slab_split_kernel<PREC, REAL, LUTM, WAYS>;
+        // a block per HX_THREADS / (32 ways) tiles
+        auto shared_tiles = [&](auto k, int ways) {
             if (*r.occ == 0) {
                 raise_smem_limit((const void*)k, smem);
                 *r.occ = 1;
             }
-            slab_pdl_launch(k, r, (int)((r.n_tiles * 32 * WAYS + HX_THREADS - 1) / HX_THREADS), HX_THREADS, smem, st);
+            SlabRun s = r;
+            const int blocks = (int)((r.n_tiles * 32 * ways + HX_THREADS - 1) / HX_THREADS);
+            s.early = pdl_early(blocks);
+            slab_pdl_launch(k, s, blocks, HX_THREADS, smem, st);
+        };
+        if (r.split == SLAB_BY_PLACE) {
+            shared_tiles(hx_slab_place_kernel<PREC, REAL, LUTM>, 4);
+            return;
+        }
+        if (r.split) {
+            constexpr int WAYS = PREC == 0 ? 8 : 4;
+            shared_tiles(hx_slab_split_kernel<PREC, REAL, LUTM, WAYS>, WAYS);
             return;
         }
         auto go = [&](auto k) { slab_go(k, r, smem, warps, st); };
         if constexpr (PREC == 0) {
             if (!r.in_order && r.n_rows <= SLAB_FP64_SUMS * 32) go(hx_slab_pad_kernel<PREC, REAL, LUTM, 4>);
             else go(hx_slab_pad_kernel<PREC, REAL, LUTM, 1>);
-        }
-        else if (r.two_sums) go(hx_slab_pad_kernel<PREC, REAL, LUTM, 2>);
+        } else if (r.two_sums) go(hx_slab_pad_kernel<PREC, REAL, LUTM, 2>);
         else go(hx_slab_pad_kernel<PREC, REAL, LUTM, 4>);
     } else if (r.cnt) {
         slab_go(hx_slab_counted_kernel<PREC, REAL, LUTM>, r, smem, r.n_tiles, st);
@@ -834,12 +882,12 @@ void hx_slab_launch(int prec, const SlabRun& run, cudaStream_t st) {
     SlabRun r = run;
     // Consecutive tiles of a warp: about 128 steps together (the pipeline fills once for them), but at
     // least four chunks for every warp that fits, so that none is left with the last long one.
-    // (by the table's tiles, not the launch's: row blocks add up alike)
-    r.split = r.padded && r.n_rows <= SLAB_SPLIT * 32 && (prec == 0 || !r.in_order);
     r.chunk = (int)std::max<long long>(1, std::min<long long>({16, 128 / std::max(1, r.tile_steps),
                                                               r.n_tiles / ((long long)sm_count() * 48 * 4)}));
     const size_t csize = (size_t)(r.lut_real ? 1 : 2) * (prec == 0 ? 8 : 4);
     const size_t smem = (size_t)(r.n_lut + 1) * (r.lut_mode == 1 ? 128 : csize);   // (and a padding entry's id)
+    // (by the table's tiles, not the launch's: row blocks add up alike)
+    if (r.padded) r.split = slab_split(prec, r.in_order, (r.n_rows + 31) / 32, r.tile_steps, r.lut_real, smem);
     if (prec == 0) slab_launch_p<0>(r, smem, st);
     else slab_launch_p<1>(r, smem, st);
 }
