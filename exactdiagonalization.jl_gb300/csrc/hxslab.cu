@@ -467,11 +467,15 @@ __device__ __forceinline__ void fma_if(double2& a, double2 c, double2 x, unsigne
 // warp's tiles.  SUMS: partial sums per row, by the entry's place in its group; mixed precision takes
 // four (a row of 93 terms is half as far from its 64-bit sum as with one) or two (SlabRun::two_sums).
 // FP64 takes four on small by-bond tables (SLAB_FP64_SUMS), else one, and does not add up a step without
-// entries (the last ones of a tile may be), since the FP64 pipe sets the pace (a warp's double-precision FMA
-// takes 16 cycles of an SM).
+// entries (the last ones of a tile may be), since the FP64 pipe sets the pace (a warp's double-precision FMA takes
+// 16 cycles of an SM).  To keep it busy, the gathers run a
+// group ahead of the additions there (complex128, chain L = 27 at k = 1 98.3 -> 94.5 us, L = 28 104.3 -> 101.1;
+// triangular 6x5 at k = 1 3596 -> 3451, square 4x8 in two passes 5321 -> 5125); in mixed precision the registers
+// for that cost more than it gives (chain L = 24 5.5 -> 6.9 us).
 template <int PREC, bool REAL, int LUTM, int SUMS>
 __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_pad_kernel(const SlabRun r) {
     typedef typename Cx<PREC>::V V;
+    constexpr bool AHEAD = PREC == 0;
     extern __shared__ __align__(16) unsigned char sm[];
     if (r.early) pdl_launch_dependents();
     const SlabLut<PREC, REAL, LUTM> lut(r, sm);
@@ -479,6 +483,16 @@ __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_pad_ker
     const V* __restrict__ xs = (const V*)r.xs;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpb = blockDim.x >> 5;
     const unsigned lim = (unsigned)r.n_lut << r.colbits;   // padding entries: from here on
+    auto gather = [&](const uint4& g, V* x) {
+        x[0] = xs[g.x & r.colmask];
+        x[1] = xs[g.y & r.colmask];
+        x[2] = xs[g.z & r.colmask];
+        x[3] = xs[g.w & r.colmask];
+    };
+    auto add = [&](V& acc, unsigned g, const V& x, bool may_be_empty) {
+        if (PREC == 0 && may_be_empty && !__any_sync(0xffffffffu, g < lim)) return;
+        fma_if(acc, lut(g >> r.colbits), x, g, lim);
+    };
     // (rows are below 2^32, so tiles below 2^27)
     const unsigned tile_end = (unsigned)(r.tile0 + r.n_tiles), hop = gridDim.x * wpb * r.chunk;
     for (unsigned c0 = (unsigned)r.tile0 + (blockIdx.x * wpb + warp) * r.chunk; c0 < tile_end; c0 += hop) {
@@ -487,25 +501,27 @@ __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_pad_ker
         unsigned q = r.moff[tile] >> 2, qt = r.moff[tile + 1] >> 2;   // groups of four steps
         const uint4* __restrict__ tp = (const uint4*)r.tab + ((size_t)q * 32 + lane);
         uint4 e = ld_stream(tp), en = ld_stream(tp + 32);
-        auto add = [&](V& acc, unsigned g, const V& x, bool may_be_empty) {
-            if (PREC == 0 && may_be_empty && !__any_sync(0xffffffffu, g < lim)) return;
-            fma_if(acc, lut(g >> r.colbits), x, g, lim);
-        };
+        V x[4];
+        if (AHEAD) gather(e, x);
         for (; tile < t1; ++tile) {
             const unsigned qn = tile + 1 < t1 ? r.moff[tile + 2] >> 2 : qt;
             V acc = czero<V>(), acc1 = acc, acc2 = acc, acc3 = acc;
             for (; q < qt; ++q) {
-                const V x0 = xs[e.x & r.colmask], x1 = xs[e.y & r.colmask];
-                const V x2 = xs[e.z & r.colmask], x3 = xs[e.w & r.colmask];
+                V xn[4];
+                if (AHEAD) gather(en, xn);
+                else gather(e, x);
                 tp += 32;
                 const uint4 e2 = ld_stream(tp + 32);
                 const bool tail = q + 1 == qt;   // (only a tile's last group may have empty steps)
-                add(acc, e.x, x0, false);
-                add(SUMS == 1 ? acc : acc1, e.y, x1, tail);
-                add(SUMS == 4 ? acc2 : acc, e.z, x2, tail);
-                add(SUMS == 4 ? acc3 : SUMS == 2 ? acc1 : acc, e.w, x3, tail);
+                add(acc, e.x, x[0], false);
+                add(SUMS == 1 ? acc : acc1, e.y, x[1], tail);
+                add(SUMS == 4 ? acc2 : acc, e.z, x[2], tail);
+                add(SUMS == 4 ? acc3 : SUMS == 2 ? acc1 : acc, e.w, x[3], tail);
                 e = en;
                 en = e2;
+#pragma unroll
+                for (int h = 0; h < 4; ++h)
+                    if (AHEAD) x[h] = xn[h];
             }
             if (SUMS == 4) acc = cadd(cadd(acc, acc1), cadd(acc2, acc3));
             if (SUMS == 2) acc = cadd(acc, acc1);
@@ -601,10 +617,11 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hx_slab_place_kernel(const Slab
 // The same through a table with masks (large sectors in many passes, where padding would double the
 // table: on 6x6 it would take 54 ms instead of 64, and 164 GB instead of 80): a lane finds its entry of a
 // step by counting the rows before it, and the pipeline reads the next group's entries and the masks
-// after those.
+// after those; in FP64 all of it a group earlier, for the gathers (6x6 131.4 -> 128.3 ms).
 template <int PREC, bool REAL, int LUTM>
 __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_kernel(const SlabRun r) {
     typedef typename Cx<PREC>::V V;
+    constexpr bool AHEAD = PREC == 0;
     extern __shared__ __align__(16) unsigned char sm[];
     if (r.early) pdl_launch_dependents();
     const SlabLut<PREC, REAL, LUTM> lut(r, sm);
@@ -622,31 +639,51 @@ __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_kernel(
         unsigned e0 = ld_stream(r.off + tile);
         unsigned k = r.moff[tile], kt = r.moff[tile + 1];
         const unsigned k1 = r.moff[t1];   // the tiles' steps (each tile has a multiple of four)
-        unsigned m[4], mn[4], e[4];
+        // m: the masks of this group, mn: of the next ones; x: the elements of this group (AHEAD) and
+        // id: their coefficients; e: the entries of this group, or (AHEAD) of the next
+        constexpr int NEXT = AHEAD ? 2 : 1;
+        unsigned m[4], mn[NEXT][4], e[4], id[4];
+        V x[4];
         ld_masks(mask, k, k1, m);
-        ld_masks(mask, k + 4, k1, mn);
+#pragma unroll
+        for (int d = 0; d < NEXT; ++d) ld_masks(mask, k + 4 * (d + 1), k1, mn[d]);
         ld_entries(tab, m, below, e0, e);
+        if (AHEAD) {
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                x[h] = xs[e[h] & r.colmask];
+                id[h] = e[h] >> r.colbits;
+            }
+            ld_entries(tab, mn[0], below, e0, e);
+        }
         for (; tile < t1; ++tile) {
             const unsigned kn = tile + 1 < t1 ? r.moff[tile + 2] : kt;
             V sums[PREC == 0 ? 1 : 4] = {};   // partial sums, as hx_slab_pad_kernel's
             unsigned rows_on = 0;             // rows of the tile with entries in this pass
             for (; k < kt; k += 4) {
-                V xv[4];
-                unsigned id[4], mc[4];
+                V xn[4];
+                unsigned idn[4], m2[4];
 #pragma unroll
                 for (int h = 0; h < 4; ++h) {
-                    xv[h] = xs[e[h] & r.colmask];
-                    id[h] = e[h] >> r.colbits;
-                    mc[h] = m[h];
-                    rows_on |= m[h];
-                    m[h] = mn[h];
+                    xn[h] = xs[e[h] & r.colmask];
+                    idn[h] = e[h] >> r.colbits;
                 }
-                ld_entries(tab, m, below, e0, e);
-                ld_masks(mask, k + 8, k1, mn);
+                ld_entries(tab, mn[NEXT - 1], below, e0, e);
+                ld_masks(mask, k + 4 * (NEXT + 1), k1, m2);
 #pragma unroll
                 for (int h = 0; h < 4; ++h) {
-                    if (PREC == 0 && h > 0 && mc[h] == 0u) continue;
-                    fma_if(sums[PREC == 0 ? 0 : h], lut(id[h]), xv[h], ~mc[h] & bit, 1u);
+                    rows_on |= m[h];
+                    if (PREC == 0 && h > 0 && m[h] == 0u) continue;
+                    fma_if(sums[PREC == 0 ? 0 : h], lut(AHEAD ? id[h] : idn[h]), AHEAD ? x[h] : xn[h], ~m[h] & bit, 1u);
+                }
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    x[h] = xn[h];
+                    id[h] = idn[h];
+                    m[h] = mn[0][h];
+#pragma unroll
+                    for (int d = 0; d + 1 < NEXT; ++d) mn[d][h] = mn[d + 1][h];
+                    mn[NEXT - 1][h] = m2[h];
                 }
             }
             V acc = sums[0];
