@@ -467,24 +467,25 @@ constexpr int64_t SLAB_TWO_SUMS = 1 << 16;
 // By group, by-bond tables of up to SLAB_SPLIT tiles: each warp takes every fourth (mixed) or eighth (FP64) group of
 // steps (triangular 4x4, 28 tiles, complex64 3.6 -> 2.3 us, complex128 11.5 -> 3.9; 5x4, 290 tiles, 5.4 -> 3.6 and
 // 23 -> 11).
-// By place, in-order tables, whose sums it keeps: four warps, each one step of every group.  Complex128 up to 1024
-// tiles (chain L = 14 2.6 us, 4.1 with a warp per tile; L = 20 3.0 and 5.0, 22 4.8 and 5.4; at 1838 tiles, L = 23,
-// 7.3 and 7.2), complex64 from 4 to 600 (L = 12, three tiles, 1.95 us and 1.86; L = 18 2.1 and 2.3, 21 2.4 and 2.6;
-// at 1003, L = 22, 3.7 and 2.9).  A block copies the coefficients for two tiles: only up to 16 KB of them.
-// In FP64 with complex coefficients and more than 16 steps by group there too (triangular 4x3 at k = 1 3.6 us, 4.1
-// by place).
+// By place: four warps, each one step of every group, with the sums of one warp's four partial sums.  In-order
+// tables in complex128 up to 1024 tiles (chain L = 14 2.6 us, 4.1 with a warp per tile; L = 20 3.0 and 5.0, 22 4.8
+// and 5.4; at 1838 tiles, L = 23, 7.3 and 7.2), in complex64 from 4 to 600 (L = 12, three tiles, 1.95 us and 1.86;
+// L = 18 2.1 and 2.3, 21 2.4 and 2.6; at 1003, L = 22, 3.7 and 2.9).  In FP64 with complex coefficients and more
+// than 16 steps by group there too (triangular 4x3 at k = 1 3.6 us, 4.1 by place).
+// By-bond tables of one pass in complex128 up to SLAB_FP64_SUMS tiles, whose rows have four partial sums: square
+// 5x5 48.0 us, 52.8 with a warp per tile and four sums, 49.6 with one sum; triangular 6x4 at k = 1 68.3, 70.1 and
+// 67.9.  Larger ones have one sum (7x4, 44600 tiles: 477 us by place, 468 with a warp per tile and one sum).
+// A block copies the coefficients for two tiles: only up to 16 KB of them.
 enum { SLAB_BY_GROUP = 1, SLAB_BY_PLACE = 2 };
 constexpr int64_t SLAB_SPLIT = 400;
-inline int slab_split(int prec, bool in_order, int64_t tiles, int tile_steps, bool real, size_t lut_bytes) {
+constexpr int64_t SLAB_FP64_SUMS = 1 << 14;
+inline int slab_split(int prec, bool in_order, bool one_pass, int64_t tiles, int tile_steps, bool real, size_t lut_bytes) {
     const bool few = lut_bytes <= 16 * 1024;
     if (prec != 0 && in_order) return few && tiles >= 4 && tiles <= 600 ? SLAB_BY_PLACE : 0;
     if (in_order && few && tiles <= 1024 && (real || tile_steps <= 16)) return SLAB_BY_PLACE;
-    return tiles <= SLAB_SPLIT ? SLAB_BY_GROUP : 0;
+    if (tiles <= SLAB_SPLIT) return SLAB_BY_GROUP;
+    return prec == 0 && !in_order && one_pass && few && tiles <= SLAB_FP64_SUMS ? SLAB_BY_PLACE : 0;
 }
-// FP64, by-bond tables: four partial sums per row up to this many tiles (triangular 6x4, 3520 tiles: 69 us, 80
-// with one sum; 7x4, 44600 tiles: 491 and 487).  In-order tables have one (chain L = 26: 30 us, 36 with four,
-// whose registers leave room for fewer warps).
-constexpr int64_t SLAB_FP64_SUMS = 1 << 14;
 // Coefficient tables of at most this many entries go to registers (real) or to one copy per shared-
 // memory bank group (SLAB_REP_BYTES in all, which keeps eight blocks of the slab kernel per SM).
 constexpr int SLAB_REG_LUT = 4;

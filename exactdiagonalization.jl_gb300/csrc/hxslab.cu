@@ -466,7 +466,7 @@ __device__ __forceinline__ void fma_if(double2& a, double2 c, double2 x, unsigne
 // group's gathers are under way, the entries of the group after the next are read, on through the
 // warp's tiles.  SUMS: partial sums per row, by the entry's place in its group; mixed precision takes
 // four (a row of 93 terms is half as far from its 64-bit sum as with one) or two (SlabRun::two_sums).
-// FP64 takes four on small by-bond tables (SLAB_FP64_SUMS), else one, and does not add up a step without
+// FP64 takes four on small by-bond tables (SLAB_FP64_SUMS; mostly by place), else one, and does not add up a step without
 // entries (the last ones of a tile may be), since the FP64 pipe sets the pace (a warp's double-precision FMA takes
 // 16 cycles of an SM).  To keep it busy, the gathers run a
 // group ahead of the additions there (complex128, chain L = 27 at k = 1 98.3 -> 94.5 us, L = 28 104.3 -> 101.1;
@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(HX_THREADS, 2) hx_slab_split_kernel(const Slab
 }
 
 // Four warps share a tile, warp w of them taking every group's step w: the sums per row of hx_slab_pad_kernel with
-// four partial sums, bit for bit, in chains a quarter as long (small in-order tables: slab_split).
+// four partial sums, bit for bit, in chains a quarter as long (slab_split).
 template <int PREC, bool REAL, int LUTM>
 __global__ void __launch_bounds__(HX_THREADS, 2) hx_slab_place_kernel(const SlabRun r) {
     typedef typename Cx<PREC>::V V;
@@ -924,7 +924,7 @@ void hx_slab_launch(int prec, const SlabRun& run, cudaStream_t st) {
     const size_t csize = (size_t)(r.lut_real ? 1 : 2) * (prec == 0 ? 8 : 4);
     const size_t smem = (size_t)(r.n_lut + 1) * (r.lut_mode == 1 ? 128 : csize);   // (and a padding entry's id)
     // (by the table's tiles, not the launch's: row blocks add up alike)
-    if (r.padded) r.split = slab_split(prec, r.in_order, (r.n_rows + 31) / 32, r.tile_steps, r.lut_real, smem);
+    if (r.padded) r.split = slab_split(prec, r.in_order, r.first && r.last, (r.n_rows + 31) / 32, r.tile_steps, r.lut_real, smem);
     if (prec == 0) slab_launch_p<0>(r, smem, st);
     else slab_launch_p<1>(r, smem, st);
 }

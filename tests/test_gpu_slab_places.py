@@ -1,5 +1,5 @@
 """The slab product of sectors around the sizes up to which four warps share a tile by place (600 and 1024 tiles of
-in-order tables), and coefficient tables below and above the size for it.  Products
+in-order tables, 400 and 16384 of others in FP64), and coefficient tables below and above the size for it.  Products
 repeated back to back, against the oracle's reduced product, 1e-12 in FP64 and 1e-5 in mixed precision (the
 bounds of the slab product's other tests)."""
 import numpy as np
