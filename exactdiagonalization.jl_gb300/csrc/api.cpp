@@ -237,7 +237,7 @@ struct edgpu_op_s {
         DevBuf<double> xsc;                 // [2 dim] the scaled x (complex64 or complex128)
     } slab;
     int slab_scaling = 0;             // scaled slab tables: 0 for sectors of 2^22 rows or more, 1 never, 2 always
-    int slab_use[2] = {0, 0};         // [precision]: products read the slab table (chosen by the autotuner)
+    int slab_use[2] = {0, 0};         // [precision]: not 0: products read the slab table (edgpu_op_slab_use's value)
     // host-buffer slab products: a second stream converting x slab by slab while the passes run
     cudaStream_t aux_st = nullptr;
     cudaEvent_t aux_fork = nullptr;
@@ -263,7 +263,6 @@ struct edgpu_op_s {
             blk_ev.push_back(e);
         }
     }
-    int slab_hint[2] = {0, 0};        // [precision]: edgpu_op_slab_use's value less one, kept for its queries
     // Lanczos: pinned host memory the steps write their alpha, beta and norm to (three doubles a step and
     // three more), and the events after which those of the even and odd steps are there
     double* lz_slots = nullptr;
@@ -2706,11 +2705,8 @@ int edgpu_op_slab_use(edgpu_op oh, int32_t precision, int32_t use, int32_t* curr
     check_prec(precision);
     require(use >= -1 && use <= 6, EDGPU_ERR_ARG, "use must be -1 (query) or 0 to 6");
     require(use <= 0 || op->slab.tab, EDGPU_ERR_STATE, "no slab table (edgpu_op_build_slabs)");
-    if (use >= 0) {
-        op->slab_use[precision] = use > 0 ? 1 : 0;
-        op->slab_hint[precision] = use > 0 ? use - 1 : 0;
-    }
-    if (current) *current = op->slab_use[precision] ? 1 + op->slab_hint[precision] : 0;
+    if (use >= 0) op->slab_use[precision] = use;
+    if (current) *current = op->slab_use[precision];
     API_END
 }
 
@@ -2786,14 +2782,14 @@ int edgpu_op_autotune(edgpu_op oh, int32_t precision, int32_t* rows_per_tile_out
     // (and the caller allows it), that schedule with 2 or 4 targets per step (4 with a map or a
     // target table) and 1, 2 or 4 lanes per row, and its target-table flavour (one lane per row).
     // With a slab table, also its multi-pass product.
-    struct Cand { int pair, nt, table, rows, pf, uni, slab = 0, hint = 0; };
+    struct Cand { int pair, nt, table, rows, pf, uni, slab = 0; };
     std::vector<Cand> cands;
     build_blob(op, precision, 0, 0);
     const bool pair_ok = op->blob[precision][0][0].tmpl.bond_ncls > 0 && op->pair_allowed;
     const bool mapped = op->space->d_map != nullptr;
     if (pair_ok) {
         if (op->slab.tab)
-            cands.push_back({1, 4, 1, -1, 0, 0, 1, 0});
+            cands.push_back({1, 4, 1, -1, 0, 0, 1});
         if (op->d_tab) {
             for (int nt : {8, 4, 2})
                 for (int pf : {0, 4, 64}) cands.push_back({1, nt, 1, -1, pf, 0});
@@ -2809,7 +2805,7 @@ int edgpu_op_autotune(edgpu_op oh, int32_t precision, int32_t* rows_per_tile_out
     Cand best = cands.front();
     double best_ms = 1e30;
     const int keep_pair = op->pair_use[precision], keep_nt = op->pair_nt[precision], keep_tab = op->tab_use[precision];
-    const int keep_uni = op->tab_uni[precision], keep_slab = op->slab_use[precision], keep_hint = op->slab_hint[precision];
+    const int keep_uni = op->tab_uni[precision], keep_slab = op->slab_use[precision];
     if (n > 0) {
         const size_t vs = precision == EDGPU_FP64 ? 16 : 8;
         void *x = nullptr, *y = nullptr;
@@ -2827,7 +2823,6 @@ int edgpu_op_autotune(edgpu_op oh, int32_t precision, int32_t* rows_per_tile_out
                 op->tab_pf[precision] = c.pf;
                 op->tab_uni[precision] = c.uni;
                 op->slab_use[precision] = c.slab;
-                op->slab_hint[precision] = c.hint;
                 launch_product(op, precision, 0, 0, x, y, 0, nullptr, nullptr, op->hs.stream(), nullptr, c.rows);
                 // one timed launch, then two back-to-back bursts of enough launches to cover about 2 ms
                 // (1 to 50 per burst), as a solver issues them; the faster burst's time per launch
@@ -2860,7 +2855,6 @@ int edgpu_op_autotune(edgpu_op oh, int32_t precision, int32_t* rows_per_tile_out
             op->tab_use[precision] = keep_tab;
             op->tab_uni[precision] = keep_uni;
             op->slab_use[precision] = keep_slab;
-            op->slab_hint[precision] = keep_hint;
             cudaFree(x);
             cudaFree(y);
             cudaEventDestroy(e0);
@@ -2878,7 +2872,6 @@ int edgpu_op_autotune(edgpu_op oh, int32_t precision, int32_t* rows_per_tile_out
     op->tab_pf[precision] = best.pf;
     op->tab_uni[precision] = best.uni;
     op->slab_use[precision] = best.slab;
-    op->slab_hint[precision] = best.hint;
     op->tuned_rows[precision] = best.rows;
     if (rows_per_tile_out) *rows_per_tile_out = best.rows;
     if (best_ms_out) *best_ms_out = best_ms;
@@ -3057,8 +3050,8 @@ static void host_product(edgpu_op_s* op, int prec, int dir, const double* x, dou
                                           op->d_tab, (const void*)op->slab.tab,
                                           (const void*)(intptr_t)(op->pair_allowed + 2 * op->pair_use[prec] +
                                                                   4 * op->pair_nt[prec] + 64 * op->tab_use[prec] +
-                                                                  128 * op->tab_uni[prec] + 256 * op->slab_use[prec] +
-                                                                  512 * op->tab_pf[prec] + (1 << 20) * op->slab_hint[prec]),
+                                                                  128 * op->tab_uni[prec] + 256 * (op->slab_use[prec] != 0) +
+                                                                  512 * op->tab_pf[prec]),
                                           (const void*)(intptr_t)slab_row_blocks(op, prec, n)};
     auto it = op->host_graphs.find(key);
     if (it == op->host_graphs.end()) {
@@ -3951,7 +3944,7 @@ int edgpu_batch_mul_device(edgpu_batch bh, int32_t precision, const void* const*
         key.push_back(batch_params(b, precision, xs, ys, &blocks).blob);   // the image (vectors, sector maps)
     } else {
         for (int i = 0; i < n; ++i) {
-            // per-sector launches read the operators' own tables (and their slab variants)
+            // per-sector launches read the operators' own tables
             key.push_back(b->ops[i]->d_tab);
             key.push_back(b->ops[i]->space->d_map);
             const edgpu_op_s* o = b->ops[i];
@@ -3959,8 +3952,7 @@ int edgpu_batch_mul_device(edgpu_batch bh, int32_t precision, const void* const*
             // the operator's own schedule (modes 5 to 7 launch with it)
             key.push_back((const void*)(intptr_t)(o->pair_allowed + 2 * o->pair_use[precision] + 4 * o->pair_nt[precision] +
                                                   64 * o->tab_use[precision] + 128 * o->tab_uni[precision] +
-                                                  256 * o->slab_use[precision] + 512 * o->tab_pf[precision] +
-                                                  (1 << 20) * o->slab_hint[precision]));
+                                                  256 * (o->slab_use[precision] != 0) + 512 * o->tab_pf[precision]));
             key.push_back((const void*)(intptr_t)o->tuned_rows[precision]);
             key.push_back((const void*)(uintptr_t)o->gen);
         }

@@ -1461,10 +1461,9 @@ __global__ void __launch_bounds__(256, 4) k_unreduce(const PW* parent, long long
                                                   VectorTables::Dev t, const V* small, V* large) {
     __shared__ W st[256 * UNRED_E + 256 * UNRED_E / 32];   // (one word in 33 spare: no bank conflicts)
     __shared__ W keep[64];
-    if (threadIdx.x < 64) keep[threadIdx.x] = g.kind == GK_TORUS && threadIdx.x < g.L1 ? (W)g.keep[threadIdx.x] : (W)0;
-    __syncthreads();
+    stage_keep<W>(keep, g);
     const bool want_arg = g.den > 1;
-    const bool ring = sizeof(W) == 4 && g.kind == GK_TORUS && g.L2 == 1 && g.nbits <= 31;
+    const bool ring = ring32<W>(g);
     const int pb = t.elem_bits;
     for (long long base = (long long)blockIdx.x * (256 * UNRED_E); base < n_parent;
          base += (long long)gridDim.x * (256 * UNRED_E)) {
