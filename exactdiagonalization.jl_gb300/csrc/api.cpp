@@ -1302,8 +1302,9 @@ void launch_slab_passes(edgpu_op_s* op, int prec, const Blob& B, const void* x, 
 
 // Row blocks of a host-buffer slab product (launch_slab_passes): EDGPU_SLAB_ROW_BLOCKS when set (1 to
 // 64); else 2 for mixed precision on sectors of 2^22 rows or more with at least 4 passes (on 6x6 k=0,
-// 252M rows: 95.2 -> 89.5 ms per H x with pinned complex128 buffers; 4 blocks gain little more,
-// and the FP64 product is slower in blocks), 1 otherwise.
+// 252M rows, with pinned complex128 buffers: 95.2 -> 89.5 ms per H x on one host, 95.5 to 97.4 ms with one block and
+// with two on others, where the writes to the host set the pace; 4 blocks gain little more, and the FP64 product
+// is slower in blocks), 1 otherwise.
 int slab_row_blocks(const edgpu_op_s* op, int prec, int64_t n) {
     const char* v = std::getenv("EDGPU_SLAB_ROW_BLOCKS");
     if (v && *v) {

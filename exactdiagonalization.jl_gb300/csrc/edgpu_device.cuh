@@ -275,7 +275,8 @@ __device__ __forceinline__ void canon_ring_n(unsigned q, int pb, bool want_arg, 
 }
 
 // Ring canonicalisation dispatched on the (warp-uniform) ring length for 1-bit sites: three instructions
-// per rotation unrolled, about five in a loop (chain L = 25, k = 3: 70 -> 61 us a product).
+// per rotation unrolled, about five in a loop (odd lengths unrolled, and dependents let in late: chain L = 25,
+// k = 3, 85 -> 70 us a product).
 __device__ __forceinline__ void canon_ring(unsigned q, int n, int L1, int w, int pb, bool want_arg, unsigned& rep,
                                            int& gbest) {
     if (w == 1) {

@@ -456,10 +456,12 @@ struct SlabRun {
 constexpr double SLAB_PAD_MOST = 1.5;
 constexpr int64_t SLAB_PAD_SMALL = 1 << 14;
 // One slab of short rows (at most this many steps per tile on average: chains): the rows' entries stay in
-// the target table's order, which fills the steps as well and costs little where few gathers per row wait
-// for each other anyway (chain L = 24, complex64: 4.9 us in order, 4.5 by bond; L = 28, complex128: 104 us
-// in order, 108 by bond).  In mixed precision such a row has four partial sums, two from SLAB_TWO_SUMS rows
-// on: the sums, bit for bit, that four and two lanes per row gave these sectors.
+// the target table's order.  That fills the steps better, which FP64 gains by (complex128, in order and by bond:
+// chain L = 24 9.65 and 11.2 us, L = 26 30.4 and 35.0, L = 28 101 and 104), and costs mixed precision, which reads
+// the same table, gathers that share fewer lines (complex64: 4.0 and 3.8 us, 9.6 and 8.9, 31.9 and 30.2).  In
+// mixed precision such a row has four partial sums, two from SLAB_TWO_SUMS rows on (chain L = 24 4.0 us, 4.1 with
+// four; L = 28 31.9 and 33.3; for 14 to 28 random terms two sums are 9 to 17% further from the 64-bit sum than four,
+// and one 21 to 28% further than two).
 constexpr int SLAB_IN_ORDER = 32;
 constexpr int64_t SLAB_TWO_SUMS = 1 << 16;
 // Several warps share a tile of a padded table where the table leaves most of the chip empty and a row's chain
@@ -479,7 +481,8 @@ constexpr int64_t SLAB_TWO_SUMS = 1 << 16;
 enum { SLAB_BY_GROUP = 1, SLAB_BY_PLACE = 2 };
 constexpr int64_t SLAB_SPLIT = 400;
 constexpr int64_t SLAB_FP64_SUMS = 1 << 14;
-inline int slab_split(int prec, bool in_order, bool one_pass, int64_t tiles, int tile_steps, bool real, size_t lut_bytes) {
+inline int slab_split(int prec, bool in_order, bool one_pass, int64_t tiles, int tile_steps, bool real,
+                      size_t lut_bytes) {
     const bool few = lut_bytes <= 16 * 1024;
     if (prec != 0 && in_order) return few && tiles >= 4 && tiles <= 600 ? SLAB_BY_PLACE : 0;
     if (in_order && few && tiles <= 1024 && (real || tile_steps <= 16)) return SLAB_BY_PLACE;
@@ -545,8 +548,8 @@ void launch_lanczos_project(int64_t n, int k, const void* V, bool c64, int64_t l
 // for other coefficients h); slot (host memory the device can address): alpha, |w| and
 // nrm2 (without one: |w|^2)
 void launch_lanczos_correct(int64_t n, int k, const void* V, bool c64, int64_t ldv, const double* h_dev,
-                            const double* hmax_dev, const double* w1, const double* v, const double* u, const double* alpha_dev,
-                            const double* beta_dev, double* w, double* scratch, unsigned* tickets, double* beta_out,
+                            const double* hmax_dev, const double* w1, const double* v, const double* u,
+                            const double* alpha_dev, const double* beta_dev, double* w, double* scratch, unsigned* tickets, double* beta_out,
                             const double* nrm2_dev, double* slot, cudaStream_t st);
 // v_next = w / beta (beta_dev: beta, 1 / beta); also writes a complex64 copy when v32 != null
 void launch_normalize(int64_t n, const double* w, const double* beta_dev, double* v_next, float* v32,

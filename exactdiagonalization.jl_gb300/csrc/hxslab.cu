@@ -21,14 +21,15 @@
 //
 // What bounds the product, and what the steps gave (complex64, H x in device time, before -> now;
 // before, every lane walked its own row's run of entries): triangular 6x5, 5.2 million rows, one pass,
-// 1167 -> 687 us; square 4x8, 18.8 million rows, two passes, 2960 -> 1750 us; square 6x6, 252 million
-// rows, 18 passes, 70.6 -> 63.9 ms; chain L = 24, 112,720 rows, 5.5 -> 4.9 us.  It was bound by the L1
+// 1168 -> 674 us; square 4x8, 18.8 million rows, two passes, 2963 -> 1715 us; square 6x6, 252 million
+// rows, 18 passes, 70.6 -> 64.0 ms; chain L = 24, 112,720 rows, 5.6 -> 4.0 us.  It was bound by the L1
 // data pipe (every entry load and every gather a line of its own); now a gather touches 0.2 (chains) to
 // 0.5 (tori) lines per entry, and the L1 tag lookups of those lines and the L2 requests behind them
-// share the limit (24 sectors of the triangular 6x4, 113,000 rows each: 352 us of tag lookups in 394 us;
+// share the limit (24 sectors of the triangular 6x4, 113,000 rows each: 352 us of tag lookups in 376 us;
 // one launch over all of them, or more padding, gained nothing).  In FP64 the FP64 pipe sets the pace,
-// before and now (chain L = 28 107.6 -> 104.3 us, 6x6 130 -> 131.5 ms): a double-precision FMA occupies
-// it for 16 cycles of an SM per warp, so the mean filling of the steps counts there.
+// before and now (chain L = 28 106.7 -> 100.9 us, triangular 6x5 at k = 1 3502 -> 3448, 6x6 130.1 -> 128.4 ms): a
+// double-precision FMA occupies it for 16 cycles of an SM per warp, so the mean filling of the steps counts
+// there.
 #include "hx_bond.cuh"
 
 #include <algorithm>
@@ -183,7 +184,8 @@ __global__ void __launch_bounds__(HX_THREADS) hx_slab_fill_kernel(const HxParams
                     if (has) {
                         const unsigned ph = p.want_arg ? (unsigned)num[g] : 0u;
                         const unsigned ap = (unsigned)__ldg(s.amp_id + ((ti << 2) | v)) * (unsigned)p.den + ph;
-                        const unsigned id = s.scaled ? ap : (ap * (unsigned)p.nd + (unsigned)ri) * (unsigned)p.nd + (unsigned)sx;
+                        const unsigned nd = (unsigned)p.nd;
+                        const unsigned id = s.scaled ? ap : (ap * nd + (unsigned)ri) * nd + (unsigned)sx;
                         entry = ((unsigned)c - (unsigned)q * wc) | (id << s.colbits);
                     }
                     if (s.in_order) {   // (one slab)
@@ -466,9 +468,9 @@ __device__ __forceinline__ void fma_if(double2& a, double2 c, double2 x, unsigne
 // group's gathers are under way, the entries of the group after the next are read, on through the
 // warp's tiles.  SUMS: partial sums per row, by the entry's place in its group; mixed precision takes
 // four (a row of 93 terms is half as far from its 64-bit sum as with one) or two (SlabRun::two_sums).
-// FP64 takes four on small by-bond tables (SLAB_FP64_SUMS; mostly by place), else one, and does not add up a step without
-// entries (the last ones of a tile may be), since the FP64 pipe sets the pace (a warp's double-precision FMA takes
-// 16 cycles of an SM).  To keep it busy, the gathers run a
+// FP64 takes four on small by-bond tables (SLAB_FP64_SUMS; mostly by place), else one, and does not add up a
+// step without entries (the last ones of a tile may be), since the FP64 pipe sets the pace (a warp's
+// double-precision FMA takes 16 cycles of an SM).  To keep it busy, the gathers run a
 // group ahead of the additions there (complex128, chain L = 27 at k = 1 98.3 -> 94.5 us, L = 28 104.3 -> 101.1;
 // triangular 6x5 at k = 1 3596 -> 3451, square 4x8 in two passes 5321 -> 5125); in mixed precision the registers
 // for that cost more than it gives (chain L = 24 5.5 -> 6.9 us).
@@ -823,7 +825,8 @@ void slab_build_t(int pass, const HxParams& p, const SlabBuild& s, cudaStream_t 
     auto k = pass == 1 ? hx_slab_count_kernel<W, PREC> : hx_slab_fill_kernel<W, PREC>;
     raise_smem_limit((const void*)k, smem);
     const long long warps = threads / 32;
-    const int blocks = (int)std::max<long long>(1, std::min<long long>((s.n_tiles + warps - 1) / warps, (long long)sm_count() * 16));
+    const long long need = (s.n_tiles + warps - 1) / warps;
+    const int blocks = (int)std::max<long long>(1, std::min<long long>(need, (long long)sm_count() * 16));
     k<<<blocks, threads, smem, st>>>(p, s);
     EDGPU_CUDA(cudaGetLastError());
 }
@@ -924,7 +927,8 @@ void hx_slab_launch(int prec, const SlabRun& run, cudaStream_t st) {
     const size_t csize = (size_t)(r.lut_real ? 1 : 2) * (prec == 0 ? 8 : 4);
     const size_t smem = (size_t)(r.n_lut + 1) * (r.lut_mode == 1 ? 128 : csize);   // (and a padding entry's id)
     // (by the table's tiles, not the launch's: row blocks add up alike)
-    if (r.padded) r.split = slab_split(prec, r.in_order, r.first && r.last, (r.n_rows + 31) / 32, r.tile_steps, r.lut_real, smem);
+    if (r.padded)
+        r.split = slab_split(prec, r.in_order, r.first && r.last, (r.n_rows + 31) / 32, r.tile_steps, r.lut_real, smem);
     if (prec == 0) slab_launch_p<0>(r, smem, st);
     else slab_launch_p<1>(r, smem, st);
 }

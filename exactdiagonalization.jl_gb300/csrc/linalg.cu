@@ -310,8 +310,8 @@ __device__ __forceinline__ float2 lz_top(const float2& v) { return v; }
 template <typename VT>
 __global__ void __launch_bounds__(LZ_AXPY_THREADS, 8)
 k_lz_correct(long long n, int K, const VT* V, long long ldv, const double2* h, const double* hmax, const double2* w1,
-             const double2* v, const double2* u, const double* alpha, const double* beta, double2* w, double* partial, double* beta_out,
-             const double* nrm2, double* slot, unsigned* ticket) {
+             const double2* v, const double2* u, const double* alpha, const double* beta, double2* w, double* partial,
+             double* beta_out, const double* nrm2, double* slot, unsigned* ticket) {
     __shared__ double2 hs[LZ_CHUNK];
     __shared__ float2 hf[LZ_CHUNK];
     __shared__ double red[LZ_AXPY_THREADS / 32];
@@ -486,7 +486,8 @@ static unsigned lz_correct_blocks(int64_t n) {
 
 void launch_lanczos_alpha(int64_t n, const double* v, double* w, const float* y32, double* scratch, unsigned* tickets,
                           double* alpha_dev, cudaStream_t st) {
-    const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>((n + LZ_THREADS - 1) / LZ_THREADS, (n < (1 << 20) ? 1ll : 4ll) * std::max(1, sm_count())));
+    const int64_t need = (n + LZ_THREADS - 1) / LZ_THREADS, most = (n < (1 << 20) ? 1ll : 4ll) * std::max(1, sm_count());
+    const unsigned blocks = (unsigned)std::max<int64_t>(1, std::min<int64_t>(need, most));
     k_lz_alpha<<<blocks, LZ_THREADS, 0, st>>>(n, (const double2*)v, (double2*)w, (const float2*)y32, (double2*)scratch,
                                              alpha_dev, tickets);
     EDGPU_CUDA(cudaGetLastError());
@@ -522,8 +523,8 @@ void launch_lanczos_project(int64_t n, int k, const void* V, bool c64, int64_t l
 }
 
 void launch_lanczos_correct(int64_t n, int k, const void* V, bool c64, int64_t ldv, const double* h_dev,
-                            const double* hmax_dev, const double* w1, const double* v, const double* u, const double* alpha_dev,
-                            const double* beta_dev, double* w, double* scratch, unsigned* tickets, double* beta_out,
+                            const double* hmax_dev, const double* w1, const double* v, const double* u,
+                            const double* alpha_dev, const double* beta_dev, double* w, double* scratch, unsigned* tickets, double* beta_out,
                             const double* nrm2_dev, double* slot, cudaStream_t st) {
     const dim3 grid(lz_correct_blocks(n));
     auto go = [&](auto* basis, auto kern) {

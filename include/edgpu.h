@@ -240,8 +240,9 @@ int edgpu_op_targets_info(edgpu_op op, int64_t* entries, int32_t* entry_bytes);
  * product up to the order of the additions (the passes are added in order: reproducible run to
  * run).  *built = 0 (nothing kept) when the table would exceed max_bytes, the sector has 2^32 rows or
  * more, a row has more than 255 targets, the terms of one pair slot have different couplings, or the
- * coefficient table does not fit; the autotuner then never picks it.  A new build replaces the old
- * one; new coupling values rewrite its coefficient table in place. */
+ * coefficient table does not fit; the autotuner then never picks it.  The table takes the fastest of its
+ * forms that fits max_bytes; the smallest has 4 bytes per entry, a byte per row and slab and 4 bytes per
+ * 32 rows and slab (a scaled table 17 bytes per row more).  A new build replaces the old one; new coupling values rewrite its coefficient table in place. */
 int edgpu_op_build_slabs(edgpu_op op, int64_t slab_bytes, int64_t max_bytes, int32_t* built);
 int edgpu_op_free_slabs(edgpu_op op);
 /* Slabs (passes), columns per slab and entries of the slab table; zeros without one. */
