@@ -698,10 +698,13 @@ __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_kernel(
 }
 
 // The same through a table with the rows' counts (where the caller's limit has no room for masks): step k's
-// rows are those with more than k entries, so the masks come from ballots.
+// rows are those with more than k entries, so the masks come from ballots.  Its targets do not lie by bond
+// (triangular 6x5 at k = 1, complex64 905 us, 674 padded by bond; complex128, where the FP64 pipe sets the pace,
+// 3443 and 3448, 3554 without the gathers ahead).
 template <int PREC, bool REAL, int LUTM>
 __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_counted_kernel(const SlabRun r) {
     typedef typename Cx<PREC>::V V;
+    constexpr bool AHEAD = PREC == 0;
     extern __shared__ __align__(16) unsigned char sm[];
     if (r.early) pdl_launch_dependents();
     const SlabLut<PREC, REAL, LUTM> lut(r, sm);
@@ -723,21 +726,40 @@ __global__ void __launch_bounds__(HX_THREADS, PREC == 0 ? 3 : 4) hx_slab_counted
             return e;
         };
         V sums[PREC == 0 ? 1 : 4] = {};   // partial sums, as hx_slab_pad_kernel's
-        unsigned e[4];
+        // (AHEAD as in the masked kernel: x and id of this group, e the entries of the next)
+        V x[4];
+        unsigned e[4], id[4];
 #pragma unroll
         for (int h = 0; h < 4; ++h) e[h] = next(h);
-        for (unsigned k = 0; k < steps; k += 4) {
-            V xv[4];
-            unsigned id[4];
+        if (AHEAD) {
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
-                xv[h] = xs[e[h] & r.colmask];
+                x[h] = xs[e[h] & r.colmask];
                 id[h] = e[h] >> r.colbits;
             }
 #pragma unroll
-            for (int h = 0; h < 4; ++h) e[h] = next(k + 4 + h);
+            for (int h = 0; h < 4; ++h) e[h] = next(4 + h);
+        }
+        for (unsigned k = 0; k < steps; k += 4) {
+            V xn[4];
+            unsigned idn[4];
 #pragma unroll
-            for (int h = 0; h < 4; ++h) fma_if(sums[PREC == 0 ? 0 : h], lut(id[h]), xv[h], k + h, cnt);
+            for (int h = 0; h < 4; ++h) {
+                xn[h] = xs[e[h] & r.colmask];
+                idn[h] = e[h] >> r.colbits;
+            }
+#pragma unroll
+            for (int h = 0; h < 4; ++h) e[h] = next(k + (AHEAD ? 8 : 4) + h);
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                if (PREC == 0 && h > 0 && k + h >= steps) continue;
+                fma_if(sums[PREC == 0 ? 0 : h], lut(AHEAD ? id[h] : idn[h]), AHEAD ? x[h] : xn[h], k + h, cnt);
+            }
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                x[h] = xn[h];
+                id[h] = idn[h];
+            }
         }
         V acc = sums[0];
         if constexpr (PREC != 0) acc = cadd(cadd(acc, sums[1]), cadd(sums[2], sums[3]));
