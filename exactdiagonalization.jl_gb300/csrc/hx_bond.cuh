@@ -133,8 +133,10 @@ __device__ __forceinline__ int bond_row_count(W b, const BondTables<W, PREC>& bt
 
 // acc (or sum) += element x of one target in FP64 with trivial characters, with as few double-precision
 // operations as its form needs: the FP64 pipe takes 16 cycles of an SM for each of a warp's.  An amplitude
-// that all pairs share is applied to the row's sum; the ratio of the orbit sizes is 1 for nearly all
-// targets (equal) and skipped there.  (With characters this form gained on long rings, chain L = 25, k = 3,
+// that all pairs share is applied to the row's sum; the ratio of the orbit sizes is 1 for nearly all targets, and
+// skipped in the fused gradient where it is for the whole warp (equal).  Per target and lane that branch cost the
+// products more than the operations it saved (without tables, k = 0, complex128: chain L = 26 66 us with it, 54
+// without, 61 in the nine-operation form; L = 18 12.5, 10.8 and 10.7).  (With characters this form gained on long rings, chain L = 25, k = 3,
 // but lost on tori, triangular 5x4, k = (1, 2): 86 -> 102 us; and maps, tables and all groups add alike.)
 __device__ __forceinline__ void bond_add_fp64(const HxParams& p, double2 a, const double* rrow, bool equal, int sx,
                                               double2 x, double2& acc, double2& sum) {
@@ -143,7 +145,7 @@ __device__ __forceinline__ void bond_add_fp64(const HxParams& p, double2 a, cons
             sum.x += x.x;
             sum.y += x.y;
         } else {
-            const double f = rrow[sx];
+            const double f = rrow[sx];   // (1 for equal sizes)
             sum.x = fma_r(f, x.x, sum.x);
             sum.y = fma_r(f, x.y, sum.y);
         }
@@ -379,6 +381,19 @@ __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W,
         V xv[NT];
 #pragma unroll
         for (int h = 0; h < NT; ++h) xv[h] = (c[h] >= 0) ? x[c[h]] : czero<V>();
+        if constexpr (PREC == 0 && !GRAD) {
+            if (p.bond_slot >= 0 && !(GK != GK_TRIVIAL && sc.want_arg)) {
+                // one branch a step, not one or two per target, whose element and ratio then wait together (the
+                // ratio is exactly 1 for equal orbit sizes, and a missing x is 0)
+#pragma unroll
+                for (int h = 0; h < NT; ++h) {
+                    const double f = GK == GK_TRIVIAL ? 1.0 : rrow[c[h] >= 0 ? sx[h] : 0];
+                    sum.x = fma_r(f, xv[h].x, sum.x);
+                    sum.y = fma_r(f, xv[h].y, sum.y);
+                }
+                continue;
+            }
+        }
 #pragma unroll
         for (int h = 0; h < NT; ++h) {
             if (grad_one) {
@@ -418,10 +433,9 @@ __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W,
             }
             if (PREC == 0 && !(GK != GK_TRIVIAL && sc.want_arg)) {
                 if constexpr (PREC == 0) {
-                    // equal: this target's ratio of the orbit sizes is 1; in the fused gradient, all of the warp's
-                    // (a warp branch there, where the FP64 pipe is all that counts)
-                    const bool equal = GK == GK_TRIVIAL ||
-                                       (GRAD ? !__any_sync(0xffffffffu, c[h] >= 0 && sx[h] != ri) : sx[h] == ri);
+                    // equal: the ratio of the orbit sizes is 1 for all of the warp's targets (a warp branch in the
+                    // fused gradient, where the FP64 pipe is all that counts)
+                    const bool equal = GK == GK_TRIVIAL || (GRAD && !__any_sync(0xffffffffu, c[h] >= 0 && sx[h] != ri));
                     if (c[h] >= 0 && want_y) bond_add_fp64(p, bt.amp[ti[h]], rrow, equal, sx[h], xv[h], acc, sum);
                 }
             } else if (c[h] >= 0 && want_y) {
