@@ -145,7 +145,7 @@ __device__ __forceinline__ void bond_add_fp64(const HxParams& p, double2 a, cons
             sum.x += x.x;
             sum.y += x.y;
         } else {
-            const double f = rrow[sx];   // (1 for equal sizes)
+            const double f = rrow[sx];
             sum.x = fma_r(f, x.x, sum.x);
             sum.y = fma_r(f, x.y, sum.y);
         }
@@ -381,10 +381,12 @@ __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W,
         V xv[NT];
 #pragma unroll
         for (int h = 0; h < NT; ++h) xv[h] = (c[h] >= 0) ? x[c[h]] : czero<V>();
-        if constexpr (PREC == 0 && !GRAD) {
+        if constexpr (PREC == 0 && !GRAD && GK != GK_TORUS && GK != GK_GENERIC) {
             if (p.bond_slot >= 0 && !(GK != GK_TRIVIAL && sc.want_arg)) {
                 // one branch a step, not one or two per target, whose element and ratio then wait together (the
-                // ratio is exactly 1 for equal orbit sizes, and a missing x is 0)
+                // ratio is exactly 1 for equal orbit sizes, and a missing x is 0).  Where a torus search or a
+                // general group's sets the time it gains nothing, and the code costs (triangular 6x3, k = (2, 1):
+                // 64.7 us without it, 65.1 with).
 #pragma unroll
                 for (int h = 0; h < NT; ++h) {
                     const double f = GK == GK_TRIVIAL ? 1.0 : rrow[c[h] >= 0 ? sx[h] : 0];
@@ -433,9 +435,10 @@ __device__ __forceinline__ void bond_tile(const HxParams& p, const RowsTables<W,
             }
             if (PREC == 0 && !(GK != GK_TRIVIAL && sc.want_arg)) {
                 if constexpr (PREC == 0) {
-                    // equal: the ratio of the orbit sizes is 1 for all of the warp's targets (a warp branch in the
-                    // fused gradient, where the FP64 pipe is all that counts)
-                    const bool equal = GK == GK_TRIVIAL || (GRAD && !__any_sync(0xffffffffu, c[h] >= 0 && sx[h] != ri));
+                    // equal: this target's ratio of the orbit sizes is 1; in the fused gradient, all of the warp's
+                    // (a warp branch there, where the FP64 pipe is all that counts)
+                    const bool equal = GK == GK_TRIVIAL ||
+                                       (GRAD ? !__any_sync(0xffffffffu, c[h] >= 0 && sx[h] != ri) : sx[h] == ri);
                     if (c[h] >= 0 && want_y) bond_add_fp64(p, bt.amp[ti[h]], rrow, equal, sx[h], xv[h], acc, sum);
                 }
             } else if (c[h] >= 0 && want_y) {
